@@ -230,3 +230,76 @@ def tolerance(case):
     if kind == "layer":
         return {"rel": 1.6e-2}
     return {"rel": {"f32": 2.6e-6, "f16": 1.2e-3, "bf16": 1e-2}[dtype]}
+
+
+def _exact_streaming(q, k, v, do, length, c, back, q_start=0):
+    """One sequence of one batch entry in 64 bits: ``q [H, Tq, D]`` holds positions ``q_start ..``, ``k``, ``v``
+    ``[H, T, D]``.  Chunk by chunk against the chunk's key window; ``(o, dq, dk, dv)``, the gradients None without
+    ``do``."""
+    q, k, v = q.double(), k.double(), v.double()
+    scale = q.shape[-1] ** -0.5
+    o = torch.zeros_like(q)
+    dq, dk, dv = (None, None, None) if do is None else (torch.zeros_like(t) for t in (q, k, v))
+    for lo in range(q_start // c * c, length, c):
+        r0, r1 = max(lo, q_start), min(lo + c, length)
+        k0 = max(lo - back * c, 0)
+        qi, ki, vi = q[:, r0 - q_start:r1 - q_start], k[:, k0:r1], v[:, k0:r1]
+        if r0 >= r1:
+            continue
+        p = torch.softmax(qi @ ki.mT * scale, dim=-1)
+        o[:, r0 - q_start:r1 - q_start] = p @ vi
+        if do is not None:
+            doi = do[:, r0:r1].double()
+            dv[:, k0:r1] += p.mT @ doi
+            ds = p * (doi @ vi.mT - (doi * (p @ vi)).sum(-1, keepdim=True)) * scale
+            dq[:, r0:r1] = ds @ ki
+            dk[:, k0:r1] += ds.mT @ qi
+    return o, dq, dk, dv
+
+
+def exact(case, seed):
+    """What ``run`` returns, in 64 bits; None where the chunks are too many for a loop over them."""
+    kind = case["kind"]
+    if kind == "softmax":
+        return torch.cat([torch.softmax(x.double(), dim=-1) for x in prepare(case, seed)["x"].split(4096)])
+    if kind == "dense":
+        st = prepare(case, seed)
+        return torch.stack([_exact_streaming(st["q"][b], st["k"][b], st["v"][b], None, int(n), case["T"], 0)[0]
+                            for b, n in enumerate(st["lens"].tolist())])
+    seqs = case["seqs"] if kind == "packed" else case["B"]
+    chunks = seqs * (case["len_hi"] if kind == "packed" else case["T"]) // case["c"]
+    rows = seqs * case["H"] * (case["len_hi"] if kind == "packed" else case["T"])
+    if chunks > 20000 or rows * case["D"] > 3.0e8:
+        return None
+    st = prepare(case, seed)
+    c, back = case["c"], case["back"]
+    if kind == "packed":
+        outs = [torch.zeros(st[n].shape, dtype=torch.float64, device="cuda") for n in ("q", "q", "k", "v")]
+        cu = st["cu"].tolist()
+        for a, z in zip(cu, cu[1:]):
+            heads = (st[n].detach()[a:z].transpose(0, 1) for n in ("q", "k", "v", "do"))
+            for out, got in zip(outs, _exact_streaming(*heads, z - a, c, back)):
+                out[a:z] = got.transpose(0, 1)
+        return tuple(outs)
+    if kind == "layer":
+        H, Hk, D = case["H"], case["H_kv"], case["D"]
+        w_qkv, w_o, cos, sin = (st[n].double() for n in ("w_qkv", "w_o", "cos", "sin"))
+        ys = []
+        for x in st["x"]:
+            q, k, v = (x.double() @ w_qkv.T).view(-1, H + 2 * Hk, D).transpose(0, 1).split((H, Hk, Hk))
+            q, k = (torch.cat([t[..., :D // 2] * cos.T - t[..., D // 2:] * sin.T,
+                               t[..., D // 2:] * cos.T + t[..., :D // 2] * sin.T], dim=-1) for t in (q, k))
+            k, v = (t.repeat_interleave(H // Hk, dim=0) for t in (k, v))
+            o = _exact_streaming(q, k, v, None, x.shape[0], c, back)[0]
+            ys.append(o.transpose(0, 1).reshape(-1, H * D) @ w_o.T)
+        return torch.stack(ys)
+    q, k, v = (st[n].detach() for n in "qkv")
+    group = q.shape[1] // k.shape[1]
+    k, v = (t.repeat_interleave(group, dim=1) for t in (k, v))
+    lens = st.get("lens")
+    lens = [case["T"]] * case["B"] if lens is None else lens.tolist()
+    do = st.get("do")
+    q_start = case["T"] - case["Tq"] if kind == "step" else 0
+    per_seq = [_exact_streaming(q[b], k[b], v[b], None if do is None else do[b], int(n), c, back, q_start) for b, n in enumerate(lens)]
+    outs = [torch.stack(ts) for ts in zip(*per_seq) if ts[0] is not None]
+    return tuple(outs) if kind == "train" else outs[0]
