@@ -730,7 +730,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     int n = 0;
     bool ok = true;
-    Item it;
+    Item it = {};
     it.b = -1;
     for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
       it = decode_item<PACKED>(a, item, n_ktiles, it);
@@ -930,13 +930,10 @@ __device__ __forceinline__ DqItem decode_dq_item(const FusedArgs& a, int item, i
   it.h = bh - it.b * a.H;
   it.row0 = 0;
   if (PACKED) {
-    if (it.b == prev.b) {
-      it.row0 = prev.row0;
-      it.len = prev.len;
-    } else {
-      it.row0 = a.cu[it.b];
-      it.len = kb_min_i32(a.cu[it.b + 1] - it.row0, a.T);
-    }
+    // always read: taking the offset and length over from `prev` when the sequence is the same gave wrong dQ for
+    // every item after the first of a sequence on its CTA (the loads hit L1, and these roles run ahead or wait for HBM)
+    it.row0 = a.cu[it.b];
+    it.len = kb_min_i32(a.cu[it.b + 1] - it.row0, a.T);
   } else {
     it.len = !a.lens ? a.T : (it.b == prev.b ? prev.len : kb_clamp_len(a.lens[(int64_t)it.b * a.lens_stride], a.T));
   }
@@ -988,7 +985,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       prefetch_tensormap(&tm_k);
       int u = 0;
       bool ok = true;
-      DqItem it;
+      DqItem it = {};
       it.b = -1;
       for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
         it = decode_dq_item<PACKED>(a, item, n_tiles_t, it);
@@ -1010,7 +1007,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       constexpr uint32_t idesc = make_idesc(BF16, kBQ, D, true, true);  // A = dS read MN-major (rows = keys), B = K MN-major
       int u = 0, m = 0;
       bool ok = true;
-      DqItem it;
+      DqItem it = {};
       it.b = -1;
       for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
         it = decode_dq_item<PACKED>(a, item, n_tiles_t, it);
@@ -1039,7 +1036,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
     int m = 0;
     bool ok = true;
-    DqItem it;
+    DqItem it = {};
     it.b = -1;
     for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
       it = decode_dq_item<PACKED>(a, item, n_tiles_t, it);

@@ -30,6 +30,8 @@ def _cu(lens):
     (2, 2, 1100, 128, 256, 2, torch.float16, [1100, 1024]),
     (3, 1, 300, 64, 10, 5, torch.bfloat16, [299, 17, 128]),
     (2, 2, 260, 128, 32, 2, torch.float16, [5, 130, 256, 257, 1, 127, 128, 129, 0, 260]),  # every kind of last tile
+    (8, 8, 2600, 128, 64, 2, torch.bfloat16, [2600, 130, 2500]),  # more tiles per sequence than CTAs: a CTA's next
+    (8, 8, 2600, 64, 100, 1, torch.float16, [130, 2600, 2571]),   # item is of the same sequence
 ])
 @pytest.mark.parametrize("single_launch", [True, False])
 def test_packed_equals_padded_bitwise(H, Hk, T, D, c, back, dtype, lens, single_launch):
