@@ -6,10 +6,23 @@
 // inputs forbids TF32).  The fp16/bf16 hot shapes are served by the tcgen05 kernels; this
 // file is what runs everywhere else.
 //
-// Work split: one CTA of 256 threads owns one tile of BM query rows (forward, dQ) or BN key
-// rows (dK/dV) of one (batch, head) and walks only the live tiles of the streaming schedule
-// (schedule.h).  Threads form a 16x16 grid: thread (ty, tx) owns rows ty+16*i and columns
-// tx+16*j of every [rows x cols] product, so row reductions are 16-lane shuffles.
+// Work split: one CTA owns one tile of BM query rows (forward, dQ) or BN key rows (dK/dV) of
+// one (batch, head) and walks only the live tiles of the streaming schedule (schedule.h).
+// Bound: the fp32 FMA pipe, then shared-memory bandwidth.  Threads form a TY x 16 grid; thread
+// (ty, tx) owns the stationary rows ty + TY*i and the streamed columns tx + 16*j of a score block.
+//   * Scores (A B^T): both operands are read along the head dimension, four elements per load, and
+//     the products are packed fp32 pairs (fma.rn.f32x2: even and odd elements of the head dimension
+//     accumulate side by side), so an 8 x 4 block costs 12 16-byte loads and 64 instructions per four
+//     head-dim elements.
+//   * The second matmul (P V, dS K, P dO, dS Q): the block goes through shared memory transposed,
+//     [streamed column][stationary row], a thread's rows next to each other, so that a row PAIR is one
+//     operand of the packed product and only the other operand has to be duplicated.
+// 8 x 4 blocks of 128 threads up to head dim 64 (three / two CTAs per SM); larger head dims leave room for one
+// CTA per SM and take 256 threads with half the rows each.  Measured on B200 (fp32, B=16 H=4 T=2000 D=64 c=32 back=4,
+// lengths 1000-2000): forward 238 -> 145 us, dQ 336 -> 202 us, dK/dV 618 -> 260 us against 4 x 4 blocks of 256
+// threads with one product per instruction, scalar loads and a division per mask element; 31-35 TFLOP/s of the
+// blocks' arithmetic.  Tiles come in with cp.async where the rows
+// are fp32, 16-byte aligned and dense, the next one while the current block is still being worked on.
 //
 // Reference semantics followed: src/streaming_attention/kernel.py:205-430 (forward),
 // 639-773 and 941-1023 (dQ), 777-937 and 1027-1129 (dK/dV), 453-514 (delta).
@@ -17,23 +30,39 @@
 
 #include "common.cuh"
 #include "sm100_host.h"
+#include "sm100_ptx.cuh"
 #include "tiles.h"
 
 namespace kb {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kPad = 4;  // floats of row padding: keeps float4 alignment, spreads banks
+
+// tile rows and thread grid by head dim (see above)
+template <int D>
+struct Cfg {
+  static constexpr int BM = tiles::generic_tile(D), BN = BM;
+  static constexpr int TY = D <= 64 ? 8 : 16;
+  static constexpr int kThreads = TY * 16;
+  static constexpr int LD = D + kPad;   // row stride of an operand tile, floats
+  static constexpr int PLD = BM + kPad; // row stride of a transposed score block
+  static constexpr int RM = BM / TY, RN = BN / 16, DV = D / 16;
+  static constexpr int VEC = DV < 4 ? DV : 4, NG = DV / VEC;  // a thread's head-dim columns: g*16*VEC + tx*VEC + e
+  static constexpr int kCtasFwd = D <= 64 ? 3 : 1, kCtasBwd = D <= 64 ? 2 : 1;
+};
 
 template <typename T>
 struct TensorArg {
   const T* p;
   int64_t sb, sh, st, sd;
+  bool vec;  // rows are dense fp32 and 16-byte aligned: cp.async takes them
 };
 
 template <typename T>
 TensorArg<T> make_arg(const kb_tensor4& t) {
-  return TensorArg<T>{static_cast<const T*>(t.data), t.stride[0], t.stride[1], t.stride[2], t.stride[3]};
+  const bool vec = sizeof(T) == 4 && reinterpret_cast<uintptr_t>(t.data) % 16 == 0 && t.stride[3] == 1 && t.stride[0] % 4 == 0 &&
+                   t.stride[1] % 4 == 0 && t.stride[2] % 4 == 0;
+  return TensorArg<T>{static_cast<const T*>(t.data), t.stride[0], t.stride[1], t.stride[2], t.stride[3], vec};
 }
 
 template <typename T>
@@ -61,44 +90,131 @@ struct BwdArgs {
   float scale_log2, sm_scale;
 };
 
-// [ROWS x D] tile of one (b, h) slice -> shared memory as fp32; rows past T read as zero.
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// [ROWS x D] tile of one (b, h) slice -> shared memory as fp32; rows past T read as zero.  Asynchronous (one
+// cp.async group, committed here) for dense aligned fp32 rows, otherwise done when it returns.
 template <int D, int ROWS, typename T>
-__device__ __forceinline__ void load_tile(float* dst, const T* slice, int64_t st, int64_t sd, int row0, int T_) {
-  constexpr int LD = D + kPad;
-  for (int idx = threadIdx.x; idx < ROWS * D; idx += kThreads) {
-    int r = idx / D, d = idx - r * D;
-    int t = row0 + r;
-    float x = 0.f;
-    if (t < T_) x = to_f32(slice[(int64_t)t * st + (int64_t)d * sd]);
-    dst[r * LD + d] = x;
+__device__ __forceinline__ void load_tile(float* dst, const TensorArg<T>& a, int b, int h, int row0, int T_) {
+  constexpr int LD = Cfg<D>::LD, kThreads = Cfg<D>::kThreads;
+  const T* slice = a.p + b * a.sb + h * a.sh;
+  if (sizeof(T) == 4 && a.vec) {
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < ROWS * (D / 4); idx += kThreads) {
+      const int r = idx / (D / 4), d = (idx - r * (D / 4)) * 4, t = row0 + r;
+      const bool in = t < T_;
+      const T* src = slice + (in ? (int64_t)t * a.st + d : 0);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm100::smem_u32(dst + r * LD + d)), "l"(src), "r"(in ? 16 : 0)
+                   : "memory");
+    }
+  } else {
+    for (int idx = threadIdx.x; idx < ROWS * D; idx += kThreads) {
+      const int r = idx / D, d = idx - r * D, t = row0 + r;
+      dst[r * LD + d] = t < T_ ? to_f32(slice[(int64_t)t * a.st + (int64_t)d * a.sd]) : 0.f;
+    }
+  }
+  cp_async_commit();
+}
+
+// acc[i][j] = sum_d A[ty + TY i][d] * Bm[tx + 16 j][d]
+template <int D>
+__device__ __forceinline__ void tile_abt(const float* A, const float* Bm, float (&acc)[Cfg<D>::RM][Cfg<D>::RN], int ty, int tx) {
+  using C = Cfg<D>;
+  uint64_t acc2[C::RM][C::RN];
+#pragma unroll
+  for (int i = 0; i < C::RM; ++i)
+#pragma unroll
+    for (int j = 0; j < C::RN; ++j) acc2[i][j] = 0ull;
+#pragma unroll 2
+  for (int d = 0; d < D; d += 4) {
+    ulonglong2 a[C::RM], b[C::RN];
+#pragma unroll
+    for (int i = 0; i < C::RM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(&A[(ty + C::TY * i) * C::LD + d]);
+#pragma unroll
+    for (int j = 0; j < C::RN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(&Bm[(tx + 16 * j) * C::LD + d]);
+#pragma unroll
+    for (int i = 0; i < C::RM; ++i)
+#pragma unroll
+      for (int j = 0; j < C::RN; ++j) {
+        acc2[i][j] = sm100::f2_fma(a[i].x, b[j].x, acc2[i][j]);
+        acc2[i][j] = sm100::f2_fma(a[i].y, b[j].y, acc2[i][j]);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < C::RM; ++i)
+#pragma unroll
+    for (int j = 0; j < C::RN; ++j) {
+      float x, y;
+      sm100::f2_unpack(acc2[i][j], x, y);
+      acc[i][j] = x + y;
+    }
+}
+
+// The block's values of one streamed column, for the thread's rows, next to each other (row ty + TY i in slot ty RM + i).
+template <int D>
+__device__ __forceinline__ void store_transposed(float* Xt, const float (&x)[Cfg<D>::RM][Cfg<D>::RN], int ty, int tx) {
+  using C = Cfg<D>;
+#pragma unroll
+  for (int j = 0; j < C::RN; ++j) {
+    float* dst = &Xt[(tx + 16 * j) * C::PLD + ty * C::RM];
+    if (C::RM % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < C::RM; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(x[i][j], x[i + 1][j], x[i + 2][j], x[i + 3][j]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < C::RM; i += 2) *reinterpret_cast<float2*>(dst + i) = make_float2(x[i][j], x[i + 1][j]);
+    }
   }
 }
 
-// acc[i][j] = sum_d A[ty+16i][d] * Bm[tx+16j][d]
-template <int D, int RM, int RN>
-__device__ __forceinline__ void tile_abt(const float* A, const float* Bm, float (&acc)[RM][RN], int ty, int tx) {
-  constexpr int LD = D + kPad;
-#pragma unroll
-  for (int i = 0; i < RM; ++i)
-#pragma unroll
-    for (int j = 0; j < RN; ++j) acc[i][j] = 0.f;
+// acc[row pair][column] += sum_kk X[row][kk] * V[kk][column], X transposed in shared memory, V [kk][LD]
+template <int D>
+__device__ __forceinline__ void tile_xv(const float* Xt, const float* V, uint64_t (&acc)[Cfg<D>::RM / 2][Cfg<D>::DV], int ty, int tx) {
+  using C = Cfg<D>;
 #pragma unroll 4
-  for (int d = 0; d < D; d += 4) {
-    float4 a[RM], b[RN];
+  for (int kk = 0; kk < C::BN; ++kk) {
+    uint64_t x[C::RM / 2];
+    const float* xp = &Xt[kk * C::PLD + ty * C::RM];
+    if (C::RM % 4 == 0) {
 #pragma unroll
-    for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(&A[(ty + 16 * i) * LD + d]);
-#pragma unroll
-    for (int j = 0; j < RN; ++j) b[j] = *reinterpret_cast<const float4*>(&Bm[(tx + 16 * j) * LD + d]);
-#pragma unroll
-    for (int i = 0; i < RM; ++i)
-#pragma unroll
-      for (int j = 0; j < RN; ++j) {
-        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-        acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-        acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+      for (int i = 0; i < C::RM / 4; ++i) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(xp + 4 * i);
+        x[2 * i] = t.x;
+        x[2 * i + 1] = t.y;
       }
+    } else {
+#pragma unroll
+      for (int i = 0; i < C::RM / 2; ++i) x[i] = *reinterpret_cast<const uint64_t*>(xp + 2 * i);
+    }
+#pragma unroll
+    for (int g = 0; g < C::NG; ++g) {
+      float v[C::VEC];
+      const float* vp = &V[kk * C::LD + g * 16 * C::VEC + tx * C::VEC];
+      if (C::VEC == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(vp);
+        v[0] = t.x, v[C::VEC > 1 ? 1 : 0] = t.y, v[C::VEC > 2 ? 2 : 0] = t.z, v[C::VEC > 3 ? 3 : 0] = t.w;
+      } else if (C::VEC == 2) {
+        const float2 t = *reinterpret_cast<const float2*>(vp);
+        v[0] = t.x, v[C::VEC > 1 ? 1 : 0] = t.y;
+      } else {
+        v[0] = *vp;
+      }
+#pragma unroll
+      for (int e = 0; e < C::VEC; ++e) {
+        const uint64_t vv = sm100::f2_pack(v[e], v[e]);
+#pragma unroll
+        for (int i = 0; i < C::RM / 2; ++i) acc[i][g * C::VEC + e] = sm100::f2_fma(x[i], vv, acc[i][g * C::VEC + e]);
+      }
+    }
   }
+}
+
+template <int D>
+__device__ __forceinline__ int col_of(int n, int tx) {  // head-dim column of a thread's n-th accumulator
+  using C = Cfg<D>;
+  return (n / C::VEC) * 16 * C::VEC + tx * C::VEC + n % C::VEC;
 }
 
 __device__ __forceinline__ float half_warp_max(float x) {
@@ -116,17 +232,59 @@ __device__ __forceinline__ int load_len(const int32_t* lens, int64_t stride, int
   return lens ? kb_clamp_len(lens[(int64_t)b * stride], T_) : T_;
 }
 
+// The live keys of query i form the interval [lo, hi) (empty for a padded row): the element form of the mask.
+__device__ __forceinline__ void live_interval(int i, int len, int c, int back, int& lo, int& hi) {
+  lo = hi = 0;
+  if (i < len) {
+    const int qc = i / c;
+    lo = kb_max_i32(0, qc - back) * c;
+    const int64_t h = (int64_t)(qc + 1) * c;
+    hi = h < len ? (int)h : len;
+  }
+}
+
+// Rows of a thread's accumulators, scaled, into the contiguous [T, D] output slice; a column vector per store
+// where the output is fp32 and aligned.
+template <int D, typename T>
+__device__ __forceinline__ void store_rows(T* slice, const uint64_t (&acc)[Cfg<D>::RM / 2][Cfg<D>::DV], const float (&scale)[Cfg<D>::RM],
+                                           const bool (&zero)[Cfg<D>::RM], int row0, int T_, int ty, int tx) {
+  using C = Cfg<D>;
+  const bool vec = sizeof(T) == 4 && C::VEC == 4 && (reinterpret_cast<uintptr_t>(slice) & 15) == 0;
+#pragma unroll
+  for (int i = 0; i < C::RM; ++i) {
+    const int r = row0 + ty + C::TY * i;
+    if (r >= T_) continue;
+    float x[C::DV];
+#pragma unroll
+    for (int n = 0; n < C::DV; ++n) {
+      float a0, a1;
+      sm100::f2_unpack(acc[i / 2][n], a0, a1);
+      x[n] = zero[i] ? 0.f : (i & 1 ? a1 : a0) * scale[i];
+    }
+    T* dst = slice + (int64_t)r * D;
+    if (vec) {
+#pragma unroll
+      for (int n = 0; n + 3 < C::DV; n += 4)
+        *reinterpret_cast<float4*>(dst + col_of<D>(n, tx)) = make_float4(x[n], x[n + 1], x[n + 2], x[n + 3]);
+    } else {
+#pragma unroll
+      for (int n = 0; n < C::DV; ++n) dst[col_of<D>(n, tx)] = from_f32<T>(x[n]);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------
-template <int D, int BM, int BN, typename T>
-__global__ void __launch_bounds__(kThreads) sa_fwd_generic_kernel(FwdArgs<T> a) {
-  constexpr int LD = D + kPad, RM = BM / 16, RN = BN / 16, DV = D / 16, PLD = BN + 1;
+template <int D, typename T>
+__global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasFwd) sa_fwd_generic_kernel(const FwdArgs<T> a) {
+  using C = Cfg<D>;
+  constexpr int BM = C::BM, BN = C::BN, RM = C::RM, RN = C::RN;
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;
-  float* Ks = Qs + BM * LD;
-  float* Vs = Ks + BN * LD;
-  float* Ps = Vs + BN * LD;
+  float* Ks = Qs + BM * C::LD;
+  float* Vs = Ks + BN * C::LD;
+  float* Pt = Vs + BN * C::LD;
 
   const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * BM;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -137,43 +295,39 @@ __global__ void __launch_bounds__(kThreads) sa_fwd_generic_kernel(FwdArgs<T> a) 
 
   const KbTileRange kr = kb_fwd_kv_range(q0, BM, BN, len, c, back);
 
-  float m[RM], l[RM], acc[RM][DV];
-  int qchunk[RM];
+  float m[RM], l[RM];
+  int lo[RM], hi[RM];
+  uint64_t acc[RM / 2][C::DV];
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
     m[i] = -INFINITY;
     l[i] = 0.f;
-    qchunk[i] = (q0 + ty + 16 * i) / c;
-#pragma unroll
-    for (int dv = 0; dv < DV; ++dv) acc[i][dv] = 0.f;
+    live_interval(q0 + ty + C::TY * i, len, c, back, lo[i], hi[i]);
   }
+#pragma unroll
+  for (int i = 0; i < RM / 2; ++i)
+#pragma unroll
+    for (int n = 0; n < C::DV; ++n) acc[i][n] = 0ull;
 
   if (kr.begin < kr.end) {
-    load_tile<D, BM>(Qs, a.q.p + b * a.q.sb + h * a.q.sh, a.q.st, a.q.sd, q0, T_);
-    const T* k_slice = a.k.p + b * a.k.sb + h * a.k.sh;
-    const T* v_slice = a.v.p + b * a.v.sb + h * a.v.sh;
+    load_tile<D, BM>(Qs, a.q, b, h, q0, T_);
+    load_tile<D, BN>(Ks, a.k, b, h, kr.begin * BN, T_);
+    load_tile<D, BN>(Vs, a.v, b, h, kr.begin * BN, T_);
     for (int kt = kr.begin; kt < kr.end; ++kt) {
       const int k0 = kt * BN;
-      __syncthreads();
-      load_tile<D, BN>(Ks, k_slice, a.k.st, a.k.sd, k0, T_);
-      load_tile<D, BN>(Vs, v_slice, a.v.st, a.v.sd, k0, T_);
+      cp_async_wait<1>();  // everything but V
       __syncthreads();
 
       float s[RM][RN];
-      tile_abt<D, RM, RN>(Qs, Ks, s, ty, tx);
-
-      int kchunk[RN];
-#pragma unroll
-      for (int j = 0; j < RN; ++j) kchunk[j] = (k0 + tx + 16 * j) / c;
+      tile_abt<D>(Qs, Ks, s, ty, tx);
 
 #pragma unroll
       for (int i = 0; i < RM; ++i) {
-        const int qi = q0 + ty + 16 * i;
         float mx = -INFINITY;
 #pragma unroll
         for (int j = 0; j < RN; ++j) {
-          const bool live = kb_live(qi, k0 + tx + 16 * j, qchunk[i], kchunk[j], len, back);
-          s[i][j] = live ? s[i][j] * a.scale_log2 : -INFINITY;
+          const int kj = k0 + tx + 16 * j;
+          s[i][j] = (kj >= lo[i] && kj < hi[i]) ? s[i][j] * a.scale_log2 : -INFINITY;
           mx = fmaxf(mx, s[i][j]);
         }
         mx = half_warp_max(mx);
@@ -183,57 +337,55 @@ __global__ void __launch_bounds__(kThreads) sa_fwd_generic_kernel(FwdArgs<T> a) 
         float rs = 0.f;
 #pragma unroll
         for (int j = 0; j < RN; ++j) {
-          const float p = exp2f(s[i][j] - m_safe);
-          Ps[(ty + 16 * i) * PLD + tx + 16 * j] = p;
-          rs += p;
+          s[i][j] = exp2f(s[i][j] - m_safe);
+          rs += s[i][j];
         }
         rs = half_warp_sum(rs);
         l[i] = l[i] * alpha + rs;
         m[i] = m_new;
 #pragma unroll
-        for (int dv = 0; dv < DV; ++dv) acc[i][dv] *= alpha;
-      }
-      __syncthreads();
-
-#pragma unroll 4
-      for (int kk = 0; kk < BN; ++kk) {
-        float pv[RM];
-#pragma unroll
-        for (int i = 0; i < RM; ++i) pv[i] = Ps[(ty + 16 * i) * PLD + kk];
-#pragma unroll
-        for (int dv = 0; dv < DV; ++dv) {
-          const float vv = Vs[kk * LD + tx + 16 * dv];
-#pragma unroll
-          for (int i = 0; i < RM; ++i) acc[i][dv] = fmaf(pv[i], vv, acc[i][dv]);
+        for (int n = 0; n < C::DV; ++n) {
+          float a0, a1;
+          sm100::f2_unpack(acc[i / 2][n], a0, a1);
+          if (i & 1) a1 *= alpha; else a0 *= alpha;
+          acc[i / 2][n] = sm100::f2_pack(a0, a1);
         }
       }
+      store_transposed<D>(Pt, s, ty, tx);
+      cp_async_wait<0>();
+      __syncthreads();  // P and V are there, K has been read
+      if (kt + 1 < kr.end) load_tile<D, BN>(Ks, a.k, b, h, k0 + BN, T_);
+      tile_xv<D>(Pt, Vs, acc, ty, tx);
+      __syncthreads();  // V and P have been read
+      if (kt + 1 < kr.end) load_tile<D, BN>(Vs, a.v, b, h, k0 + BN, T_);
     }
   }
 
+  float inv[RM];
+  bool zero[RM];
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
-    const int r = q0 + ty + 16 * i;
-    if (r >= T_) continue;
-    const bool valid = r < len;
-    const float inv = valid ? 1.f / l[i] : 0.f;
-#pragma unroll
-    for (int dv = 0; dv < DV; ++dv) o_slice[(int64_t)r * D + tx + 16 * dv] = from_f32<T>(valid ? acc[i][dv] * inv : 0.f);
-    if (lse_slice && tx == 0) lse_slice[r] = valid ? m[i] + log2f(l[i]) : 0.f;
+    const int r = q0 + ty + C::TY * i;
+    zero[i] = r >= len;
+    inv[i] = zero[i] ? 0.f : 1.f / l[i];
+    if (lse_slice && tx == 0 && r < T_) lse_slice[r] = zero[i] ? 0.f : m[i] + log2f(l[i]);
   }
+  store_rows<D, T>(o_slice, acc, inv, zero, q0, T_, ty, tx);
 }
 
 // ------------------------------------------------------------------------------------------
 // backward, dQ pass (also produces delta = rowsum(O * dO))
 // ------------------------------------------------------------------------------------------
-template <int D, int BM, int BN, typename T>
-__global__ void __launch_bounds__(kThreads) sa_bwd_dq_generic_kernel(BwdArgs<T> a) {
-  constexpr int LD = D + kPad, RM = BM / 16, RN = BN / 16, DV = D / 16, PLD = BN + 1;
+template <int D, typename T>
+__global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasBwd) sa_bwd_dq_generic_kernel(const BwdArgs<T> a) {
+  using C = Cfg<D>;
+  constexpr int BM = C::BM, BN = C::BN, RM = C::RM, RN = C::RN;
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;
-  float* dOs = Qs + BM * LD;
-  float* Ks = dOs + BM * LD;
-  float* Vs = Ks + BN * LD;
-  float* dSs = Vs + BN * LD;
+  float* dOs = Qs + BM * C::LD;
+  float* Ks = dOs + BM * C::LD;
+  float* Vs = Ks + BN * C::LD;
+  float* dSt = Vs + BN * C::LD;
 
   const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * BM;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -246,105 +398,104 @@ __global__ void __launch_bounds__(kThreads) sa_bwd_dq_generic_kernel(BwdArgs<T> 
 
   const KbTileRange kr = kb_fwd_kv_range(q0, BM, BN, len, c, back);
 
-  float acc[RM][DV], delta[RM], lse[RM];
-  int qchunk[RM];
+  uint64_t acc[RM / 2][C::DV];
+  float delta[RM], lse[RM], scale[RM];
+  bool zero[RM];
+  int lo[RM], hi[RM];
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
     delta[i] = 0.f;
     lse[i] = 0.f;
-    qchunk[i] = (q0 + ty + 16 * i) / c;
-#pragma unroll
-    for (int dv = 0; dv < DV; ++dv) acc[i][dv] = 0.f;
+    scale[i] = a.sm_scale;
+    zero[i] = false;
+    live_interval(q0 + ty + C::TY * i, len, c, back, lo[i], hi[i]);
   }
+#pragma unroll
+  for (int i = 0; i < RM / 2; ++i)
+#pragma unroll
+    for (int n = 0; n < C::DV; ++n) acc[i][n] = 0ull;
 
   if (kr.begin < kr.end) {
-    load_tile<D, BM>(Qs, a.q.p + b * a.q.sb + h * a.q.sh, a.q.st, a.q.sd, q0, T_);
-    load_tile<D, BM>(dOs, a.d_o.p + b * a.d_o.sb + h * a.d_o.sh, a.d_o.st, a.d_o.sd, q0, T_);
+    load_tile<D, BM>(Qs, a.q, b, h, q0, T_);
+    load_tile<D, BM>(dOs, a.d_o, b, h, q0, T_);
+    load_tile<D, BN>(Vs, a.v, b, h, kr.begin * BN, T_);
+    load_tile<D, BN>(Ks, a.k, b, h, kr.begin * BN, T_);
+    cp_async_wait<2>();  // Q and dO
     __syncthreads();
     const T* o_slice = a.o.p + b * a.o.sb + h * a.o.sh;
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
-      const int r = q0 + ty + 16 * i;
+      const int r = q0 + ty + C::TY * i;
       float part = 0.f;
       if (r < len) {
 #pragma unroll
-        for (int dv = 0; dv < DV; ++dv) {
-          const int d = tx + 16 * dv;
-          part = fmaf(to_f32(o_slice[(int64_t)r * a.o.st + (int64_t)d * a.o.sd]), dOs[(ty + 16 * i) * LD + d], part);
+        for (int n = 0; n < C::DV; ++n) {
+          const int d = col_of<D>(n, tx);
+          part = fmaf(to_f32(o_slice[(int64_t)r * a.o.st + (int64_t)d * a.o.sd]), dOs[(ty + C::TY * i) * C::LD + d], part);
         }
       }
       delta[i] = half_warp_sum(part);
       if (r < len) lse[i] = lse_slice[r];
     }
 
-    const T* k_slice = a.k.p + b * a.k.sb + h * a.k.sh;
-    const T* v_slice = a.v.p + b * a.v.sb + h * a.v.sh;
     for (int kt = kr.begin; kt < kr.end; ++kt) {
       const int k0 = kt * BN;
-      __syncthreads();
-      load_tile<D, BN>(Ks, k_slice, a.k.st, a.k.sd, k0, T_);
-      load_tile<D, BN>(Vs, v_slice, a.v.st, a.v.sd, k0, T_);
+      cp_async_wait<0>();
       __syncthreads();
 
       float s[RM][RN], dp[RM][RN];
-      tile_abt<D, RM, RN>(Qs, Ks, s, ty, tx);
-      tile_abt<D, RM, RN>(dOs, Vs, dp, ty, tx);
+      tile_abt<D>(Qs, Ks, s, ty, tx);
 #pragma unroll
-      for (int j = 0; j < RN; ++j) {
-        const int kj = k0 + tx + 16 * j;
-        const int kchunk = kj / c;
+      for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int i = 0; i < RM; ++i) {
-          const bool live = kb_live(q0 + ty + 16 * i, kj, qchunk[i], kchunk, len, back);
-          float ds = 0.f;
-          if (live) {
-            const float p = exp2f(s[i][j] * a.scale_log2 - lse[i]);
-            ds = p * (dp[i][j] - delta[i]);
-          }
-          dSs[(ty + 16 * i) * PLD + tx + 16 * j] = ds;
+        for (int j = 0; j < RN; ++j) {
+          const int kj = k0 + tx + 16 * j;
+          s[i][j] = (kj >= lo[i] && kj < hi[i]) ? exp2f(s[i][j] * a.scale_log2 - lse[i]) : 0.f;
         }
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (int kk = 0; kk < BN; ++kk) {
-        float dsv[RM];
+      tile_abt<D>(dOs, Vs, dp, ty, tx);
 #pragma unroll
-        for (int i = 0; i < RM; ++i) dsv[i] = dSs[(ty + 16 * i) * PLD + kk];
+      for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int dv = 0; dv < DV; ++dv) {
-          const float kv = Ks[kk * LD + tx + 16 * dv];
-#pragma unroll
-          for (int i = 0; i < RM; ++i) acc[i][dv] = fmaf(dsv[i], kv, acc[i][dv]);
+        for (int j = 0; j < RN; ++j) {
+          const int kj = k0 + tx + 16 * j;
+          s[i][j] = (kj >= lo[i] && kj < hi[i]) ? s[i][j] * (dp[i][j] - delta[i]) : 0.f;
         }
-      }
+      store_transposed<D>(dSt, s, ty, tx);
+      __syncthreads();  // dS is there, V has been read
+      if (kt + 1 < kr.end) load_tile<D, BN>(Vs, a.v, b, h, k0 + BN, T_);
+      tile_xv<D>(dSt, Ks, acc, ty, tx);
+      __syncthreads();  // K and dS have been read
+      if (kt + 1 < kr.end) load_tile<D, BN>(Ks, a.k, b, h, k0 + BN, T_);
     }
   }
 
+  store_rows<D, T>(dq_slice, acc, scale, zero, q0, T_, ty, tx);
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
-    const int r = q0 + ty + 16 * i;
-    if (r >= T_) continue;
-#pragma unroll
-    for (int dv = 0; dv < DV; ++dv) dq_slice[(int64_t)r * D + tx + 16 * dv] = from_f32<T>(acc[i][dv] * a.sm_scale);
-    if (tx == 0) delta_slice[r] = delta[i];
+    const int r = q0 + ty + C::TY * i;
+    if (tx == 0 && r < T_) delta_slice[r] = delta[i];
   }
 }
 
 // ------------------------------------------------------------------------------------------
 // backward, dK/dV pass (reads delta written by the dQ pass)
 // ------------------------------------------------------------------------------------------
-template <int D, int BM, int BN, typename T>
-__global__ void __launch_bounds__(kThreads) sa_bwd_dkdv_generic_kernel(BwdArgs<T> a) {
-  constexpr int LD = D + kPad, RM = BM / 16, RN = BN / 16, DV = D / 16, PLD = BN + 1;
+template <int D, typename T>
+__global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasBwd) sa_bwd_dkdv_generic_kernel(const BwdArgs<T> a) {
+  using C = Cfg<D>;
+  constexpr int BM = C::BM, BN = C::BN, RM = C::RM, RN = C::RN;
+  static_assert(BM == BN, "the score block is square: rows and columns swap roles here");
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;
-  float* dOs = Qs + BM * LD;
-  float* Ks = dOs + BM * LD;
-  float* Vs = Ks + BN * LD;
-  float* Ps = Vs + BN * LD;
-  float* dSs = Ps + BM * PLD;
-  float* lse_s = dSs + BM * PLD;
+  float* dOs = Qs + BM * C::LD;
+  float* Ks = dOs + BM * C::LD;
+  float* Vs = Ks + BN * C::LD;
+  float* Pt = Vs + BN * C::LD;
+  float* dSt = Pt + BM * C::PLD;
+  float* lse_s = dSt + BM * C::PLD;
   float* delta_s = lse_s + BM;
+  int* lo_s = reinterpret_cast<int*>(delta_s + BM);
+  int* hi_s = lo_s + BM;
 
   const int b = blockIdx.z, h = blockIdx.y, k0 = blockIdx.x * BN;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -358,87 +509,71 @@ __global__ void __launch_bounds__(kThreads) sa_bwd_dkdv_generic_kernel(BwdArgs<T
 
   const KbTileRange qr = kb_bwd_q_range(k0, BM, BN, len, c, back);
 
-  float acc_dk[RN][DV], acc_dv[RN][DV];
-  int kchunk[RN];
+  // stationary rows are keys here, streamed columns are queries
+  uint64_t acc_dk[RM / 2][C::DV], acc_dv[RM / 2][C::DV];
 #pragma unroll
-  for (int j = 0; j < RN; ++j) {
-    kchunk[j] = (k0 + tx + 16 * j) / c;
+  for (int i = 0; i < RM / 2; ++i)
 #pragma unroll
-    for (int dv = 0; dv < DV; ++dv) acc_dk[j][dv] = acc_dv[j][dv] = 0.f;
-  }
+    for (int n = 0; n < C::DV; ++n) acc_dk[i][n] = acc_dv[i][n] = 0ull;
 
   if (qr.begin < qr.end) {
-    load_tile<D, BN>(Ks, a.k.p + b * a.k.sb + h * a.k.sh, a.k.st, a.k.sd, k0, T_);
-    load_tile<D, BN>(Vs, a.v.p + b * a.v.sb + h * a.v.sh, a.v.st, a.v.sd, k0, T_);
-    const T* q_slice = a.q.p + b * a.q.sb + h * a.q.sh;
-    const T* do_slice = a.d_o.p + b * a.d_o.sb + h * a.d_o.sh;
+    load_tile<D, BN>(Ks, a.k, b, h, k0, T_);
+    load_tile<D, BN>(Vs, a.v, b, h, k0, T_);
     for (int qt = qr.begin; qt < qr.end; ++qt) {
       const int q0 = qt * BM;
-      __syncthreads();
-      load_tile<D, BM>(Qs, q_slice, a.q.st, a.q.sd, q0, T_);
-      load_tile<D, BM>(dOs, do_slice, a.d_o.st, a.d_o.sd, q0, T_);
+      load_tile<D, BM>(Qs, a.q, b, h, q0, T_);
+      load_tile<D, BM>(dOs, a.d_o, b, h, q0, T_);
       if (threadIdx.x < BM) {
         const int r = q0 + threadIdx.x;
         lse_s[threadIdx.x] = r < len ? lse_slice[r] : 0.f;
         delta_s[threadIdx.x] = r < len ? delta_slice[r] : 0.f;
+        live_interval(r, len, c, back, lo_s[threadIdx.x], hi_s[threadIdx.x]);
       }
+      cp_async_wait<0>();
       __syncthreads();
 
       float s[RM][RN], dp[RM][RN];
-      tile_abt<D, RM, RN>(Qs, Ks, s, ty, tx);
-      tile_abt<D, RM, RN>(dOs, Vs, dp, ty, tx);
+      tile_abt<D>(Ks, Qs, s, ty, tx);
 #pragma unroll
-      for (int i = 0; i < RM; ++i) {
-        const int ri = ty + 16 * i;
-        const int qi = q0 + ri;
-        const int qchunk = qi / c;
-        const float lse = lse_s[ri], delta = delta_s[ri];
+      for (int j = 0; j < RN; ++j) {
+        const int lo = lo_s[tx + 16 * j], hi = hi_s[tx + 16 * j];
+        const float lse = lse_s[tx + 16 * j];
 #pragma unroll
-        for (int j = 0; j < RN; ++j) {
-          const bool live = kb_live(qi, k0 + tx + 16 * j, qchunk, kchunk[j], len, back);
-          float p = 0.f, ds = 0.f;
-          if (live) {
-            p = exp2f(s[i][j] * a.scale_log2 - lse);
-            ds = p * (dp[i][j] - delta);
-          }
-          Ps[ri * PLD + tx + 16 * j] = p;
-          dSs[ri * PLD + tx + 16 * j] = ds;
+        for (int i = 0; i < RM; ++i) {
+          const int kj = k0 + ty + C::TY * i;
+          s[i][j] = (kj >= lo && kj < hi) ? exp2f(s[i][j] * a.scale_log2 - lse) : 0.f;
         }
       }
+      store_transposed<D>(Pt, s, ty, tx);
+      tile_abt<D>(Vs, dOs, dp, ty, tx);
+#pragma unroll
+      for (int j = 0; j < RN; ++j) {
+        const int lo = lo_s[tx + 16 * j], hi = hi_s[tx + 16 * j];
+        const float delta = delta_s[tx + 16 * j];
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+          const int kj = k0 + ty + C::TY * i;
+          s[i][j] = (kj >= lo && kj < hi) ? s[i][j] * (dp[i][j] - delta) : 0.f;
+        }
+      }
+      store_transposed<D>(dSt, s, ty, tx);
       __syncthreads();
-      // thread (ty, tx) now owns key rows ty+16j and head-dim columns tx+16dv
-#pragma unroll 2
-      for (int qq = 0; qq < BM; ++qq) {
-        float pk[RN], dsk[RN];
-#pragma unroll
-        for (int j = 0; j < RN; ++j) {
-          pk[j] = Ps[qq * PLD + ty + 16 * j];
-          dsk[j] = dSs[qq * PLD + ty + 16 * j];
-        }
-#pragma unroll
-        for (int dv = 0; dv < DV; ++dv) {
-          const float dov = dOs[qq * LD + tx + 16 * dv];
-          const float qv = Qs[qq * LD + tx + 16 * dv];
-#pragma unroll
-          for (int j = 0; j < RN; ++j) {
-            acc_dv[j][dv] = fmaf(pk[j], dov, acc_dv[j][dv]);
-            acc_dk[j][dv] = fmaf(dsk[j], qv, acc_dk[j][dv]);
-          }
-        }
-      }
+      tile_xv<D>(Pt, dOs, acc_dv, ty, tx);
+      tile_xv<D>(dSt, Qs, acc_dk, ty, tx);
+      __syncthreads();
     }
   }
 
+  float sc_k[RM], sc_v[RM];
+  bool zero[RM];
 #pragma unroll
-  for (int j = 0; j < RN; ++j) {
-    const int r = k0 + ty + 16 * j;
-    if (r >= T_) continue;
-#pragma unroll
-    for (int dv = 0; dv < DV; ++dv) {
-      dk_slice[(int64_t)r * D + tx + 16 * dv] = from_f32<T>(acc_dk[j][dv] * a.sm_scale);
-      dv_slice[(int64_t)r * D + tx + 16 * dv] = from_f32<T>(acc_dv[j][dv]);
-    }
+  for (int i = 0; i < RM; ++i) {
+    sc_k[i] = a.sm_scale;
+    sc_v[i] = 1.f;
+    zero[i] = false;
   }
+  store_rows<D, T>(dk_slice, acc_dk, sc_k, zero, k0, T_, ty, tx);
+  store_rows<D, T>(dv_slice, acc_dv, sc_v, zero, k0, T_, ty, tx);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -446,10 +581,9 @@ __global__ void __launch_bounds__(kThreads) sa_bwd_dkdv_generic_kernel(BwdArgs<T
 // ------------------------------------------------------------------------------------------
 template <int D, typename T>
 int launch_fwd(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s) {
-  constexpr int BM = tiles::generic_tile(D), BN = BM;
-  constexpr int LD = D + kPad;
-  constexpr size_t smem = sizeof(float) * (size_t)(BM * LD + 2 * BN * LD + BM * (BN + 1));
-  auto kern = sa_fwd_generic_kernel<D, BM, BN, T>;
+  using C = Cfg<D>;
+  constexpr size_t smem = sizeof(float) * (size_t)(C::BM * C::LD + 2 * C::BN * C::LD + C::BN * C::PLD);
+  auto kern = sa_fwd_generic_kernel<D, T>;
   int dev = 0, n_sm = 0;
   if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
   static std::atomic<bool> smem_opted_in[kMaxDevices];
@@ -467,20 +601,20 @@ int launch_fwd(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t 
   a.c = c;
   a.back = back;
   a.scale_log2 = p.sm_scale * kLog2e;
-  dim3 grid(kb_cdiv_i32(p.T, BM), p.H, p.B);
-  kern<<<grid, kThreads, smem, s>>>(a);
+  dim3 grid(kb_cdiv_i32(p.T, C::BM), p.H, p.B);
+  kern<<<grid, C::kThreads, smem, s>>>(a);
   KB_LAUNCH_CHECK("sa_fwd_generic_kernel");
   return KB_OK;
 }
 
 template <int D, typename T>
 int launch_bwd(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t s) {
-  constexpr int BM = tiles::generic_tile(D), BN = BM;
-  constexpr int LD = D + kPad;
-  constexpr size_t smem_dq = sizeof(float) * (size_t)(2 * BM * LD + 2 * BN * LD + BM * (BN + 1));
-  constexpr size_t smem_dkdv = sizeof(float) * (size_t)(2 * BM * LD + 2 * BN * LD + 2 * BM * (BN + 1) + 2 * BM);
-  auto kern_dq = sa_bwd_dq_generic_kernel<D, BM, BN, T>;
-  auto kern_dkdv = sa_bwd_dkdv_generic_kernel<D, BM, BN, T>;
+  using C = Cfg<D>;
+  constexpr size_t smem_dq = sizeof(float) * (size_t)(2 * C::BM * C::LD + 2 * C::BN * C::LD + C::BN * C::PLD);
+  constexpr size_t smem_dkdv = sizeof(float) * (size_t)(2 * C::BM * C::LD + 2 * C::BN * C::LD + 2 * C::BM * C::PLD + 4 * C::BM);
+  static_assert(smem_dkdv <= 232448, "shared memory exceeds the 227 KB a CTA may have");
+  auto kern_dq = sa_bwd_dq_generic_kernel<D, T>;
+  auto kern_dkdv = sa_bwd_dkdv_generic_kernel<D, T>;
   int dev = 0, n_sm = 0;
   if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
   static std::atomic<bool> dq_opted_in[kMaxDevices], dkdv_opted_in[kMaxDevices];
@@ -505,13 +639,13 @@ int launch_bwd(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t 
   a.back = back;
   a.scale_log2 = p.sm_scale * kLog2e;
   a.sm_scale = p.sm_scale;
-  dim3 grid_q(kb_cdiv_i32(p.T, BM), p.H, p.B), grid_k(kb_cdiv_i32(p.T, BN), p.H, p.B);
+  dim3 grid_q(kb_cdiv_i32(p.T, C::BM), p.H, p.B), grid_k(kb_cdiv_i32(p.T, C::BN), p.H, p.B);
   if (!(p.flags & KB_FLAG_BWD_SKIP_DQ)) {
-    kern_dq<<<grid_q, kThreads, smem_dq, s>>>(a);
+    kern_dq<<<grid_q, C::kThreads, smem_dq, s>>>(a);
     KB_LAUNCH_CHECK("sa_bwd_dq_generic_kernel");
   }
   if (!(p.flags & KB_FLAG_BWD_SKIP_DKDV)) {
-    kern_dkdv<<<grid_k, kThreads, smem_dkdv, s>>>(a);
+    kern_dkdv<<<grid_k, C::kThreads, smem_dkdv, s>>>(a);
     KB_LAUNCH_CHECK("sa_bwd_dkdv_generic_kernel");
   }
   return KB_OK;

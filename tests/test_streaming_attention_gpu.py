@@ -331,3 +331,35 @@ def test_dynamic_shapes_compile_into_few_graphs(lens_mode):
             out = api(q, k, v, lens, context_size=16, back_contexts=2, autotune=False)
             out.backward(torch.randn_like(out))
             assert torch._dynamo.utils.counters["stats"]["unique_graphs"] <= 4
+
+
+
+@pytest.mark.parametrize("D", [16, 32, 64, 128, 256])
+@pytest.mark.parametrize("T,c,back,layout", [(1, 1, 0, "bhtd"), (63, 7, 3, "odd"), (65, 64, 1, "bthd"), (129, 200, 0, "bhtd"), (200, 10, 5, "odd")])
+def test_fp32_tiles_edges_and_layouts(D, T, c, back, layout):
+    """The fp32 kernels one row around their tiles (64, 32 for D = 256), on rows that take asynchronous copies (dense,
+    16-byte aligned) and rows that do not, against dense attention in 64 bits.  Bounds: the fp32 ones of the grid."""
+    from kernels_b200.streaming_attention import streaming_attention
+
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+
+    def make():
+        if layout == "odd":  # rows start 4 bytes past a 16-byte boundary
+            return torch.randn(2 * 3 * T * D + 1, generator=g, device="cuda")[1:].view(2, 3, T, D)
+        x = torch.randn((2, T, 3, D) if layout == "bthd" else (2, 3, T, D), generator=g, device="cuda")
+        return x.transpose(1, 2) if layout == "bthd" else x
+
+    q, k, v, do = (make() for _ in range(4))
+    lens = torch.tensor([T, max(T - 2, 0)], dtype=torch.int32, device="cuda")
+    live = torch.arange(T, device="cuda")[None] < lens[:, None]
+    chunk = torch.arange(T, device="cuda") // c
+    diff = chunk[:, None] - chunk[None]
+    mask = ((diff >= 0) & (diff <= back))[None] & live[:, :, None] & live[:, None]
+    ref = [t.double().requires_grad_() for t in (q, k, v)]
+    scores = (ref[0] @ ref[1].mT * D**-0.5).masked_fill(~mask[:, None], -1e300)
+    want = (torch.softmax(scores, -1) @ ref[2]) * live[:, None, :, None]
+    got_in = [t.requires_grad_() for t in (q, k, v)]
+    got = streaming_attention(*got_in, lens, c, back)
+    assert (got - want).abs().max() <= 5e-6
+    for a, b in zip(torch.autograd.grad(got, got_in, do), torch.autograd.grad(want, ref, do.double())):
+        assert (a - b).abs().max() <= 5e-5
