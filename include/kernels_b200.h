@@ -157,6 +157,21 @@ typedef struct kb_sa_fwd_fp8_params {
 KB_API int kb_sa_fwd_fp8(const kb_sa_fwd_fp8_params* p, void* stream);
 
 /*
+ * The 8-bit inputs of kb_sa_fwd_fp8 from a [B, H, T, 128] fp32 / f16 / bf16 tensor, in one pass: `x8` contiguous
+ * e4m3 bytes, `scale` [B, H, ceil(T/128)] fp32 (largest magnitude of the tile of 128 rows / 448, at least 1e-12).
+ * Rows must be dense and 16-byte aligned (KB_ERR_UNSUPPORTED otherwise, and for other head dims).
+ */
+typedef struct kb_quantize_fp8_params {
+  kb_tensor4 x;
+  void* x8;
+  float* scale;
+  int32_t B, H, T, D;
+  int32_t dtype;
+} kb_quantize_fp8_params;
+
+KB_API int kb_quantize_fp8(const kb_quantize_fp8_params* p, void* stream);
+
+/*
  * Streaming attention backward: dQ, dK, dV from (q, k, v, o, lse, do).
  * Replaces both launches in `attention_backward_adapter`
  * (src/streaming_attention/kernel.py:1363-1442: `_streaming_attn_bwd_precompute`, lines

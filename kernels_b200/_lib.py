@@ -25,7 +25,7 @@ KB_NOALLOC_MAX_ROWS = 1 << 21
 _DTYPES = {torch.float32: KB_F32, torch.float16: KB_F16, torch.bfloat16: KB_BF16}
 
 EXPORTS = (
-    "kb_sa_fwd", "kb_sa_fwd_fp8", "kb_sa_bwd", "kb_sa_bwd_workspace_bytes", "kb_sa_bwd_noalloc", "kb_sa_fwd_varlen", "kb_sa_bwd_varlen",
+    "kb_sa_fwd", "kb_sa_fwd_fp8", "kb_quantize_fp8", "kb_sa_bwd", "kb_sa_bwd_workspace_bytes", "kb_sa_bwd_noalloc", "kb_sa_fwd_varlen", "kb_sa_bwd_varlen",
     "kb_sa_bwd_varlen_workspace_bytes", "kb_qkv_rope_proj", "kb_out_proj", "kb_fa_fwd", "kb_softmax_fwd", "kb_sa_plan", "kb_sa_tile_config",
     "kb_launch_count", "kb_strerror", "kb_last_cuda_error", "kb_version", "kb_selftest_wait_timeout",
 )
@@ -91,6 +91,13 @@ class SaVarlenParams(C.Structure):
     ]
 
 
+class QuantizeFp8Params(C.Structure):
+    _fields_ = [
+        ("x", Tensor4), ("x8", C.c_void_p), ("scale", C.c_void_p),
+        ("B", C.c_int32), ("H", C.c_int32), ("T", C.c_int32), ("D", C.c_int32), ("dtype", C.c_int32),
+    ]
+
+
 class QkvProjParams(C.Structure):
     _fields_ = [
         ("x", C.c_void_p), ("w", C.c_void_p), ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p),
@@ -134,6 +141,8 @@ def load() -> C.CDLL:
     lib.kb_sa_bwd.argtypes = [C.POINTER(SaBwdParams), C.c_void_p]
     lib.kb_sa_fwd_fp8.argtypes = [C.POINTER(SaFwdFp8Params), C.c_void_p]
     lib.kb_sa_fwd_fp8.restype = C.c_int
+    lib.kb_quantize_fp8.argtypes = [C.POINTER(QuantizeFp8Params), C.c_void_p]
+    lib.kb_quantize_fp8.restype = C.c_int
     lib.kb_sa_bwd_noalloc.argtypes = [C.POINTER(SaBwdParams), C.c_void_p]
     lib.kb_sa_bwd_noalloc.restype = C.c_int
     lib.kb_sa_fwd_varlen.argtypes = [C.POINTER(SaVarlenParams), C.c_void_p]
@@ -186,6 +195,19 @@ def tensor4(t: torch.Tensor) -> Tensor4:
     for i in range(4):
         out.stride[i] = t.stride(i)
     return out
+
+
+def plain_call(*tensors) -> bool:
+    """Whether a call on these tensors is ordinary eager execution on a GPU: nothing traces, transforms or intercepts
+    it (compilation, functorch transforms, forward-mode AD, saved-tensor hooks, dispatch or function modes, tensor
+    subclasses).  Entry points that have a shorter way for such calls ask this and leave everything else as it is."""
+    return (
+        not torch.compiler.is_compiling()
+        and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda for t in tensors)
+        and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+        and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+        and torch._C._autograd._top_saved_tensors_default_hooks(True) is None
+    )
 
 
 def launch_count() -> int:

@@ -392,6 +392,13 @@ uint64_t kb_sa_bwd_varlen_workspace_bytes(int32_t B, int32_t H, int32_t total_ro
   return 0;
 }
 
+int kb_quantize_fp8(const kb_quantize_fp8_params* p, void* stream) {
+  if (!p || p->B < 0 || p->H < 0 || p->T < 0 || p->D < 0) return KB_ERR_BAD_ARGUMENT;
+  if (p->B == 0 || p->H == 0 || p->T == 0) return KB_OK;
+  if (!p->x.data || !p->x8 || !p->scale) return KB_ERR_BAD_ARGUMENT;
+  return kb::quantize_fp8(*p, static_cast<cudaStream_t>(stream));
+}
+
 int kb_softmax_fwd(const kb_softmax_params* p, void* stream) {
   if (!p || p->rows < 0 || p->cols < 0) return KB_ERR_BAD_ARGUMENT;
   if (!kb::dtype_ok(p->dtype)) return KB_ERR_UNSUPPORTED;

@@ -12,6 +12,7 @@ import pytest
 import torch
 
 from kernels_b200 import _lib
+from kernels_b200.streaming_attention import quantize_fp8_tiles
 from oracle import streaming_attention_oracle as SO
 
 pytestmark = pytest.mark.gpu
@@ -91,3 +92,41 @@ def test_fp8_forward_rejects_what_the_kernel_does_not_take():
     assert lib.kb_sa_fwd_fp8(ctypes.byref(p), None) == _lib.KB_ERR_UNSUPPORTED  # fp32 output
     p.out_dtype, p.H_kv = _lib.KB_BF16, 3
     assert lib.kb_sa_fwd_fp8(ctypes.byref(p), None) == 1
+
+
+def _quantize_expressions(x):
+    """The definition as tensor expressions (every step of it rounds the way the kernel has to)."""
+    B, H, T, D = x.shape
+    n = -(-T // 128)
+    xf = torch.nn.functional.pad(x.float(), (0, 0, 0, n * 128 - T))
+    tiles = xf.view(B, H, n, 128, D)
+    scale = (tiles.abs().amax(dim=(-1, -2)) / 448.0).clamp_min(1e-12)
+    return (tiles / scale[..., None, None]).view(B, H, n * 128, D)[:, :, :T].to(torch.float8_e4m3fn), scale
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,H,T,order", [(1, 1, 1, "bhtd"), (2, 3, 127, "bthd"), (1, 2, 128, "bhtd"), (2, 2, 129, "bthd"), (1, 5, 1000, "bhtd"),
+                                         (3, 1, 300, "odd")])
+def test_quantize_gives_the_expressions_bytes(dtype, B, H, T, order):
+    """Both sides are the same fp32 operations, so bytes and scales are equal; "odd" rows start off a 16-byte
+    boundary and take the expressions themselves."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    shape = (B, T, H, 128) if order == "bthd" else (B, H, T, 128)
+    if order == "odd":
+        x = torch.randn(B * H * T * 128 + 1, generator=g, device="cuda").to(dtype)[1:].view(shape)
+    else:
+        x = torch.randn(shape, generator=g, device="cuda").to(dtype)
+        x = x.transpose(1, 2) if order == "bthd" else x
+    with torch.no_grad():
+        tile = x[0, 0, :min(T, 100)]
+        tile.mul_(0)  # an all-zero (part of a) tile: scale 1e-12 if nothing else is in it
+        if T > 128:  # special values in a tile of their own
+            x[-1, -1, -1, :3] = torch.tensor([float("nan"), float("inf"), -float("inf")])
+            x[0, -1, 128:, ::7] = -0.0
+    before = _lib.launch_count()
+    x8, scale = quantize_fp8_tiles(x)
+    assert _lib.launch_count() - before == (0 if order == "odd" else 1)
+    want8, want_scale = _quantize_expressions(x)
+    assert x8.is_contiguous() and scale.is_contiguous() and x8.shape == x.shape
+    assert torch.equal(x8.view(torch.uint8), want8.contiguous().view(torch.uint8))
+    assert torch.equal(scale.nan_to_num(-1.0), want_scale.nan_to_num(-1.0))
