@@ -164,3 +164,35 @@ def test_softmax_many_calls_side_stream_poisoned_output():
     assert float(err.max()) <= 1e-6, (
         f"softmax call {i} row {r} col {c}: got {float(got[i, r, c])!r}, oracle {float(ref[i, r, c])!r}, "
         f"|err| {float(err.max()):.3e}; {int((err > 1e-6).sum())} elements off, {int(torch.isnan(got).sum())} never written")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("cols", [1, 7, 15, 129, 1003, 2055, 5001, 16390, 20000, 32773])
+@pytest.mark.parametrize("start", [0, 1, 5])
+def test_softmax_rows_off_16_byte_boundaries(dtype, cols, start):
+    """Odd row lengths and first rows off a boundary, against the 64-bit result: fp32 to 1e-6 absolute (results are
+    at most 1), 16-bit to half a unit in the last place of the result (plus that fp32 error).  Nothing outside the
+    rows is written; an infinity, a NaN and a row of only -inf come out as the tensor expressions give them."""
+    from kernels_b200 import _lib
+
+    import ctypes
+
+    rows = 9
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = (torch.randn(rows * cols + start, generator=g, device="cuda") * 2.0).to(dtype)
+    xv = x[start:].view(rows, cols)
+    xv[1] = -float("inf")
+    xv[2, cols // 2] = float("inf")
+    xv[3, cols - 1] = float("nan")
+    xv[4, 0] = -float("inf") if cols > 1 else 0.0
+    y = torch.full((rows * cols + start + 16,), 7.0, dtype=dtype, device="cuda")
+    p = _lib.SoftmaxParams()
+    p.x, p.y = xv.data_ptr(), y[start:].data_ptr()
+    p.rows, p.cols, p.x_row_stride, p.y_row_stride, p.dtype = rows, cols, cols, cols, _lib.dtype_code(dtype)
+    _lib.check(_lib.load().kb_softmax_fwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream), "kb_softmax_fwd")
+    got, want = y[start:start + rows * cols].view(rows, cols), torch.softmax(xv.double(), dim=-1)
+    assert (y[:start] == 7).all() and (y[start + rows * cols:] == 7).all()
+    half_ulp = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    assert torch.equal(got.isnan(), want.isnan())
+    err = (got.double() - want).nan_to_num(0.0).abs()
+    assert (err <= 1e-6 + half_ulp * want.nan_to_num(0.0)).all(), float(err.max())
