@@ -652,7 +652,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           const int c0 = y0 + cc * 32;
-          const bool all_dead = !warp_full && __all_sync(0xffffffffu, c0 + 32 <= lo || c0 >= hi);
+          const uint32_t live = warp_full ? ~0u : live_word(c0, lo, hi);
+          const bool all_dead = !warp_full && __all_sync(0xffffffffu, live == 0u);
           if (all_dead) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) p[cc * 32 + i] = 0.f;
@@ -666,9 +667,9 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             p[i + 2] = ex2_approx(fmaf(__uint_as_float(s[i + 2]), scale, -lv.z));
             p[i + 3] = ex2_approx(fmaf(__uint_as_float(s[i + 3]), scale, -lv.w));
           }
-          if (!warp_full && !__all_sync(0xffffffffu, lo <= c0 && c0 + 32 <= hi)) {
+          if (!warp_full && !__all_sync(0xffffffffu, live == ~0u)) {
 #pragma unroll
-            for (int i = cc * 32; i < cc * 32 + 32; ++i) p[i] = (y0 + i >= lo && y0 + i < hi) ? p[i] : 0.f;
+            for (int i = 0; i < 32; ++i) p[cc * 32 + i] = (live & (1u << i)) ? p[cc * 32 + i] : 0.f;
           }
         }
       }

@@ -108,12 +108,27 @@ struct alignas(1024) FwdSmem {
 enum WaitSite { kWaitQ = 1, kWaitQEmpty, kWaitOFree, kWaitKEmpty, kWaitVEmpty, kWaitKFull, kWaitVFull, kWaitSReady, kWaitPReady, kWaitEpilogue };
 constexpr int kErrSmemAlign = 11;
 
+// Which of the 32 columns from c0 on lie in the row's live interval [lo, hi).  WORD: as the bits of one word (half the
+// instructions per element); otherwise two compares per element.  Words everywhere but in the straight-line instance
+// for head dim 128, whose items are masked at sequence ends only and whose code the words make slower (bf16 c=256
+// T=16384 without lengths: 888 us with compares, 919 with words; 8-bit: 215 / 241; while
+// c=64 T=8192: 895 / 811 us, fp16 D=64 c=10: 340 / 270, dense D=64 with lengths: 434 / 399).
+template <bool WORD>
+struct LiveCols {
+  uint32_t word;
+  int c0, lo, hi;
+  __device__ __forceinline__ LiveCols(int c0_, int lo_, int hi_) : word(WORD ? live_word(c0_, lo_, hi_) : 0u), c0(c0_), lo(lo_), hi(hi_) {}
+  __device__ __forceinline__ bool all() const { return WORD ? word == ~0u : (lo <= c0 && c0 + 32 <= hi); }
+  __device__ __forceinline__ bool none() const { return WORD ? word == 0u : (c0 + 32 <= lo || c0 >= hi); }
+  __device__ __forceinline__ bool operator[](int i) const { return WORD ? (word & (1u << i)) != 0 : (c0 + i >= lo && c0 + i < hi); }
+};
+
 // One 128 x 128 block of scores for the thread's row, in two passes over the row in TMEM, 64 columns at a
 // time, so that at most 64 scores are live in registers (holding all 128 leaves the softmax warps no register to
 // spare at the 168 the launch gives them, and every spill sits on the kernel's critical chain).
 // Pass 1 (softmax_row_max): the row maximum of the masked scores.  kMasked = false is the fast path for blocks
 // in which every element of the warp's rows is live.
-template <bool kMasked>
+template <bool kMasked, bool WORD>
 __device__ __forceinline__ float softmax_row_max(uint32_t t_s, int k0, int lo, int hi) {
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -127,8 +142,9 @@ __device__ __forceinline__ float softmax_row_max(uint32_t t_s, int k0, int lo, i
       const int c0 = k0 + half * 64 + cc * 32;
       // a 32-column group that is live for every row of the warp needs no select, one that is masked for every
       // row contributes nothing (chunk boundaries that are multiples of 32 never leave a mixed group)
-      const bool all_live = !kMasked || __all_sync(0xffffffffu, lo <= c0 && c0 + 32 <= hi);
-      const bool all_dead = kMasked && __all_sync(0xffffffffu, c0 + 32 <= lo || c0 >= hi);
+      const LiveCols<WORD> live(c0, lo, hi);
+      const bool all_live = !kMasked || __all_sync(0xffffffffu, live.all());
+      const bool all_dead = kMasked && __all_sync(0xffffffffu, live.none());
       if (all_dead) continue;
       // 3-input max: two scores per instruction
 #pragma unroll
@@ -138,8 +154,8 @@ __device__ __forceinline__ float softmax_row_max(uint32_t t_s, int k0, int lo, i
           const int j = cc * 32 + i + 2 * e;
           float a = __uint_as_float(s[j]), b = __uint_as_float(s[j + 1]);
           if (!all_live) {
-            a = (c0 + i + 2 * e >= lo && c0 + i + 2 * e < hi) ? a : -INFINITY;
-            b = (c0 + i + 2 * e + 1 >= lo && c0 + i + 2 * e + 1 < hi) ? b : -INFINITY;
+            a = live[i + 2 * e] ? a : -INFINITY;
+            b = live[i + 2 * e + 1] ? b : -INFINITY;
           }
           mx[e] = fmax3(mx[e], a, b);
         }
@@ -153,7 +169,7 @@ __device__ __forceinline__ float softmax_row_max(uint32_t t_s, int k0, int lo, i
 // into TMEM over S (P of columns 32 j .. 32 j + 31 lands on columns 16 j .. 16 j + 15: the second half of P
 // overwrites only scores of the first half, which are in registers by then); the row sum goes into `sum`.
 // FP8: P is written as e4m3, four values per TMEM column (64 keys = 16 columns at 16 half), for the 8-bit P V.
-template <bool BF16, bool kMasked, bool FP8>
+template <bool BF16, bool kMasked, bool FP8, bool WORD>
 __device__ __forceinline__ void softmax_exp_half(uint32_t t_s, int half, float scale, float m_used, int k0, int lo, int hi,
                                                  float (&sum)[4]) {
   const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
@@ -167,8 +183,9 @@ __device__ __forceinline__ void softmax_exp_half(uint32_t t_s, int half, float s
 #pragma unroll
   for (int cc = 0; cc < 2; ++cc) {
     const int c0 = k0 + half * 64 + cc * 32;
-    const bool all_live = !kMasked || __all_sync(0xffffffffu, lo <= c0 && c0 + 32 <= hi);
-    const bool all_dead = kMasked && __all_sync(0xffffffffu, c0 + 32 <= lo || c0 >= hi);
+    const LiveCols<WORD> live(c0, lo, hi);
+    const bool all_live = !kMasked || __all_sync(0xffffffffu, live.all());
+    const bool all_dead = kMasked && __all_sync(0xffffffffu, live.none());
     uint32_t pk[16];
     if (all_dead) {
 #pragma unroll
@@ -182,8 +199,8 @@ __device__ __forceinline__ void softmax_exp_half(uint32_t t_s, int half, float s
     for (int i = 0; i < 16; ++i) {
       float s0 = __uint_as_float(s[cc * 32 + 2 * i]), s1 = __uint_as_float(s[cc * 32 + 2 * i + 1]);
       if (!all_live) {
-        s0 = (c0 + 2 * i >= lo && c0 + 2 * i < hi) ? s0 : -INFINITY;
-        s1 = (c0 + 2 * i + 1 >= lo && c0 + 2 * i + 1 < hi) ? s1 : -INFINITY;
+        s0 = live[2 * i] ? s0 : -INFINITY;
+        s1 = live[2 * i + 1] ? s1 : -INFINITY;
       }
       const uint64_t x = f2_fma(f2_pack(s0, s1), scale2, negm2);
       float x0, x1;
@@ -223,12 +240,13 @@ __device__ __forceinline__ float softmax_load_row_max(uint32_t t_s, uint32_t (&s
 #pragma unroll
   for (int cc = 0; cc < kBN / 32; ++cc) {
     const int c0 = k0 + cc * 32;
-    const bool all_live = !kMasked || __all_sync(0xffffffffu, lo <= c0 && c0 + 32 <= hi);
-    dead[cc] = kMasked && __all_sync(0xffffffffu, c0 + 32 <= lo || c0 >= hi);
+    const LiveCols<true> live(c0, lo, hi);
+    const bool all_live = !kMasked || __all_sync(0xffffffffu, live.all());
+    dead[cc] = kMasked && __all_sync(0xffffffffu, live.none());
     if (dead[cc]) continue;
     if (!all_live) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) s[cc * 32 + i] = (c0 + i >= lo && c0 + i < hi) ? s[cc * 32 + i] : 0xff800000u;  // -inf
+      for (int i = 0; i < 32; ++i) s[cc * 32 + i] = live[i] ? s[cc * 32 + i] : 0xff800000u;  // -inf
     }
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
@@ -651,6 +669,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         KB_FACC(1);
         const bool warp_full = __all_sync(0xffffffffu, lo <= k0 && k0 + kBN <= hi);
+        constexpr bool kWord = !FAST;
         constexpr bool kHold = (D == 64) && !FP8;  // one pass with the row's scores held in registers
         uint32_t s_held[kHold ? kBN : 1];
         bool dead_held[kBN / 32];
@@ -659,7 +678,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           row_max = warp_full ? softmax_load_row_max<false>(t_s, reinterpret_cast<uint32_t(&)[kBN]>(s_held), dead_held, k0, lo, hi)
                               : softmax_load_row_max<true>(t_s, reinterpret_cast<uint32_t(&)[kBN]>(s_held), dead_held, k0, lo, hi);
         } else {
-          row_max = warp_full ? softmax_row_max<false>(t_s, k0, lo, hi) : softmax_row_max<true>(t_s, k0, lo, hi);
+          row_max = warp_full ? softmax_row_max<false, kWord>(t_s, k0, lo, hi) : softmax_row_max<true, kWord>(t_s, k0, lo, hi);
         }
         const float m_new = fmaxf(m_used, row_max * scale);
         // lazy rescale: keep the old reference maximum unless the new one is larger by more than the threshold
@@ -678,10 +697,10 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           if (warp_full) softmax_exp_held<BF16, false>(t_s, reinterpret_cast<const uint32_t(&)[kBN]>(s_held), dead_held, scale, m_exp, sum);
           else softmax_exp_held<BF16, true>(t_s, reinterpret_cast<const uint32_t(&)[kBN]>(s_held), dead_held, scale, m_exp, sum);
         } else {
-          if (warp_full) softmax_exp_half<BF16, false, FP8>(t_s, 0, scale, m_exp, k0, lo, hi, sum);
-          else softmax_exp_half<BF16, true, FP8>(t_s, 0, scale, m_exp, k0, lo, hi, sum);
-          if (warp_full) softmax_exp_half<BF16, false, FP8>(t_s, 1, scale, m_exp, k0, lo, hi, sum);
-          else softmax_exp_half<BF16, true, FP8>(t_s, 1, scale, m_exp, k0, lo, hi, sum);
+          if (warp_full) softmax_exp_half<BF16, false, FP8, kWord>(t_s, 0, scale, m_exp, k0, lo, hi, sum);
+          else softmax_exp_half<BF16, true, FP8, kWord>(t_s, 0, scale, m_exp, k0, lo, hi, sum);
+          if (warp_full) softmax_exp_half<BF16, false, FP8, kWord>(t_s, 1, scale, m_exp, k0, lo, hi, sum);
+          else softmax_exp_half<BF16, true, FP8, kWord>(t_s, 1, scale, m_exp, k0, lo, hi, sum);
         }
         // the rescale of O comes after the exponentials: the row's scores are dead by now, which keeps the
         // registers of the two from being live together

@@ -379,6 +379,16 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+// ---- masks -------------------------------------------------------------------------------
+// Bit j: whether column c0 + j lies in [lo, hi).  Selecting by a constant bit of one word costs half of two compares
+// per element.  (PTX shifts clamp: an amount of 32 or more gives 0.)
+__device__ __forceinline__ uint32_t live_word(int c0, int lo, int hi) {
+  uint32_t from_lo, from_hi;
+  asm("shl.b32 %0, %1, %2;" : "=r"(from_lo) : "r"(~0u), "r"(max(lo - c0, 0)));
+  asm("shl.b32 %0, %1, %2;" : "=r"(from_hi) : "r"(~0u), "r"(max(hi - c0, 0)));
+  return from_lo & ~from_hi;
+}
+
 // ---- small math helpers ------------------------------------------------------------------
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
