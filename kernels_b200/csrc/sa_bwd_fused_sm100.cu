@@ -106,6 +106,7 @@ struct FusedArgs {
   const int32_t* cu;
   int32_t total, n_ptiles;
   KbFastDiv fd_tiles, fd_H, fd_Hk, fd_group, fd_c;  // division by ceil(T / 128), H, Hk, group and c
+  int32_t item_rot, item_rot_dq;  // main / dQ kernel, see KbItemWalk
   float scale_log2, sm_scale;
   int32_t* status;
 };
@@ -157,7 +158,8 @@ struct Item {
 // The tiles of an item: for every query head of the key/value head's group (hq = 0 .. group - 1), the
 // query tiles of `qr` (tq = 0 ..); t is the running index over both.
 struct Cursor {
-  int item, n, g, t, tq, hq, group;
+  KbItemWalk<> walk;
+  int n, g, t, tq, hq, group;
   Item it;
   bool valid;
   __device__ __forceinline__ int q_tiles() const { return it.qr.end - it.qr.begin; }
@@ -196,12 +198,12 @@ __device__ __forceinline__ Item decode_item(const FusedArgs& a, int item, int n_
 // row0 and is b-th in the batch; floor(row0 / 128) + b + kt is unique per (b, kt) and below
 // floor(total / 128) + B + 1 (a sequence ends at most one tile later than its rows alone would need).
 __device__ __forceinline__ int ptile_id(int row0, int b, int kt) { return (row0 >> 7) + b + kt; }
-// first live item at or after `item` (stride gridDim.x)
+// first live item from the walk's position on
 template <bool PACKED>
 __device__ __forceinline__ void seek_live(const FusedArgs& a, Cursor& c, int n_items, int n_ktiles) {
   c.valid = false;
-  for (; c.item < n_items; c.item += gridDim.x) {
-    c.it = decode_item<PACKED>(a, c.item, n_ktiles, c.it);
+  for (; c.walk.item() < n_items; c.walk.next()) {
+    c.it = decode_item<PACKED>(a, c.walk.item(), n_ktiles, c.it);
     if (c.it.qr.begin < c.it.qr.end) {
       c.valid = true;
       return;
@@ -210,8 +212,7 @@ __device__ __forceinline__ void seek_live(const FusedArgs& a, Cursor& c, int n_i
 }
 template <bool PACKED>
 __device__ __forceinline__ Cursor cursor_first(const FusedArgs& a, int n_items, int n_ktiles) {
-  Cursor c;
-  c.item = blockIdx.x;
+  Cursor c{KbItemWalk<>(a.item_rot)};
   c.n = c.g = c.t = c.tq = c.hq = 0;
   c.group = a.group;
   c.it.b = -1;
@@ -228,7 +229,7 @@ __device__ __forceinline__ void cursor_next(const FusedArgs& a, Cursor& c, int n
   c.hq = 0;
   c.t = 0;
   ++c.n;
-  c.item += gridDim.x;
+  c.walk.next();
   seek_live<PACKED>(a, c, n_items, n_ktiles);
 }
 // `h` is the QUERY head, `row0` the sequence's first row (packed batch only)
@@ -454,19 +455,19 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         }
       };
       // This thread keeps no cursor: all it needs of the schedule is how many tiles each live item has.
-      // Tiles of the first live item at or after `item` (stride gridDim.x), 0 if there is none.
-      auto next_live = [&](int& item) -> int {
+      // Tiles of the first live item from the walk's position on, 0 if there is none.
+      auto next_live = [&](KbItemWalk<>& walk) -> int {
         Item prev;
         prev.b = -1;
-        for (; item < n_items; item += gridDim.x) {
-          const Item it = decode_item<PACKED>(a, item, n_ktiles, prev);
+        for (; walk.item() < n_items; walk.next()) {
+          const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles, prev);
           if (it.qr.begin < it.qr.end) return (it.qr.end - it.qr.begin) * a.group;
         }
         return 0;
       };
 
-      int item = blockIdx.x;
-      int cnt = next_live(item);  // tiles of the current item
+      KbItemWalk<> walk(a.item_rot);
+      int cnt = next_live(walk);  // tiles of the current item
       int n = 0, g = 0;           // live items, tiles so far
       bool ok = cnt > 0 && issue_s(0, 0, true) && issue_dp(0, 0, true, cnt == 1);
       KB_ACC(11);
@@ -495,8 +496,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           // S(g+1): of this item, or the first of the next live one.  (Looking for the next item before the wait for
           // P instead, off the chain, as the other classes' loop below does, measured 1 % slower in this one.)
           if (last) {
-            item += gridDim.x;
-            cnt_next = next_live(item);
+            walk.next();
+            cnt_next = next_live(walk);
           }
           const bool more = !last || cnt_next > 0;
           if (more && !issue_s(last ? n + 1 : n, g + 1, last)) return false;
@@ -543,8 +544,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             // The look for the next live item (a decode per candidate) is done here, before the wait for P: from
             // that wait to the issue of S(g+1) the thread is on the kernel's critical chain.
             if (last) {
-              item += gridDim.x;
-              cnt_next = next_live(item);
+              walk.next();
+              cnt_next = next_live(walk);
             }
             const bool more = !last || cnt_next > 0;
             const int n_next = last ? n + 1 : n;                           // item of tile g + 1
@@ -733,8 +734,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     bool ok = true;
     Item it = {};
     it.b = -1;
-    for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-      it = decode_item<PACKED>(a, item, n_ktiles, it);
+    for (KbItemWalk<> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
+      it = decode_item<PACKED>(a, walk.item(), n_ktiles, it);
       const int kr = it.k0 + row;
       if (it.qr.begin >= it.qr.end) {
         // the whole key tile lies in the padding: its gradients are zeros (rare; plain stores).  A packed
@@ -988,8 +989,8 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       bool ok = true;
       DqItem it = {};
       it.b = -1;
-      for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-        it = decode_dq_item<PACKED>(a, item, n_tiles_t, it);
+      for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
+        it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t, it);
         for (int j = it.kr.begin; j < it.kr.end; ++j, ++u) {
           const int s = u % kDqStages;
           if (u >= kDqStages && !mbar_wait<kRelaxedNs>(&sm.empty[s], ((u / kDqStages) - 1) & 1, ctx, kWDqEmpty)) { ok = false; break; }
@@ -1010,8 +1011,8 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       bool ok = true;
       DqItem it = {};
       it.b = -1;
-      for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-        it = decode_dq_item<PACKED>(a, item, n_tiles_t, it);
+      for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
+        it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t, it);
         if (it.kr.begin >= it.kr.end) continue;
         const uint32_t acc = tmem + (m & 1) * 128;
         if (m >= 2 && !mbar_wait(&sm.acc_free[m & 1], ((m >> 1) - 1) & 1, ctx, kWDqAccFree)) break;
@@ -1039,8 +1040,8 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     bool ok = true;
     DqItem it = {};
     it.b = -1;
-    for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-      it = decode_dq_item<PACKED>(a, item, n_tiles_t, it);
+    for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
+      it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t, it);
       const int qi = it.qt * kBQ + row;
       if (it.kr.begin >= it.kr.end) {
         // the whole query tile lies in the padding: its gradient is zero (rare; plain stores); a packed batch
@@ -1197,6 +1198,8 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.fd_c = kb_fastdiv_make(c);
   fa.scale_log2 = p.sm_scale * kLog2e;
   fa.sm_scale = p.sm_scale;
+  fa.item_rot = kb_item_rotation((int32_t)grid_main, n_tiles, p.lens || PACKED);
+  fa.item_rot_dq = kb_item_rotation((int32_t)grid, n_tiles, p.lens || PACKED);
   fa.status = p.status;
   if (!(p.flags & KB_FLAG_BWD_SKIP_DKDV)) {
     main_kern<<<grid_main, kThreads, sizeof(FusedSmem<D>), s>>>(tm_k, tm_v, tm_q, tm_do, tm_dk, tm_dv, fa);

@@ -20,7 +20,7 @@
 // O_A at 256, O_B at 384.  One CTA per SM.
 //
 // The kernel is persistent: the grid is one CTA per SM and every CTA walks the work items
-// (batch, head, 256-row q block) item = blockIdx.x, blockIdx.x + gridDim.x, ...  Barriers and
+// (batch, head, 256-row q block) in the order of KbItemWalk (schedule.h).  Barriers and
 // TMEM are set up once; the producer runs ahead into the next item (its Q is loaded as soon as
 // the last S of the current item has been issued) and the softmax warps write the current
 // item's O while the MMAs of the next one already run, so the pipeline is not drained and
@@ -82,6 +82,7 @@ struct FwdArgs {
   // extent is 1, o_sb = lse_sb = 0) and T is the longest sequence.  NULL: the padded layout.
   const int32_t* cu;
   KbFastDiv fd_qblocks, fd_H, fd_c, fd_group;  // division by ceil(T / 256), H, c and H / H_kv (query heads per K/V head)
+  int32_t item_rot;  // see KbItemWalk
   float scale_log2;
   int32_t* status;
   // 8-bit (e4m3) inputs only: one dequantisation scale per tile of 128 rows of q [B, H, n128], k and v
@@ -383,8 +384,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       prefetch_tensormap(&tm_v);
       int kc = 0, vc = 0, na = 0;
       bool ok = true;
-      for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-        const Item it = decode(item);
+      for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
+        const Item it = decode(walk.item());
         if (!it.act[0] && !it.act[1]) continue;
         // the Q buffers are free once every S of the previous item has been issued and has run
         if (na > 0 && !mbar_wait(&sm.q_empty, (na - 1) & 1, ctx, kWaitQEmpty)) break;
@@ -425,8 +426,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       long long acc_t[10] = {0};
       long long tl = clock64();
 #endif
-      for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-        const Item it = decode(item);
+      for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
+        const Item it = decode(walk.item());
         if (!it.act[0] && !it.act[1]) continue;
         KB_FACC(0);
         if (!mbar_wait(&sm.q_full, na & 1, ctx, kWaitQ)) break;
@@ -615,8 +616,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     long long acc_t[8] = {0};
     long long tl = clock64();
 #endif
-    for (int item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-      const Item it = decode(item);
+    for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
+      const Item it = decode(walk.item());
       const int qi = it.q0 + x * kBM + row;
       const int orow = it.row0 + qi - a.q_start;  // this thread's row of o and lse
       uint16_t* o_row = static_cast<uint16_t*>(a.o) + it.b * a.o_sb + it.h * a.o_sh + orow * a.o_st;
@@ -861,6 +862,7 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   const int64_t n_items = (int64_t)p.B * p.H * kb_cdiv_i32(Tq, kBM * kQTiles);
   if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
   const unsigned grid = (unsigned)(n_items < n_sm ? n_items : n_sm);  // persistent: one CTA per SM
+  a.item_rot = kb_item_rotation((int32_t)grid, kb_cdiv_i32(Tq, kBM * kQTiles), p.lens || p.cu_seqlens);
   kern<<<grid, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
   KB_LAUNCH_CHECK("sa_fwd_sm100_kernel");
   return KB_OK;

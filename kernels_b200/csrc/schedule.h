@@ -86,6 +86,49 @@ KB_HD int32_t kb_fastdiv(int32_t n, const KbFastDiv& f) {
   return (int32_t)((hi + (uint32_t)n) >> f.shift);
 }
 
+// The order in which the CTAs of a persistent kernel take the work items.  Wave w hands out the items
+// [w G, (w + 1) G) (G = CTAs): neighbouring items run at the same time and share their K / V rows in L2.  Inside a
+// wave CTA x takes number (x + w r) mod G.  An item's place in its sequence is item mod n (n = items per sequence and
+// head); with r = 0 a CTA meets only n / gcd(G, n) of the places.  Where sequences differ in length the late places are
+// often padding, and with few places per CTA some CTAs get much more work than others (n = 4, G = 148: CTA 0 only the
+// first quarter of every sequence).  r > 0 makes G + r and n coprime, which spreads the places.
+//
+// Only where the lengths differ and a CTA would meet at most four places.  Measured (B200, r = 0 / r = 1): packed batch
+// of 256 sequences of 128-1024 rows, forward 951 / 843 us, main backward kernel 1286 / 1081, dQ 497 / 402; fp16 D=64
+// c=10 T=1353 (n = 6, three places) forward 261 / 235 us.  With eight and more places nothing is gained, and an odd r
+// separates the CTAs of an SM pair from the two key tiles of one chunk, whose common Q / dO tiles the pair fetches
+// together: main kernel, bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r.
+inline int32_t kb_gcd(int32_t a, int32_t b) {
+  while (b) {
+    const int32_t t = a % b;
+    a = b;
+    b = t;
+  }
+  return a;
+}
+inline int32_t kb_item_rotation(int32_t ctas, int32_t items_per_seq, bool ragged) {
+  const int32_t n = items_per_seq;
+  if (!ragged || ctas < 1 || n < 1 || n / kb_gcd(ctas, n) > 4) return 0;
+  int32_t r = 0;
+  while (kb_gcd(ctas + r, n) != 1) ++r;  // among n consecutive numbers one is coprime to n
+  return r % ctas;
+}
+#if defined(__CUDACC__)
+// ROT = false: r = 0 known at compile time.
+template <bool ROT = true>
+struct KbItemWalk {
+  int32_t base, off, rot;
+  __device__ __forceinline__ explicit KbItemWalk(int32_t rotation) : base(0), off((int32_t)blockIdx.x), rot(rotation) {}
+  __device__ __forceinline__ int32_t item() const { return base + off; }  // the walk ends at the first item() >= n_items
+  __device__ __forceinline__ void next() {
+    base += (int32_t)gridDim.x;
+    if (!ROT) return;
+    off += rot;
+    if (off >= (int32_t)gridDim.x) off -= (int32_t)gridDim.x;
+  }
+};
+#endif
+
 // The two tile ranges above with the divisions by the chunk length done by kb_fastdiv (same
 // results; the persistent kernels call these).
 KB_HD KbTileRange kb_fwd_kv_range_fd(int32_t q0, int32_t tile_q, int32_t tile_k, int32_t len, int32_t c,
