@@ -190,11 +190,21 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def tensor4(t: torch.Tensor) -> Tensor4:
-    out = Tensor4()
-    out.data = t.data_ptr()
-    for i in range(4):
-        out.stride[i] = t.stride(i)
-    return out
+    strides = t.stride()
+    if len(strides) < 4:
+        raise IndexError(f"a four-dimensional tensor is needed, got {len(strides)} dimensions")
+    return Tensor4(t.data_ptr(), strides[:4])
+
+
+def launch(entry, params, device: torch.device) -> int:
+    """``entry(&params, stream)`` on ``device`` and its current stream; the status code.  The device is only switched
+    where it is not current already, and the stream is asked for as the handle it is needed as: a few microseconds of
+    calls that take about twenty."""
+    index = device.index
+    if index == torch._C._cuda_getDevice():
+        return entry(C.byref(params), torch._C._cuda_getCurrentRawStream(index))
+    with torch.cuda.device(device):
+        return entry(C.byref(params), torch.cuda.current_stream(device).cuda_stream)
 
 
 def plain_call(*tensors) -> bool:

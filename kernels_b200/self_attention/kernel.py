@@ -9,7 +9,6 @@ as in the reference.  There is no CPU or eager fallback.
 
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -53,9 +52,7 @@ def attention_forward_adapter(
     p.flags = _lib.KB_FLAG_PRESCALE_QK if prescale else 0
     p.status = _lib.status_words().data_ptr()
     lib = _lib.load()
-    with torch.cuda.device(q.device):
-        rc = lib.kb_fa_fwd(ctypes.byref(p), torch.cuda.current_stream(q.device).cuda_stream)
-    _lib.check(rc, "kb_fa_fwd")
+    _lib.check(_lib.launch(lib.kb_fa_fwd, p, q.device), "kb_fa_fwd")
     return O
 
 

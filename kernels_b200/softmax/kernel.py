@@ -7,8 +7,6 @@ There is no CPU or eager fallback.
 
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from .. import _lib
@@ -30,9 +28,7 @@ def softmax(x: torch.Tensor) -> torch.Tensor:
     p.x_row_stride, p.y_row_stride = x2.stride(0) if rows else cols, cols
     p.dtype = _lib.dtype_code(x.dtype)
     lib = _lib.load()
-    with torch.cuda.device(x.device):
-        rc = lib.kb_softmax_fwd(ctypes.byref(p), torch.cuda.current_stream(x.device).cuda_stream)
-    _lib.check(rc, "kb_softmax_fwd")
+    _lib.check(_lib.launch(lib.kb_softmax_fwd, p, x.device), "kb_softmax_fwd")
     return y.view(*shape)
 
 

@@ -11,7 +11,6 @@ fp16 or bf16.  Forward only (inference); head_dim 128.  There is no other path: 
 
 from __future__ import annotations
 
-import ctypes
 import math
 from typing import Optional
 
@@ -49,8 +48,7 @@ def quantize_fp8_tiles(x: torch.Tensor):
         p.x, p.x8, p.scale = _lib.tensor4(x), x8.data_ptr(), scale.data_ptr()
         p.B, p.H, p.T, p.D = B, H, T, D
         p.dtype = _lib.dtype_code(x.dtype)
-        with torch.cuda.device(x.device):
-            rc = _lib.load().kb_quantize_fp8(ctypes.byref(p), torch.cuda.current_stream(x.device).cuda_stream)
+        rc = _lib.launch(_lib.load().kb_quantize_fp8, p, x.device)
         if rc != _lib.KB_ERR_UNSUPPORTED:
             _lib.check(rc, "kb_quantize_fp8")
             return x8, scale
@@ -107,8 +105,6 @@ def streaming_attention_fp8(
     p.sm_scale = float(sm_scale)
     p.flags = 0
     p.status = _lib.status_words().data_ptr()
-    with torch.cuda.device(q8.device):
-        rc = _lib.load().kb_sa_fwd_fp8(ctypes.byref(p), torch.cuda.current_stream(q8.device).cuda_stream)
-    _lib.check(rc, "kb_sa_fwd_fp8")
+    _lib.check(_lib.launch(_lib.load().kb_sa_fwd_fp8, p, q8.device), "kb_sa_fwd_fp8")
     del lens_keep
     return (o, lse) if return_lse else o

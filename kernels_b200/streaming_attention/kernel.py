@@ -14,7 +14,6 @@ chunk and of the ``back_contexts`` chunks before it, and only to positions ``< l
 
 from __future__ import annotations
 
-import ctypes
 import logging
 from typing import Optional
 
@@ -140,14 +139,12 @@ def attention_forward_adapter(
     p.flags = _flags(prescale_qk, precision)
     p.status = _lib.status_words().data_ptr()
     p.H_kv = k.shape[1]
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        rc = lib.kb_sa_fwd(ctypes.byref(p), stream)
-        if rc == _lib.KB_ERR_UNSUPPORTED and k.shape[1] != H:
-            # no kernel with shared key/value heads for this dtype / head_dim / layout: repeat the heads
-            k_rep, v_rep = (t.repeat_interleave(H // t.shape[1], dim=1) for t in (k, v))
-            p.k, p.v, p.H_kv = _lib.tensor4(k_rep), _lib.tensor4(v_rep), H
-            rc = lib.kb_sa_fwd(ctypes.byref(p), stream)
+    rc = _lib.launch(lib.kb_sa_fwd, p, q.device)
+    if rc == _lib.KB_ERR_UNSUPPORTED and k.shape[1] != H:
+        # no kernel with shared key/value heads for this dtype / head_dim / layout: repeat the heads
+        k_rep, v_rep = (t.repeat_interleave(H // t.shape[1], dim=1) for t in (k, v))
+        p.k, p.v, p.H_kv = _lib.tensor4(k_rep), _lib.tensor4(v_rep), H
+        rc = _lib.launch(lib.kb_sa_fwd, p, q.device)
     _lib.check(rc, "kb_sa_fwd")
     del lens_keep
 
@@ -235,21 +232,19 @@ def attention_backward_adapter(
     p.flags = _flags(prescale_qk, precision)
     p.status = _lib.status_words().data_ptr()
     p.H_kv = k.shape[1]
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        rc = lib.kb_sa_bwd(ctypes.byref(p), stream)
-        if rc == _lib.KB_ERR_UNSUPPORTED and k.shape[1] != H:
-            # no kernel with shared key/value heads for this call: repeat the heads, then add up the
-            # gradients of a group's copies
-            group = H // k.shape[1]
-            k_rep, v_rep = (t.repeat_interleave(group, dim=1) for t in (k, v))
-            dk_rep, dv_rep = torch.empty_like(k_rep), torch.empty_like(v_rep)
-            p.k, p.v, p.H_kv = _lib.tensor4(k_rep), _lib.tensor4(v_rep), H
-            p.dk, p.dv = dk_rep.data_ptr(), dv_rep.data_ptr()
-            rc = lib.kb_sa_bwd(ctypes.byref(p), stream)
-            if rc == 0:
-                DK.copy_(dk_rep.view(B, k.shape[1], group, T, D).float().sum(dim=2))
-                DV.copy_(dv_rep.view(B, k.shape[1], group, T, D).float().sum(dim=2))
+    rc = _lib.launch(lib.kb_sa_bwd, p, q.device)
+    if rc == _lib.KB_ERR_UNSUPPORTED and k.shape[1] != H:
+        # no kernel with shared key/value heads for this call: repeat the heads, then add up the
+        # gradients of a group's copies
+        group = H // k.shape[1]
+        k_rep, v_rep = (t.repeat_interleave(group, dim=1) for t in (k, v))
+        dk_rep, dv_rep = torch.empty_like(k_rep), torch.empty_like(v_rep)
+        p.k, p.v, p.H_kv = _lib.tensor4(k_rep), _lib.tensor4(v_rep), H
+        p.dk, p.dv = dk_rep.data_ptr(), dv_rep.data_ptr()
+        rc = _lib.launch(lib.kb_sa_bwd, p, q.device)
+        if rc == 0:
+            DK.copy_(dk_rep.view(B, k.shape[1], group, T, D).float().sum(dim=2))
+            DV.copy_(dv_rep.view(B, k.shape[1], group, T, D).float().sum(dim=2))
     _lib.check(rc, "kb_sa_bwd")
     del lens_keep
     return DQ, DK, DV
@@ -317,8 +312,7 @@ def streaming_attention_reference(q, k, v, context_size, back_contexts, lens, sc
     return out, res_mask, sparsity_fraction
 
 
-@torch.compile(fullgraph=True, dynamic=True)
-def _streaming_attention(
+def _streaming_attention_eager(
     q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision
 ):
     requires_grad = any(t.requires_grad for t in (q, k, v))
@@ -331,6 +325,9 @@ def _streaming_attention(
     if return_lse:
         return O, LSE
     return O
+
+
+_streaming_attention = torch.compile(_streaming_attention_eager, fullgraph=True, dynamic=True)
 
 
 def streaming_attention(
@@ -366,13 +363,21 @@ def streaming_attention(
     Signature and semantics follow ``streaming_attention`` of the reference
     (kernel.py:1599-1652).
     """
-    if not torch.compiler.is_compiling():
-        for t in (q, k, v):
-            torch._dynamo.mark_static(t, 1)
-            torch._dynamo.mark_static(t, 3)
+    # The compiled function is one operator call, so compiling it changes no result.  An ordinary call goes to the
+    # operator directly: guards, the compiled wrapper and its autograd function took 300 of the 500 us of host time of
+    # a forward + backward pass, more than the kernels of a small one.  Everything that looks inside (an outer
+    # compilation, transforms, hooks, modes) still meets the compiled function.
+    if _lib.plain_call(q, k, v):
+        attention = _streaming_attention_eager
+    else:
+        attention = _streaming_attention
+        if not torch.compiler.is_compiling():
+            for t in (q, k, v):
+                torch._dynamo.mark_static(t, 1)
+                torch._dynamo.mark_static(t, 3)
     if sm_scale is None:
         sm_scale = q.size(-1) ** -0.5
-    return _streaming_attention(
+    return attention(
         q=q, k=k, v=v, lens=lens,
         context_size=context_size, back_contexts=back_contexts, sm_scale=sm_scale,
         autotune=autotune, return_lse=return_lse, prescale_qk=prescale_qk, precision=precision,

@@ -18,7 +18,6 @@ path: shapes the kernels do not take raise.
 
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -63,9 +62,7 @@ def qkv_rope_projection(x: torch.Tensor, w_qkv: torch.Tensor, heads: int, kv_hea
     p.B, p.T, p.E, p.H, p.H_kv, p.D = B, T, E, heads, kv_heads, head_dim
     p.dtype = _lib.dtype_code(x.dtype)
     p.status = _lib.status_words().data_ptr()
-    with torch.cuda.device(x.device):
-        rc = _lib.load().kb_qkv_rope_proj(ctypes.byref(p), torch.cuda.current_stream(x.device).cuda_stream)
-    _lib.check(rc, "kb_qkv_rope_proj")
+    _lib.check(_lib.launch(_lib.load().kb_qkv_rope_proj, p, x.device), "kb_qkv_rope_proj")
     return q, k, v
 
 
@@ -85,7 +82,5 @@ def output_projection(o: torch.Tensor, w_o: torch.Tensor) -> torch.Tensor:
     p.B, p.T, p.H, p.D, p.E_out = B, T, H, D, w_o.shape[0]
     p.dtype = _lib.dtype_code(o.dtype)
     p.status = _lib.status_words().data_ptr()
-    with torch.cuda.device(o.device):
-        rc = _lib.load().kb_out_proj(ctypes.byref(p), torch.cuda.current_stream(o.device).cuda_stream)
-    _lib.check(rc, "kb_out_proj")
+    _lib.check(_lib.launch(_lib.load().kb_out_proj, p, o.device), "kb_out_proj")
     return y

@@ -17,7 +17,6 @@ queries are placed at the end of a zero tensor of ``T`` rows, the whole-sequence
 performance path).  There is no CPU path.
 """
 
-import ctypes
 import math
 from typing import Optional
 
@@ -69,8 +68,7 @@ def streaming_attention_step(
     p.status = _lib.status_words().data_ptr()
     p.H_kv = k.shape[1]
     p.q_start = T - Tq
-    with torch.cuda.device(q.device):
-        rc = _lib.load().kb_sa_fwd(ctypes.byref(p), torch.cuda.current_stream(q.device).cuda_stream)
+    rc = _lib.launch(_lib.load().kb_sa_fwd, p, q.device)
     del lens_keep
     if rc == _lib.KB_ERR_UNSUPPORTED:
         # no tcgen05 kernel for this dtype / head_dim / layout: whole-sequence call of the generic kernels

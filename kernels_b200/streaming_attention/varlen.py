@@ -19,7 +19,6 @@ those kernels do not take (fp32, head_dim 16, 32 or 256) run sequence by sequenc
 operator and its generic CUDA kernels (see ``streaming_attention_varlen``).
 """
 
-import ctypes
 import math
 from typing import Optional
 
@@ -74,9 +73,7 @@ class _StreamingAttentionVarlen(torch.autograd.Function):
         p.o, p.lse = o.data_ptr(), lse.data_ptr()
         cu_dev = cu.to(q.device) if single_launch else None
         p.cu_seqlens_dev = cu_dev.data_ptr() if single_launch else None
-        with torch.cuda.device(q.device):
-            rc = _lib.load().kb_sa_fwd_varlen(ctypes.byref(p), torch.cuda.current_stream(q.device).cuda_stream)
-        _lib.check(rc, "kb_sa_fwd_varlen")
+        _lib.check(_lib.launch(_lib.load().kb_sa_fwd_varlen, p, q.device), "kb_sa_fwd_varlen")
         ctx.mark_non_differentiable(lse)
         ctx.save_for_backward(q, k, v, o, lse)
         ctx.cu, ctx.max_len, ctx.cu_dev = cu, max_len, cu_dev
@@ -116,9 +113,7 @@ class _StreamingAttentionVarlen(torch.autograd.Function):
         p.dq, p.dk, p.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
         p.delta_ws, p.ds_ws, p.ds_ws_bytes, p.lanes = delta.data_ptr(), ds_ws.data_ptr(), lanes * ws_bytes, lanes
         p.cu_seqlens_dev = ctx.cu_dev.data_ptr() if ctx.cu_dev is not None else None
-        with torch.cuda.device(q.device):
-            rc = lib.kb_sa_bwd_varlen(ctypes.byref(p), torch.cuda.current_stream(q.device).cuda_stream)
-        _lib.check(rc, "kb_sa_bwd_varlen")
+        _lib.check(_lib.launch(lib.kb_sa_bwd_varlen, p, q.device), "kb_sa_bwd_varlen")
         return dq, dk, dv, None, None, None, None, None
 
 

@@ -363,3 +363,29 @@ def test_fp32_tiles_edges_and_layouts(D, T, c, back, layout):
     assert (got - want).abs().max() <= 5e-6
     for a, b in zip(torch.autograd.grad(got, got_in, do), torch.autograd.grad(want, ref, do.double())):
         assert (a - b).abs().max() <= 5e-5
+
+def test_ordinary_calls_equal_the_compiled_function():
+    """An ordinary call reaches the operator directly, one under saved-tensor hooks or inside a compiled function goes
+    through the compiled wrapper: the same kernels, so the same bits; both refuse a second derivative."""
+    from kernels_b200.streaming_attention import kernel as K
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(2, 2, 200, 64, generator=g, device="cuda", dtype=torch.float16).requires_grad_() for _ in range(3))
+    do = torch.randn(2, 2, 200, 64, generator=g, device="cuda", dtype=torch.float16)
+    lens = torch.tensor([200, 77], dtype=torch.int32, device="cuda")
+
+    def step(fn, hooks):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t) if hooks else torch.enable_grad():
+            o = fn(q, k, v, lens, 24, 2)
+        return (o, *torch.autograd.grad(o, (q, k, v), do))
+
+    torch._dynamo.utils.counters["stats"].clear()
+    want = step(K.streaming_attention, False)
+    assert torch._dynamo.utils.counters["stats"]["unique_graphs"] == 0
+    compiled = torch.compile(lambda *a: K.streaming_attention(*a) * 1, fullgraph=True)
+    for got in (step(K.streaming_attention, True), step(compiled, False)):
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    o = K.streaming_attention(q, k, v, lens, 24, 2)
+    dq, = torch.autograd.grad(o, (q,), do.clone().requires_grad_(), create_graph=True)
+    with pytest.raises(RuntimeError):
+        dq.float().sum().backward()
