@@ -100,8 +100,8 @@ struct alignas(1024) FwdSmem {
   uint8_t k[kStagesK][kBN * D * 2];
   uint8_t v[kStagesV][kBN * D * 2];
   uint8_t o_stage[kQTiles][kBM * 128];  // one 64-column panel of a q tile's output on its way to a TMA store
-  uint64_t q_full, k_full[kStagesK], k_empty[kStagesK], v_full[kStagesV], v_empty[kStagesV];
-  uint64_t q_empty, s_ready[kQTiles], p_ready[kQTiles], o_done[kQTiles], o_free[kQTiles];
+  uint64_t q_full[kQTiles], k_full[kStagesK], k_empty[kStagesK], v_full[kStagesV], v_empty[kStagesV];
+  uint64_t q_empty[kQTiles], s_ready[kQTiles], p_ready[kQTiles], o_done[kQTiles], o_free[kQTiles];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -343,8 +343,6 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   };
 
   if (threadIdx.x == 0) {
-    mbar_init(&sm.q_full, 1);
-    mbar_init(&sm.q_empty, 1);
     for (int s = 0; s < kStagesK; ++s) {
       mbar_init(&sm.k_full[s], 1);
       mbar_init(&sm.k_empty[s], 1);
@@ -354,6 +352,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_init(&sm.v_empty[s], 1);
     }
     for (int x = 0; x < kQTiles; ++x) {
+      mbar_init(&sm.q_full[x], 1);
+      mbar_init(&sm.q_empty[x], 1);
       mbar_init(&sm.s_ready[x], 1);
       mbar_init(&sm.p_ready[x], kBM);
       mbar_init(&sm.o_done[x], 1);
@@ -375,28 +375,31 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   constexpr int kOutPanels = D / 64;               // of a 16-bit output row
 
   // Barrier phases are counted over the whole life of the CTA: kc / vc = K / V tiles so far,
-  // na = items with at least one live q tile so far, per q tile: tiles and items so far.
+  // per q tile: tiles and items so far.
   if (warp == kProducerWarp) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
       prefetch_tensormap(&tm_q);
       prefetch_tensormap(&tm_k);
       prefetch_tensormap(&tm_v);
-      int kc = 0, vc = 0, na = 0;
+      int kc = 0, vc = 0;
+      int items_x[kQTiles] = {0, 0};  // items in which q tile x was live so far
       bool ok = true;
       for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
         const Item it = decode(walk.item());
         if (!it.act[0] && !it.act[1]) continue;
-        // the Q buffers are free once every S of the previous item has been issued and has run
-        if (na > 0 && !mbar_wait(&sm.q_empty, (na - 1) & 1, ctx, kWaitQEmpty)) break;
-        mbar_expect_tx(&sm.q_full, (it.act[0] ? kTileBytes : 0) + (it.act[1] ? kTileBytes : 0));
-#pragma unroll
-        for (int x = 0; x < kQTiles; ++x) {
-          if (!it.act[x]) continue;
+        // a Q buffer is free once the last S of its q tile in the previous item has run
+        auto load_q = [&](int x) -> bool {
+          if (!it.act[x]) return true;
+          if (items_x[x] > 0 && !mbar_wait(&sm.q_empty[x], (items_x[x] - 1) & 1, ctx, kWaitQEmpty)) return false;
+          ++items_x[x];
+          mbar_expect_tx(&sm.q_full[x], kTileBytes);
 #pragma unroll
           for (int p = 0; p < kPanels; ++p)
-            tma_load_4d(sm.q[x] + p * kPanelBytes, &tm_q, &sm.q_full, p * kPanelElems, it.row0 + it.q0 - a.q_start + x * kBM, it.h, PACKED ? 0 : it.b);
-        }
+            tma_load_4d(sm.q[x] + p * kPanelBytes, &tm_q, &sm.q_full[x], p * kPanelElems, it.row0 + it.q0 - a.q_start + x * kBM, it.h, PACKED ? 0 : it.b);
+          return true;
+        };
+        if (!load_q(0)) break;
         const int h_kv = kb_fastdiv(it.h, a.fd_group);  // the K/V head this query head reads
         for (int t = it.u_begin; t < it.u_end; ++t, ++kc, ++vc) {
           const int sk = kc % kStagesK, sv = vc % kStagesV;
@@ -405,12 +408,13 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           mbar_expect_tx(&sm.k_full[sk], kTileBytes);
 #pragma unroll
           for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.k[sk] + p * kPanelBytes, &tm_k, &sm.k_full[sk], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
+          // (order of need: Q of tile A and the first K, then Q of tile B)
+          if (t == it.u_begin && !load_q(1)) { ok = false; break; }
           if (vc >= kStagesV && !mbar_wait(&sm.v_empty[sv], ((vc / kStagesV) - 1) & 1, ctx, kWaitVEmpty)) { ok = false; break; }
           mbar_expect_tx(&sm.v_full[sv], kTileBytes);
 #pragma unroll
           for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.v[sv] + p * kPanelBytes, &tm_v, &sm.v_full[sv], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
         }
-        ++na;
       }
     }
   } else if (warp == kMmaWarp) {
@@ -418,7 +422,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (lane == 0) {
       constexpr uint32_t idesc_qk = FP8 ? make_idesc_e4m3(kBM, kBN, false, false) : make_idesc(BF16, kBM, kBN, false, false);
       constexpr uint32_t idesc_pv = FP8 ? make_idesc_e4m3(kBM, D, false, true) : make_idesc(BF16, kBM, D, false, true);
-      int kbase = 0, na = 0;            // K (= V) tiles of earlier items, live items so far
+      int kbase = 0;                    // K (= V) tiles of earlier items
       int tiles_x[kQTiles] = {0, 0};    // S / P blocks of q tile x so far
       int items_x[kQTiles] = {0, 0};    // items in which q tile x was live so far
       bool ok = true;
@@ -426,12 +430,25 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       long long acc_t[10] = {0};
       long long tl = clock64();
 #endif
-      for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
-        const Item it = decode(walk.item());
-        if (!it.act[0] && !it.act[1]) continue;
+      // FAST: the first S of tile A of an item is issued ahead, between the last P V of tile A and that of tile B of the
+      // item before it, where its Q and K have landed by then (`ahead`): tile A's softmax warps go from one item to the
+      // next without waiting for tile B's last block.  (Q has a barrier pair per q tile for this: a Q buffer is free
+      // after ITS tile's last S.)  bf16 D=128 c=256 T=16384: 865 -> 830 us, T=2048: 116 -> 109, 8-bit 217 -> 211, dense
+      // D=64 397 -> 378.  In the general schedule the same step measured 235 -> 270 us (fp16 D=64 c=10) and 846 -> 923
+      // (packed, c=64); the barrier pairs alone 240 -> 234 and 803 -> 779 (bf16 c=64 T=8192).
+      KbItemWalk<!FAST> walk(a.item_rot);
+      Item next;
+      auto seek = [&]() -> bool {  // the first live item from the walk's position on
+        for (; walk.item() < n_items; walk.next()) {
+          next = decode(walk.item());
+          if (next.act[0]) return true;  // (tile B is never live without tile A)
+        }
+        return false;
+      };
+      bool more = seek(), ahead = false;
+      while (ok && more) {
+        const Item it = next;
         KB_FACC(0);
-        if (!mbar_wait(&sm.q_full, na & 1, ctx, kWaitQ)) break;
-        KB_FACC(1);
         // Step s issues, per q tile x:  PV_x(s - 1) then S_x(s), each q tile walking its own key tiles in order.
         // When tile B's range starts d key tiles after tile A's (chunks shorter than the 256-row item: the two q
         // tiles then see different windows) and the K / V rings can hold d + 1 tiles, both q tiles start at step
@@ -485,10 +502,12 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           KB_FACC(6);
           return true;
         };
-        // S_x = Q_x K^T, K being ring tile ki
-        auto issue_s = [&](int x, int ki, bool release_k) -> bool {
+        // S_x = Q_x K^T, K being ring tile ki; `first` / `last` of the q tile's key tiles
+        auto issue_s = [&](int x, int ki, bool release_k, bool first, bool last) -> bool {
           const int sk = ki % kStagesK;
           KB_FACC(2);
+          if (first && !mbar_wait(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) return false;
+          KB_FACC(1);
           if (!mbar_wait(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) return false;
           KB_FACC(7);
           tc_fence_after();
@@ -502,10 +521,28 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
           }
           if (release_k) mma_commit(&sm.k_empty[sk]);
+          if (last) mma_commit(&sm.q_empty[x]);
           mma_commit(&sm.s_ready[x]);
           ++tiles_x[x];
           KB_FACC(8);
           return true;
+        };
+        const bool was_ahead = ahead;
+        ahead = false;
+        auto look_ahead = [&] {  // for the next live item; FAST: while the thread would wait for the last P of tile A
+          walk.next();
+          more = seek();
+        };
+        // After the last P V of tile A and before that of tile B, the first S of tile A of that item
+        auto issue_ahead = [&]() -> bool {
+          const int ki = kbase + (it.u_end - it.u_begin);
+          ahead = more && mbar_test(&sm.q_full[0], (items_x[0] + 1) & 1) && mbar_test(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1);
+          if (!ahead) return true;
+          ++items_x[0];  // (the S belongs to the next item's count)
+          const bool b_too = next.act[1] && next.kr[1].begin == next.kr[0].begin;  // tile B uses the key tile as well
+          const bool done = issue_s(0, ki, !b_too, true, next.kr[0].end - next.kr[0].begin == 1);
+          --items_x[0];
+          return done;
         };
         if (FAST && it.act[0] && it.act[1] && d == 0 && n_x[0] == n_x[1]) {
           // Both q tiles on the same key tiles at the same steps: ring tile kbase + i is the i-th key tile of both,
@@ -513,26 +550,26 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           using Yes = std::true_type;
           using No = std::false_type;
           const int n = n_x[0];
-          ok = issue_s(0, kbase, false) && issue_s(1, kbase, true);
+          ok = (was_ahead || issue_s(0, kbase, false, true, n == 1)) && issue_s(1, kbase, true, true, n == 1);
           if (n == 1) {
-            mma_commit(&sm.q_empty);  // every S of this item has been issued
-            ok = ok && issue_pv(Yes{}, Yes{}, 0, kbase, false) && issue_pv(Yes{}, Yes{}, 1, kbase, true);
+            look_ahead();
+            ok = ok && issue_pv(Yes{}, Yes{}, 0, kbase, false) && issue_ahead() && issue_pv(Yes{}, Yes{}, 1, kbase, true);
           } else {
-            ok = ok && issue_pv(Yes{}, No{}, 0, kbase, false) && issue_s(0, kbase + 1, false) &&
-                 issue_pv(Yes{}, No{}, 1, kbase, true) && issue_s(1, kbase + 1, true);
-            if (n == 2) mma_commit(&sm.q_empty);
+            ok = ok && issue_pv(Yes{}, No{}, 0, kbase, false) && issue_s(0, kbase + 1, false, false, n == 2) &&
+                 issue_pv(Yes{}, No{}, 1, kbase, true) && issue_s(1, kbase + 1, true, false, n == 2);
             for (int step = 2; ok && step < n; ++step) {
-              ok = issue_pv(No{}, No{}, 0, kbase + step - 1, false) && issue_s(0, kbase + step, false) &&
-                   issue_pv(No{}, No{}, 1, kbase + step - 1, true) && issue_s(1, kbase + step, true);
-              if (step == n - 1) mma_commit(&sm.q_empty);
+              ok = issue_pv(No{}, No{}, 0, kbase + step - 1, false) && issue_s(0, kbase + step, false, false, step == n - 1) &&
+                   issue_pv(No{}, No{}, 1, kbase + step - 1, true) && issue_s(1, kbase + step, true, false, step == n - 1);
             }
-            ok = ok && issue_pv(No{}, Yes{}, 0, kbase + n - 1, false) && issue_pv(No{}, Yes{}, 1, kbase + n - 1, true);
+            look_ahead();
+            ok = ok && issue_pv(No{}, Yes{}, 0, kbase + n - 1, false) && issue_ahead() && issue_pv(No{}, Yes{}, 1, kbase + n - 1, true);
           }
         } else {
           // (the same two issue sequences, written out: through the lambdas this path measured 3-4 % slower)
           for (int step = 0; ok && step <= n_steps; ++step) {
   #pragma unroll
             for (int x = 0; x < kQTiles; ++x) {
+              if (FAST && x == 0 && step == n_steps) look_ahead();
               const bool pv_live = it.act[x] && step - 1 >= first_x[x] && step - 1 < first_x[x] + n_x[x];
               const bool s_live = it.act[x] && step >= first_x[x] && step < first_x[x] + n_x[x];
               if (pv_live) {
@@ -568,10 +605,13 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 if (u == it.kr[x].end - 1) mma_commit(&sm.o_done[x]);
                 KB_FACC(6);
               }
-              if (s_live) {
+              if (FAST && x == 0 && step == n_steps && !issue_ahead()) { ok = false; break; }
+              if (s_live && !(x == 0 && step == 0 && was_ahead)) {
                 const int t = it.kr[x].begin + (step - first_x[x]);
                 const int ki = kbase + (t - it.u_begin), sk = ki % kStagesK;
                 KB_FACC(2);
+                if (step == first_x[x] && !mbar_wait(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) { ok = false; break; }
+                KB_FACC(1);
                 if (!mbar_wait(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) { ok = false; break; }
                 KB_FACC(7);
                 tc_fence_after();
@@ -585,16 +625,16 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                   }
                 }
                 if (last_user(x, t)) mma_commit(&sm.k_empty[sk]);
+                if (t == it.kr[x].end - 1) mma_commit(&sm.q_empty[x]);
                 mma_commit(&sm.s_ready[x]);
                 ++tiles_x[x];
                 KB_FACC(8);
               }
             }
-            if (step == n_steps - 1) mma_commit(&sm.q_empty);  // every S of this item has been issued
           }
         }
+        if (!FAST) look_ahead();
         kbase += it.u_end - it.u_begin;
-        ++na;
 #pragma unroll
         for (int x = 0; x < kQTiles; ++x) items_x[x] += it.act[x] ? 1 : 0;
       }
