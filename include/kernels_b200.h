@@ -234,6 +234,11 @@ KB_API int kb_sa_bwd(const kb_sa_bwd_params* p, void* stream);
 KB_API uint64_t kb_sa_bwd_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, int32_t dtype,
                                           int32_t context_size, int32_t back_contexts);
 
+/* Host-only: the same for the fp32 kernels of kb_sa_bwd, which evaluate the scores once when `ds_ws` holds this many
+ * bytes (fp32 dS tiles of 64 x 64, 32 x 32 at D = 256) and run their two passes otherwise.  0 for other dtypes. */
+KB_API uint64_t kb_sa_bwd_generic_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, int32_t dtype,
+                                                  int32_t context_size, int32_t back_contexts);
+
 /*
  * Streaming attention backward without caller-provided scratch.  No counterpart in the
  * reference (its Python op body allocates `delta` itself, kernel.py:1380); it exists for hosts

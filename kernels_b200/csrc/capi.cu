@@ -379,6 +379,14 @@ uint64_t kb_sa_bwd_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, i
   return 0;
 }
 
+uint64_t kb_sa_bwd_generic_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, int32_t dtype, int32_t context_size,
+                                           int32_t back_contexts) {
+  const bool head_dim_ok = D == 16 || D == 32 || D == 64 || D == 128 || D == 256;
+  if (B <= 0 || H <= 0 || T <= 0 || !head_dim_ok || dtype != KB_F32 || context_size < 1 || back_contexts < 0) return 0;
+  const int32_t c = kb_clamp_context(context_size, T);
+  return kb::sa_bwd_generic_workspace_bytes(B, H, T, D, c, kb_clamp_back(back_contexts, T, c));
+}
+
 uint64_t kb_sa_bwd_varlen_workspace_bytes(int32_t B, int32_t H, int32_t total_rows, int32_t max_len, int32_t D,
                                           int32_t dtype, int32_t context_size, int32_t back_contexts) {
 #ifdef KB_HAVE_SM100_BWD_FUSED

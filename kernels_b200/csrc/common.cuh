@@ -58,6 +58,7 @@ struct AttnShape {
 
 // ---- launchers implemented in the kernel translation units -----------------------------
 int sa_fwd_generic(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s);
+size_t sa_bwd_generic_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, int32_t c, int32_t back);
 int sa_bwd_generic(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t s);
 int sa_fwd_sm100(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s);
 int sa_fwd_sm100_fp8(const kb_sa_fwd_fp8_params& p, int32_t c, int32_t back, cudaStream_t s);

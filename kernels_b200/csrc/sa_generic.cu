@@ -24,6 +24,10 @@
 // blocks' arithmetic.  Tiles come in with cp.async where the rows
 // are fp32, 16-byte aligned and dense, the next one while the current block is still being worked on.
 //
+// Backward: the dQ pass and the dK/dV pass each evaluate the scores and dP.  fp32 calls with a dS scratch evaluate them
+// once instead: delta, dK/dV (which saves its dS tiles), dQ = dS K (sa_bwd_dq_saved_generic_kernel).  Same case: 202 +
+// 260 -> 11 + 264 + 65 us.
+//
 // Reference semantics followed: src/streaming_attention/kernel.py:205-430 (forward),
 // 639-773 and 941-1023 (dQ), 777-937 and 1027-1129 (dK/dV), 453-514 (delta).
 #include <math.h>
@@ -84,11 +88,28 @@ struct BwdArgs {
   T* dk;
   T* dv;
   float* delta;
+  float* ds;  // dS scratch (single evaluation): tile (b, h, key tile, slot) of BM x BN floats
+  int32_t W;  // its slots per key tile
   const int32_t* lens;
   int64_t lens_stride;
   int32_t H, T_, c, back;
   float scale_log2, sm_scale;
 };
+
+// Most query tiles a key tile meets (the schedule with len = T; a shorter sequence only clips it).
+inline int32_t ds_slots(int32_t T, int32_t tile, int32_t c, int32_t back) {
+  int32_t w = 1;
+  for (int32_t k0 = 0; k0 < T; k0 += tile) {
+    const KbTileRange r = kb_bwd_q_range(k0, tile, tile, T, c, back);
+    w = kb_max_i32(w, r.end - r.begin);
+  }
+  return w;
+}
+template <int D, typename T>
+__device__ __forceinline__ float* ds_tile(const BwdArgs<T>& a, int64_t bh, int kt, int slot) {
+  constexpr int BM = Cfg<D>::BM;
+  return a.ds + ((bh * kb_cdiv_i32(a.T_, BM) + kt) * a.W + slot) * (int64_t)(BM * BM);
+}
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -480,7 +501,8 @@ __global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasBwd) sa_bwd_dq_
 // ------------------------------------------------------------------------------------------
 // backward, dK/dV pass (reads delta written by the dQ pass)
 // ------------------------------------------------------------------------------------------
-template <int D, typename T>
+// SAVE: the dS tiles also go to the scratch, [query][key slot] as they lie in shared memory.
+template <int D, typename T, bool SAVE>
 __global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasBwd) sa_bwd_dkdv_generic_kernel(const BwdArgs<T> a) {
   using C = Cfg<D>;
   constexpr int BM = C::BM, BN = C::BN, RM = C::RM, RN = C::RN;
@@ -558,6 +580,13 @@ __global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasBwd) sa_bwd_dkd
       }
       store_transposed<D>(dSt, s, ty, tx);
       __syncthreads();
+      if (SAVE) {
+        float4* dst = reinterpret_cast<float4*>(ds_tile<D, T>(a, bh, blockIdx.x, qt - qr.begin));
+        for (int idx = threadIdx.x; idx < BM * BN / 4; idx += C::kThreads) {
+          const int r = idx / (BN / 4), k4 = (idx - r * (BN / 4)) * 4;
+          dst[idx] = *reinterpret_cast<const float4*>(&dSt[r * C::PLD + k4]);
+        }
+      }
       tile_xv<D>(Pt, dOs, acc_dv, ty, tx);
       tile_xv<D>(dSt, Qs, acc_dk, ty, tx);
       __syncthreads();
@@ -574,6 +603,113 @@ __global__ void __launch_bounds__(Cfg<D>::kThreads, Cfg<D>::kCtasBwd) sa_bwd_dkd
   }
   store_rows<D, T>(dk_slice, acc_dk, sc_k, zero, k0, T_, ty, tx);
   store_rows<D, T>(dv_slice, acc_dv, sc_v, zero, k0, T_, ty, tx);
+}
+
+// ------------------------------------------------------------------------------------------
+// backward with the scores evaluated once (fp32): delta, then dK/dV saving dS, then dQ = dS K
+// ------------------------------------------------------------------------------------------
+// Sixteen lanes per row with the columns the dQ pass gives them, so that delta has the same bits.
+template <int D, typename T>
+__global__ void __launch_bounds__(256) sa_bwd_delta_generic_kernel(const BwdArgs<T> a) {
+  using C = Cfg<D>;
+  const int b = blockIdx.z, h = blockIdx.y, tx = threadIdx.x & 15;
+  const int len = load_len(a.lens, a.lens_stride, b, a.T_);
+  const T* o_slice = a.o.p + b * a.o.sb + h * a.o.sh;
+  const T* g_slice = a.d_o.p + b * a.d_o.sb + h * a.d_o.sh;
+#pragma unroll
+  for (int it = 0; it < C::BM / 16; ++it) {
+    const int r = blockIdx.x * C::BM + it * 16 + (threadIdx.x >> 4);
+    float part = 0.f;
+    if (r < len) {
+#pragma unroll
+      for (int n = 0; n < C::DV; ++n) {
+        const int64_t d = col_of<D>(n, tx);
+        part = fmaf(to_f32(o_slice[(int64_t)r * a.o.st + d * a.o.sd]), to_f32(g_slice[(int64_t)r * a.d_o.st + d * a.d_o.sd]), part);
+      }
+    }
+    part = half_warp_sum(part);
+    if (tx == 0 && r < a.T_) a.delta[((int64_t)b * a.H + h) * a.T_ + r] = part;
+  }
+}
+
+// One CTA per query tile: streams the saved dS tiles of its key tiles with the matching K tiles.  A third of the
+// dQ pass's arithmetic for one write and one read of 4 bytes per score (202 -> 65 us, dK/dV pass 260 -> 264).  Small
+// CTAs with single buffers: five or more on an SM cover each other's loads.
+template <int D, typename T>
+__global__ void __launch_bounds__(Cfg<D>::kThreads) sa_bwd_dq_saved_generic_kernel(const BwdArgs<T> a) {
+  using C = Cfg<D>;
+  constexpr int BM = C::BM, BN = C::BN, RM = C::RM, SLD = BN + kPad;
+  extern __shared__ __align__(16) float smem[];
+  float* Ss = smem;  // dS tile, [query][key slot]
+  float* Ks = Ss + BM * SLD;
+
+  const int b = blockIdx.z, h = blockIdx.y, qt = blockIdx.x, q0 = qt * BM;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int T_ = a.T_;
+  const int len = load_len(a.lens, a.lens_stride, b, T_);
+  const int64_t bh = (int64_t)b * a.H + h;
+  const KbTileRange kr = kb_fwd_kv_range(q0, BM, BN, len, a.c, a.back);
+
+  float acc[RM][C::DV];
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int n = 0; n < C::DV; ++n) acc[i][n] = 0.f;
+
+  for (int kt = kr.begin; kt < kr.end; ++kt) {
+    // the slot this query tile has in key tile kt's list: both schedules name the same pairs
+    const KbTileRange qr = kb_bwd_q_range(kt * BN, BM, BN, len, a.c, a.back);
+    const float* src = ds_tile<D, T>(a, bh, kt, qt - qr.begin);
+    for (int idx = threadIdx.x; idx < BM * BN / 4; idx += C::kThreads) {
+      const int r = idx / (BN / 4), k4 = (idx - r * (BN / 4)) * 4;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm100::smem_u32(Ss + r * SLD + k4)), "l"(src + idx * 4) : "memory");
+    }
+    load_tile<D, BN>(Ks, a.k, b, h, kt * BN, T_);
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll 2
+    for (int s4 = 0; s4 < BN; s4 += 4) {
+      float4 x[RM];
+#pragma unroll
+      for (int i = 0; i < RM; ++i) x[i] = *reinterpret_cast<const float4*>(&Ss[(ty + C::TY * i) * SLD + s4]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int slot = s4 + e, key = slot / RM + C::TY * (slot % RM);  // see store_transposed
+        float k[C::DV];
+#pragma unroll
+        for (int n = 0; n < C::DV; n += C::VEC) {
+          const float* kp = &Ks[key * C::LD + col_of<D>(n, tx)];
+          if constexpr (C::VEC == 4) {
+            const float4 t = *reinterpret_cast<const float4*>(kp);
+            k[n] = t.x, k[n + 1] = t.y, k[n + 2] = t.z, k[n + 3] = t.w;
+          } else {
+#pragma unroll
+            for (int v = 0; v < C::VEC; ++v) k[n + v] = kp[v];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+          const float xv = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+#pragma unroll
+          for (int n = 0; n < C::DV; ++n) acc[i][n] = fmaf(xv, k[n], acc[i][n]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+
+  uint64_t out[RM / 2][C::DV];
+  float scale[RM];
+  bool zero[RM];
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    scale[i] = a.sm_scale;
+    zero[i] = false;
+#pragma unroll
+    for (int n = 0; n < C::DV; ++n)
+      if (i % 2 == 0) out[i / 2][n] = sm100::f2_pack(acc[i][n], acc[i + 1][n]);
+  }
+  store_rows<D, T>(a.dq + bh * T_ * D, out, scale, zero, q0, T_, ty, tx);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -614,7 +750,7 @@ int launch_bwd(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t 
   constexpr size_t smem_dkdv = sizeof(float) * (size_t)(2 * C::BM * C::LD + 2 * C::BN * C::LD + 2 * C::BM * C::PLD + 4 * C::BM);
   static_assert(smem_dkdv <= 232448, "shared memory exceeds the 227 KB a CTA may have");
   auto kern_dq = sa_bwd_dq_generic_kernel<D, T>;
-  auto kern_dkdv = sa_bwd_dkdv_generic_kernel<D, T>;
+  auto kern_dkdv = sa_bwd_dkdv_generic_kernel<D, T, false>;
   int dev = 0, n_sm = 0;
   if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
   static std::atomic<bool> dq_opted_in[kMaxDevices], dkdv_opted_in[kMaxDevices];
@@ -631,6 +767,8 @@ int launch_bwd(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t 
   a.dk = static_cast<T*>(p.dk);
   a.dv = static_cast<T*>(p.dv);
   a.delta = p.delta_ws;
+  a.ds = nullptr;
+  a.W = 0;
   a.lens = p.lens;
   a.lens_stride = p.lens_stride;
   a.H = p.H;
@@ -640,6 +778,29 @@ int launch_bwd(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t 
   a.scale_log2 = p.sm_scale * kLog2e;
   a.sm_scale = p.sm_scale;
   dim3 grid_q(kb_cdiv_i32(p.T, C::BM), p.H, p.B), grid_k(kb_cdiv_i32(p.T, C::BN), p.H, p.B);
+  if constexpr (sizeof(T) == 4) {
+    // Scores evaluated once where the caller gives the scratch (and asks for no single pass): three launches, 14 instead
+    // of 18 multiplications per pair and head-dim element over forward and backward.
+    const uint32_t passes = KB_FLAG_BWD_SKIP_DQ | KB_FLAG_BWD_SKIP_DKDV | KB_FLAG_BWD_SKIP_DELTA | KB_FLAG_BWD_TWO_PASS;
+    if (p.ds_ws && !(p.flags & passes) && reinterpret_cast<uintptr_t>(p.ds_ws) % 16 == 0 &&
+        p.ds_ws_bytes >= sa_bwd_generic_workspace_bytes(p.B, p.H, p.T, D, c, back)) {
+      constexpr size_t smem_saved = sizeof(float) * (size_t)(C::BM * (C::BN + kPad) + C::BN * C::LD);
+      auto kern_save = sa_bwd_dkdv_generic_kernel<D, T, true>;
+      auto kern_saved = sa_bwd_dq_saved_generic_kernel<D, T>;
+      static std::atomic<bool> save_opted_in[kMaxDevices], saved_opted_in[kMaxDevices];
+      KB_CUDA_TRY(opt_in_smem_once(kern_save, smem_dkdv, dev, save_opted_in));
+      KB_CUDA_TRY(opt_in_smem_once(kern_saved, smem_saved, dev, saved_opted_in));
+      a.ds = static_cast<float*>(p.ds_ws);
+      a.W = ds_slots(p.T, C::BM, c, back);
+      sa_bwd_delta_generic_kernel<D, T><<<grid_q, 256, 0, s>>>(a);
+      KB_LAUNCH_CHECK("sa_bwd_delta_generic_kernel");
+      kern_save<<<grid_k, C::kThreads, smem_dkdv, s>>>(a);
+      KB_LAUNCH_CHECK("sa_bwd_dkdv_generic_kernel");
+      kern_saved<<<grid_q, C::kThreads, smem_saved, s>>>(a);
+      KB_LAUNCH_CHECK("sa_bwd_dq_saved_generic_kernel");
+      return KB_OK;
+    }
+  }
   if (!(p.flags & KB_FLAG_BWD_SKIP_DQ)) {
     kern_dq<<<grid_q, C::kThreads, smem_dq, s>>>(a);
     KB_LAUNCH_CHECK("sa_bwd_dq_generic_kernel");
@@ -677,6 +838,12 @@ int sa_fwd_generic(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStrea
     default:
       return KB_ERR_UNSUPPORTED;
   }
+}
+
+// Bytes of dS scratch the single-evaluation fp32 backward needs; c and back already clamped to T.
+size_t sa_bwd_generic_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, int32_t c, int32_t back) {
+  const int32_t tile = tiles::generic_tile(D);
+  return (size_t)B * H * kb_cdiv_i32(T, tile) * ds_slots(T, tile, c, back) * tile * tile * sizeof(float);
 }
 
 int sa_bwd_generic(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_t s) {

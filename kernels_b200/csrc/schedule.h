@@ -95,9 +95,9 @@ KB_HD int32_t kb_fastdiv(int32_t n, const KbFastDiv& f) {
 //
 // Only where the lengths differ and a CTA would meet at most four places.  Measured (B200, r = 0 / r = 1): packed batch
 // of 256 sequences of 128-1024 rows, forward 951 / 843 us, main backward kernel 1286 / 1081, dQ 497 / 402; fp16 D=64
-// c=10 T=1353 (n = 6, three places) forward 261 / 235 us.  With eight and more places nothing is gained, and an odd r
-// separates the CTAs of an SM pair from the two key tiles of one chunk, whose common Q / dO tiles the pair fetches
-// together: main kernel, bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r.
+// c=10 T=1353 (n = 6, three places) forward 261 / 235 us.  With eight and more places nothing is gained, and
+// an odd r can cost: main kernel, bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r (with an even one
+// CTAs 2 m and 2 m + 1 always have the two key tiles of one chunk, which stream the same Q / dO tiles).
 inline int32_t kb_gcd(int32_t a, int32_t b) {
   while (b) {
     const int32_t t = a % b;

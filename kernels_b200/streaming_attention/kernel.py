@@ -49,6 +49,9 @@ def _ds_scratch_for(device: torch.device, stream_ptr: int, nbytes: int):
         total = _device_total_bytes[idx] = torch.cuda.get_device_properties(idx).total_memory
     if nbytes > _MAX_DS_SCRATCH_BYTES or nbytes > total // 4:
         return None
+    if torch.cuda.is_current_stream_capturing():
+        # a graph keeps what it captured: memory of its own, not a buffer that later calls share, grow and free
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
     key = (idx, stream_ptr)
     buf = _ds_scratch.get(key)
     if buf is None or buf.numel() < nbytes:
@@ -181,8 +184,9 @@ def attention_backward_adapter(
     """Backward op body: ``(dQ, dK, dV)`` through ``kb_sa_bwd``.
 
     Scratch is allocated here and handed to the library: ``delta = rowsum(O * dO)`` as
-    ``[B, H, T]`` fp32 (reference: kernel.py:1380) and, for the tcgen05 backward that evaluates
-    the scores once, room for the 16-bit dS tiles (``kb_sa_bwd_workspace_bytes``; it grows with
+    ``[B, H, T]`` fp32 (reference: kernel.py:1380) and, for the backward kernels that evaluate
+    the scores once, room for the dS tiles (``kb_sa_bwd_workspace_bytes``, fp32:
+    ``kb_sa_bwd_generic_workspace_bytes``; it grows with
     ``(back_contexts + 1) * context_size``; one buffer per device and stream, kept between calls).
     When that room exceeds ``_MAX_DS_SCRATCH_BYTES`` or a quarter of the device's memory, it is
     withheld and the library runs its two-pass kernels, which need none.  ``do`` may arrive in another dtype or with any strides
@@ -213,7 +217,8 @@ def attention_backward_adapter(
     lib = _lib.load()
     ds_ws = None
     if q.numel():
-        ws_bytes = int(lib.kb_sa_bwd_workspace_bytes(
+        workspace_bytes = lib.kb_sa_bwd_generic_workspace_bytes if q.dtype == torch.float32 else lib.kb_sa_bwd_workspace_bytes
+        ws_bytes = int(workspace_bytes(
             B, H, T, D, _lib.dtype_code(q.dtype), _clamp_i32(context_size), _clamp_i32(back_contexts)))
         ds_ws = _ds_scratch_for(q.device, torch.cuda.current_stream(q.device).cuda_stream, ws_bytes)
     lens_keep, lens_ptr, lens_stride = _lens_arg(lens, q.device)

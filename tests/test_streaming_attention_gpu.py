@@ -336,10 +336,16 @@ def test_dynamic_shapes_compile_into_few_graphs(lens_mode):
 
 @pytest.mark.parametrize("D", [16, 32, 64, 128, 256])
 @pytest.mark.parametrize("T,c,back,layout", [(1, 1, 0, "bhtd"), (63, 7, 3, "odd"), (65, 64, 1, "bthd"), (129, 200, 0, "bhtd"), (200, 10, 5, "odd")])
-def test_fp32_tiles_edges_and_layouts(D, T, c, back, layout):
+@pytest.mark.parametrize("scratch", [True, False])
+def test_fp32_tiles_edges_and_layouts(D, T, c, back, layout, scratch, monkeypatch):
     """The fp32 kernels one row around their tiles (64, 32 for D = 256), on rows that take asynchronous copies (dense,
-    16-byte aligned) and rows that do not, against dense attention in 64 bits.  Bounds: the fp32 ones of the grid."""
+    16-byte aligned) and rows that do not, against dense attention in 64 bits.  Bounds: the fp32 ones of the grid.
+    Both backward forms: scores evaluated once (with the dS scratch) and two passes (without)."""
+    from kernels_b200.streaming_attention import kernel as K
     from kernels_b200.streaming_attention import streaming_attention
+
+    if not scratch:
+        monkeypatch.setattr(K, "_ds_scratch_for", lambda *_: None)
 
     g = torch.Generator(device="cuda").manual_seed(T + D)
 
@@ -361,7 +367,10 @@ def test_fp32_tiles_edges_and_layouts(D, T, c, back, layout):
     got_in = [t.requires_grad_() for t in (q, k, v)]
     got = streaming_attention(*got_in, lens, c, back)
     assert (got - want).abs().max() <= 5e-6
-    for a, b in zip(torch.autograd.grad(got, got_in, do), torch.autograd.grad(want, ref, do.double())):
+    before = K._lib.launch_count()
+    grads = torch.autograd.grad(got, got_in, do)
+    assert K._lib.launch_count() - before == (3 if scratch else 2)
+    for a, b in zip(grads, torch.autograd.grad(want, ref, do.double())):
         assert (a - b).abs().max() <= 5e-5
 
 def test_ordinary_calls_equal_the_compiled_function():
@@ -389,3 +398,31 @@ def test_ordinary_calls_equal_the_compiled_function():
     dq, = torch.autograd.grad(o, (q,), do.clone().requires_grad_(), create_graph=True)
     with pytest.raises(RuntimeError):
         dq.float().sum().backward()
+
+
+def test_fp32_backward_scratch_belongs_to_the_graph_that_captured_it():
+    """A captured backward takes its dS scratch from the graph's memory: later calls on the capturing stream neither use
+    nor replace it, and a replay after them gives the first result again."""
+    from kernels_b200.streaming_attention import kernel as K
+
+    g = torch.Generator(device="cuda").manual_seed(7)
+    q, k, v, do = (torch.randn(1, 2, 150, 64, generator=g, device="cuda") for _ in range(4))
+
+    def grads(a, b, c, d):
+        o, lse = torch.ops.alexdremov_streaming_attention.forward(a, b, c, None, 16, 2, 0.125, False, True, False, "ieee")
+        return torch.ops.alexdremov_streaming_attention.backward(a, b, c, None, o, lse, d, 16, 2, 0.125, False, False, "ieee")
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = [t.clone() for t in grads(q, k, v, do)]
+        side.synchronize()
+        kept = dict(K._ds_scratch)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            got = grads(q, k, v, do)
+        assert {i: b.data_ptr() for i, b in K._ds_scratch.items()} == {i: b.data_ptr() for i, b in kept.items()}
+        grads(*(torch.randn(1, 2, 700, 64, generator=g, device="cuda") for _ in range(4)))
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
