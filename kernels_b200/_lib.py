@@ -211,11 +211,12 @@ def launch(entry, params, device: torch.device) -> int:
 
 def plain_call(*tensors) -> bool:
     """Whether a call on these tensors is ordinary eager execution on a GPU: nothing traces, transforms or intercepts
-    it (compilation, functorch transforms, forward-mode AD, saved-tensor hooks, dispatch or function modes, tensor
+    it (compilation, jit tracing, functorch transforms, forward-mode AD, saved-tensor hooks, dispatch or function modes, tensor
     subclasses).  Entry points that have a shorter way for such calls ask this and leave everything else as it is."""
     return (
         not torch.compiler.is_compiling()
         and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda for t in tensors)
+        and torch._C._get_tracing_state() is None
         and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
         and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
         and torch._C._autograd._top_saved_tensors_default_hooks(True) is None

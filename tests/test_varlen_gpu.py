@@ -32,6 +32,10 @@ def _cu(lens):
     (2, 2, 260, 128, 32, 2, torch.float16, [5, 130, 256, 257, 1, 127, 128, 129, 0, 260]),  # every kind of last tile
     (8, 8, 2600, 128, 64, 2, torch.bfloat16, [2600, 130, 2500]),  # more tiles per sequence than CTAs: a CTA's next
     (8, 8, 2600, 64, 100, 1, torch.float16, [130, 2600, 2571]),   # item is of the same sequence
+    # few tiles per sequence, more items than CTAs: the padded and the one-launch call shift their items from wave to
+    # wave, the launches per sequence do not
+    (4, 4, 500, 64, 10, 4, torch.float16, [(37 * i) % 501 for i in range(60)]),
+    (4, 2, 1000, 128, 64, 2, torch.bfloat16, [(61 * i) % 1001 for i in range(40)]),
 ])
 @pytest.mark.parametrize("single_launch", [True, False])
 def test_packed_equals_padded_bitwise(H, Hk, T, D, c, back, dtype, lens, single_launch):
