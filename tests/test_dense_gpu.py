@@ -166,17 +166,37 @@ def test_softmax_many_calls_side_stream_poisoned_output():
         f"|err| {float(err.max()):.3e}; {int((err > 1e-6).sum())} elements off, {int(torch.isnan(got).sum())} never written")
 
 
+def _softmax_bound(dtype, cols):
+    """Relative bound on a softmax element and an absolute floor.  In units of 2^-24: the exponent's rounding (|x - max| up
+    to 48 in these tests), the longest chain of additions of one thread (64 elements of a vector kernel, cols / 256 of the
+    scalar one) and 16 for the tree above it, exp2f / expf, the reciprocal and the products.  Then half a unit in the last
+    place of a 16-bit result; the floor is half the spacing of the type's subnormals."""
+    rel = (48 + 64 + cols // 256 + 16) * 2.0 ** -24
+    half_ulp, floor = {torch.float32: (0.0, 2.0 ** -125), torch.float16: (2.0 ** -11, 2.0 ** -25), torch.bfloat16: (2.0 ** -8, 2.0 ** -125)}[dtype]
+    return rel + half_ulp, floor
+
+
+def _softmax_into(xv, yv):
+    """``kb_softmax_fwd`` on rows where they lie (the public function allocates its own, aligned result)."""
+    import ctypes
+
+    from kernels_b200 import _lib
+
+    p = _lib.SoftmaxParams()
+    p.x, p.y = xv.data_ptr(), yv.data_ptr()
+    p.rows, p.cols = xv.shape
+    p.x_row_stride, p.y_row_stride, p.dtype = xv.stride(0), yv.stride(0), _lib.dtype_code(xv.dtype)
+    _lib.check(_lib.load().kb_softmax_fwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream), "kb_softmax_fwd")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("cols", [1, 7, 15, 129, 1003, 2055, 5001, 16390, 20000, 32773])
 @pytest.mark.parametrize("start", [0, 1, 5])
 def test_softmax_rows_off_16_byte_boundaries(dtype, cols, start):
-    """Odd row lengths and first rows off a boundary, against the 64-bit result: fp32 to 1e-6 absolute (results are
-    at most 1), 16-bit to half a unit in the last place of the result (plus that fp32 error).  Nothing outside the
-    rows is written; an infinity, a NaN and a row of only -inf come out as the tensor expressions give them."""
-    from kernels_b200 import _lib
-
-    import ctypes
-
+    """Odd row lengths and first rows off a boundary, against the 64-bit result, element by element.  In four rows one
+    element holds nearly all the mass: the first, the last, the first on a boundary and the first after the last vector
+    (leaving it out of the maximum or the sum would show).  Nothing outside the rows is written; an infinity, a NaN and
+    a row of only -inf come out as the tensor expressions give them."""
     rows = 9
     g = torch.Generator(device="cuda").manual_seed(cols)
     x = (torch.randn(rows * cols + start, generator=g, device="cuda") * 2.0).to(dtype)
@@ -185,14 +205,45 @@ def test_softmax_rows_off_16_byte_boundaries(dtype, cols, start):
     xv[2, cols // 2] = float("inf")
     xv[3, cols - 1] = float("nan")
     xv[4, 0] = -float("inf") if cols > 1 else 0.0
+    per_vec = 16 // x.element_size()
+    for row, place in ((5, "first"), (6, "last"), (7, "boundary"), (8, "tail")):
+        head = min(-(start + row * cols) % per_vec, cols)  # elements before the row's first 16-byte boundary
+        at = {"first": 0, "last": cols - 1, "boundary": head, "tail": head + (cols - head) // per_vec * per_vec}[place]
+        xv[row, min(at, cols - 1)] = 30.0
     y = torch.full((rows * cols + start + 16,), 7.0, dtype=dtype, device="cuda")
-    p = _lib.SoftmaxParams()
-    p.x, p.y = xv.data_ptr(), y[start:].data_ptr()
-    p.rows, p.cols, p.x_row_stride, p.y_row_stride, p.dtype = rows, cols, cols, cols, _lib.dtype_code(dtype)
-    _lib.check(_lib.load().kb_softmax_fwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream), "kb_softmax_fwd")
-    got, want = y[start:start + rows * cols].view(rows, cols), torch.softmax(xv.double(), dim=-1)
+    got = y[start:start + rows * cols].view(rows, cols)
+    _softmax_into(xv, got)
+    want = torch.softmax(xv.double(), dim=-1)
     assert (y[:start] == 7).all() and (y[start + rows * cols:] == 7).all()
-    half_ulp = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
     assert torch.equal(got.isnan(), want.isnan())
-    err = (got.double() - want).nan_to_num(0.0).abs()
-    assert (err <= 1e-6 + half_ulp * want.nan_to_num(0.0)).all(), float(err.max())
+    rel, floor = _softmax_bound(dtype, cols)
+    excess = (got.double() - want).nan_to_num(0.0).abs() - rel * want.nan_to_num(0.0)
+    assert float(excess.max()) <= floor
+
+
+# one length of every instance (1, 2, 4, 8 vectors a lane; 2, 4, 8 a thread of 256; 8 of 512; 1 024 threads in fp32; the
+# scalar kernel) for 16-byte vectors of 8 and of 4 elements, aligned and odd
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("cols", [96, 97, 200, 201, 480, 481, 1000, 1001, 2000, 2001, 4000, 4001, 8000, 8001, 16000, 16001, 20000, 20001, 32000,
+                                  32001, 40000, 40001])
+def test_softmax_rows_of_extreme_values(dtype, cols):
+    """Rows at the ends of the type's range (a mask of its lowest value among them), whole and with one ordinary element,
+    against the 64-bit result: 1 / n where all elements are equal, whatever their size."""
+    from kernels_b200.softmax import softmax
+
+    info = torch.finfo(dtype)
+    values = [v for v in (info.min, info.max, 3e9, -1e10, 1e10, -1e12, 65504.0, -65504.0, 7e4, -7e4, 1e6, -1e8) if abs(v) <= info.max]
+    x = torch.empty((4 * len(values), cols), dtype=dtype, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    for i, v in enumerate(values):
+        x[4 * i:4 * i + 4] = v
+        x[4 * i + 1, cols // 3] = 0.5  # one ordinary element in a row of the value
+        x[4 * i + 2] = torch.randn(cols, generator=g, device="cuda").to(dtype)  # one element of the value in an ordinary row
+        x[4 * i + 2, cols - 1] = v
+        x[4 * i + 3, :cols // 2] = info.min  # half the row masked
+    got = softmax(x)
+    want = torch.softmax(x.double(), dim=-1)
+    rel, floor = _softmax_bound(dtype, cols)
+    assert not got.isnan().any(), [values[i // 4] for i in range(len(x)) if got[i].isnan().any()]
+    excess = (got.double() - want).abs() - rel * want
+    assert float(excess.max()) <= floor
