@@ -169,28 +169,26 @@ struct Cursor {
   __device__ __forceinline__ int q0() const { return (it.qr.begin + tq) * kBQ; }   // its first query row
 };
 
-// `prev` is the item decoded before (b = -1: none): consecutive items mostly share the batch index
-// and with it the sequence length, which saves the global load.
+// First row and length of sequence b.  Both decoders read them for every item (the loads hit L1) and keep nothing from
+// the item before.  They used to take them over from it when the sequence was the same; in the packed dQ kernel that came
+// with a wrong dQ for every item after the first of a sequence on its CTA, which went away when the values were read and
+// the item structs initialised, in one change.  Why is not known: as C++ the carry-over was right.
 template <bool PACKED>
-__device__ __forceinline__ Item decode_item(const FusedArgs& a, int item, int n_ktiles, const Item& prev) {
+__device__ __forceinline__ void read_sequence(const FusedArgs& a, int b, int& row0, int& len) {
+  row0 = PACKED ? a.cu[b] : 0;
+  if (PACKED) len = kb_min_i32(a.cu[b + 1] - row0, a.T);
+  else len = a.lens ? kb_clamp_len(a.lens[(int64_t)b * a.lens_stride], a.T) : a.T;
+}
+
+template <bool PACKED>
+__device__ __forceinline__ Item decode_item(const FusedArgs& a, int item, int n_ktiles) {
   Item it;
   const int bh = kb_fastdiv(item, a.fd_tiles);
   it.kt = item - bh * n_ktiles;
   it.b = kb_fastdiv(bh, a.fd_Hk);
   it.hk = bh - it.b * a.Hk;
   it.k0 = it.kt * kBK;
-  it.row0 = 0;
-  if (PACKED) {
-    if (it.b == prev.b) {
-      it.row0 = prev.row0;
-      it.len = prev.len;
-    } else {
-      it.row0 = a.cu[it.b];
-      it.len = kb_min_i32(a.cu[it.b + 1] - it.row0, a.T);
-    }
-  } else {
-    it.len = !a.lens ? a.T : (it.b == prev.b ? prev.len : kb_clamp_len(a.lens[(int64_t)it.b * a.lens_stride], a.T));
-  }
+  read_sequence<PACKED>(a, it.b, it.row0, it.len);
   it.qr = kb_bwd_q_range_fd(it.k0, kBQ, kBK, it.len, a.c, a.back, a.fd_c);
   return it;
 }
@@ -203,7 +201,7 @@ template <bool PACKED>
 __device__ __forceinline__ void seek_live(const FusedArgs& a, Cursor& c, int n_items, int n_ktiles) {
   c.valid = false;
   for (; c.walk.item() < n_items; c.walk.next()) {
-    c.it = decode_item<PACKED>(a, c.walk.item(), n_ktiles, c.it);
+    c.it = decode_item<PACKED>(a, c.walk.item(), n_ktiles);
     if (c.it.qr.begin < c.it.qr.end) {
       c.valid = true;
       return;
@@ -212,10 +210,8 @@ __device__ __forceinline__ void seek_live(const FusedArgs& a, Cursor& c, int n_i
 }
 template <bool PACKED>
 __device__ __forceinline__ Cursor cursor_first(const FusedArgs& a, int n_items, int n_ktiles) {
-  Cursor c{KbItemWalk<>(a.item_rot)};
-  c.n = c.g = c.t = c.tq = c.hq = 0;
+  Cursor c{KbItemWalk<>(a.item_rot)};  // (everything after the walk starts as zero)
   c.group = a.group;
-  c.it.b = -1;
   seek_live<PACKED>(a, c, n_items, n_ktiles);
   return c;
 }
@@ -461,10 +457,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       // This thread keeps no cursor: all it needs of the schedule is how many tiles each live item has.
       // Tiles of the first live item from the walk's position on, 0 if there is none.
       auto next_live = [&](KbItemWalk<>& walk) -> int {
-        Item prev;
-        prev.b = -1;
         for (; walk.item() < n_items; walk.next()) {
-          const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles, prev);
+          const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles);
           if (it.qr.begin < it.qr.end) return (it.qr.end - it.qr.begin) * a.group;
         }
         return 0;
@@ -736,10 +730,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     int n = 0;
     bool ok = true;
-    Item it = {};
-    it.b = -1;
     for (KbItemWalk<> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
-      it = decode_item<PACKED>(a, walk.item(), n_ktiles, it);
+      const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles);
       const int kr = it.k0 + row;
       if (it.qr.begin >= it.qr.end) {
         // the whole key tile lies in the padding: its gradients are zeros (rare; plain stores).  A packed
@@ -928,21 +920,13 @@ struct DqItem {
   KbTileRange kr;  // key tiles [begin, end) the query tile visits: the forward schedule
 };
 template <bool PACKED>
-__device__ __forceinline__ DqItem decode_dq_item(const FusedArgs& a, int item, int n_qtiles, const DqItem& prev) {
+__device__ __forceinline__ DqItem decode_dq_item(const FusedArgs& a, int item, int n_qtiles) {
   DqItem it;
   const int bh = kb_fastdiv(item, a.fd_tiles);
   it.qt = item - bh * n_qtiles;
   it.b = kb_fastdiv(bh, a.fd_H);
   it.h = bh - it.b * a.H;
-  it.row0 = 0;
-  if (PACKED) {
-    // always read: taking the offset and length over from `prev` when the sequence is the same gave wrong dQ for
-    // every item after the first of a sequence on its CTA (the loads hit L1, and these roles run ahead or wait for HBM)
-    it.row0 = a.cu[it.b];
-    it.len = kb_min_i32(a.cu[it.b + 1] - it.row0, a.T);
-  } else {
-    it.len = !a.lens ? a.T : (it.b == prev.b ? prev.len : kb_clamp_len(a.lens[(int64_t)it.b * a.lens_stride], a.T));
-  }
+  read_sequence<PACKED>(a, it.b, it.row0, it.len);
   it.kr = kb_fwd_kv_range_fd(it.qt * kBQ, kBQ, kBK, it.len, a.c, a.back, a.fd_c);
   return it;
 }
@@ -991,10 +975,8 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       prefetch_tensormap(&tm_k);
       int u = 0;
       bool ok = true;
-      DqItem it = {};
-      it.b = -1;
       for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
-        it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t, it);
+        const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
         for (int j = it.kr.begin; j < it.kr.end; ++j, ++u) {
           const int s = u % kDqStages;
           if (u >= kDqStages && !mbar_wait<kRelaxedNs>(&sm.empty[s], ((u / kDqStages) - 1) & 1, ctx, kWDqEmpty)) { ok = false; break; }
@@ -1013,10 +995,8 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       constexpr uint32_t idesc = make_idesc(BF16, kBQ, D, true, true);  // A = dS read MN-major (rows = keys), B = K MN-major
       int u = 0, m = 0;
       bool ok = true;
-      DqItem it = {};
-      it.b = -1;
       for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
-        it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t, it);
+        const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
         if (it.kr.begin >= it.kr.end) continue;
         const uint32_t acc = tmem + (m & 1) * 128;
         if (m >= 2 && !mbar_wait(&sm.acc_free[m & 1], ((m >> 1) - 1) & 1, ctx, kWDqAccFree)) break;
@@ -1042,10 +1022,8 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
     int m = 0;
     bool ok = true;
-    DqItem it = {};
-    it.b = -1;
     for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
-      it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t, it);
+      const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
       const int qi = it.qt * kBQ + row;
       if (it.kr.begin >= it.kr.end) {
         // the whole query tile lies in the padding: its gradient is zero (rare; plain stores); a packed batch

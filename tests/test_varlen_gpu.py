@@ -32,6 +32,12 @@ def _cu(lens):
     (2, 2, 260, 128, 32, 2, torch.float16, [5, 130, 256, 257, 1, 127, 128, 129, 0, 260]),  # every kind of last tile
     (8, 8, 2600, 128, 64, 2, torch.bfloat16, [2600, 130, 2500]),  # more tiles per sequence than CTAs: a CTA's next
     (8, 8, 2600, 64, 100, 1, torch.float16, [130, 2600, 2571]),   # item is of the same sequence
+    # the same in the long-item class (head dim 128, chunks of 128 rows or more), first of a sequence between others
+    (8, 8, 2600, 128, 256, 2, torch.bfloat16, [130, 2600, 2500]),
+    (8, 8, 2600, 128, 130, 3, torch.float16, [2571, 2600, 1]),
+    # ... and with shared key/value heads: more (key tile, key/value head) items per sequence than CTAs too
+    (16, 8, 2600, 128, 256, 2, torch.bfloat16, [2500, 77, 2600]),
+    (16, 8, 2600, 64, 64, 2, torch.float16, [300, 2600, 2500]),
     # few tiles per sequence, more items than CTAs: the padded and the one-launch call shift their items from wave to
     # wave, the launches per sequence do not
     (4, 4, 500, 64, 10, 4, torch.float16, [(37 * i) % 501 for i in range(60)]),
@@ -72,6 +78,44 @@ def test_packed_equals_padded_bitwise(H, Hk, T, D, c, back, dtype, lens, single_
     assert torch.equal(qs.grad, _pack(qp.grad, lens))
     assert torch.equal(ks.grad, _pack(kp.grad, lens))
     assert torch.equal(vs.grad, _pack(vp.grad, lens))
+
+
+@pytest.mark.parametrize("D,c,back,dtype", [(128, 64, 2, torch.bfloat16), (128, 256, 2, torch.bfloat16), (64, 100, 1, torch.float16)])
+def test_more_tiles_per_sequence_than_ctas_against_64_bits(D, c, back, dtype):
+    """Padded and packed, ragged, every CTA of the main and the dQ kernel meeting several tiles of one sequence: every
+    128-row tile of every head against the 64-bit result (a tile computed with another item's sequence would be off by
+    about 1).  Bounds: four times the largest error of a tile measured over 800 random cases (3.3e-3 bf16, 4.3e-4 fp16)."""
+    from kernels_b200.streaming_attention import streaming_attention, streaming_attention_varlen
+
+    H, T, lens = 8, 2600, [130, 2600, 2571]
+    assert H * -(-T // 128) > torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v, do = (torch.randn(3, H, T, D, generator=g, device="cuda").to(dtype) for _ in range(4))
+    chunk = torch.arange(T, device="cuda") // c
+    diff = chunk[:, None] - chunk[None]
+    mask = (diff >= 0) & (diff <= back)
+
+    padded_in = [t.clone().requires_grad_() for t in (q, k, v)]
+    padded = streaming_attention(*padded_in, torch.tensor(lens, dtype=torch.int32, device="cuda"), c, back)
+    padded = [padded.detach(), *torch.autograd.grad(padded, padded_in, do)]
+    packed_in = [_pack(t, lens).requires_grad_() for t in (q, k, v)]
+    packed = streaming_attention_varlen(*packed_in, _cu(lens), c, back)
+    packed = [packed.detach(), *torch.autograd.grad(packed, packed_in, _pack(do, lens))]
+    bound = {torch.bfloat16: 1.3e-2, torch.float16: 1.8e-3}[dtype]
+    r0 = 0
+    for b, L in enumerate(lens):
+        ref = [t[b, :, :L].double().requires_grad_() for t in (q, k, v)]
+        scores = (ref[0] @ ref[1].mT * D**-0.5).masked_fill(~mask[:L, :L], -1e300)
+        want = torch.softmax(scores, -1) @ ref[2]
+        want = [want.detach(), *torch.autograd.grad(want, ref, do[b, :, :L].double())]
+        for name, exact, pad, pack in zip(("o", "dq", "dk", "dv"), want, padded, packed):
+            for form, got in (("padded", pad[b, :, :L]), ("packed", pack[r0:r0 + L].transpose(0, 1))):
+                for t0 in range(0, L, 128):
+                    e, x = exact[:, t0:t0 + 128], got[:, t0:t0 + 128].double()
+                    rel = (x - e).norm(dim=(1, 2)) / e.norm(dim=(1, 2))
+                    assert float(rel.max()) <= bound, (form, name, b, t0, rel.tolist())
+            assert not pad[b, :, L:].any(), name  # padding rows are zeros
+        r0 += L
 
 
 def test_packed_against_oracle_per_sequence():
