@@ -25,23 +25,28 @@ from .. import _lib
 logger = logging.getLogger(__name__)
 
 _SUPPORTED_HEAD_DIMS = (16, 32, 64, 128, 256)
-# Largest dS scratch the backward op will allocate for the single-evaluation kernels.
+# Largest dS scratch the backward op will allocate for the single-evaluation kernels, and for those of fp32.
 _MAX_DS_SCRATCH_BYTES = 48 << 30
+_MAX_F32_DS_SCRATCH_BYTES = 1 << 30
 
 
 _device_total_bytes: dict = {}
 _ds_scratch: dict = {}
 
 
-def _ds_scratch_for(device: torch.device, stream_ptr: int, nbytes: int):
-    """The dS scratch of the single-evaluation backward: one buffer per (device, stream), kept between
-    calls and grown when a larger problem arrives, or ``None`` when the problem's scratch is withheld.
+def _ds_scratch_for(device: torch.device, stream_ptr: int, nbytes: int, dtype: torch.dtype):
+    """The dS scratch of the single-evaluation backward, or ``None`` when the problem's scratch is withheld.
+
+    16-bit: one buffer per (device, stream), kept between calls and grown when a larger problem arrives.  Calls on one
+    stream run one after the other, so they can share a buffer; calls on different streams get their own.
+    fp32: memory of the call's own, back in torch's pool when the op returns.  Its tiles take 4 bytes per score and the
+    two-pass kernels serve the same calls at 1.2-1.5 times the time, so a program in full precision keeps nothing it did
+    not ask for and gives at most ``_MAX_F32_DS_SCRATCH_BYTES`` for the duration of the backward.
 
     Whether to provide it is decided from sizes alone (no query of the driver on the hot path): at most
-    ``_MAX_DS_SCRATCH_BYTES`` and at most a quarter of the device's total memory.  Calls on one stream run
-    one after the other, so they can share a buffer; calls on different streams get their own.
+    ``_MAX_DS_SCRATCH_BYTES`` (fp32: ``_MAX_F32_DS_SCRATCH_BYTES``) and at most a quarter of the device's total memory.
     """
-    if nbytes <= 0:
+    if nbytes <= 0 or (dtype == torch.float32 and nbytes > _MAX_F32_DS_SCRATCH_BYTES):
         return None
     idx = device.index if device.index is not None else torch.cuda.current_device()
     total = _device_total_bytes.get(idx)
@@ -49,9 +54,12 @@ def _ds_scratch_for(device: torch.device, stream_ptr: int, nbytes: int):
         total = _device_total_bytes[idx] = torch.cuda.get_device_properties(idx).total_memory
     if nbytes > _MAX_DS_SCRATCH_BYTES or nbytes > total // 4:
         return None
-    if torch.cuda.is_current_stream_capturing():
-        # a graph keeps what it captured: memory of its own, not a buffer that later calls share, grow and free
-        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    if dtype == torch.float32 or torch.cuda.is_current_stream_capturing():
+        # (a graph keeps what it captured: memory of its own, not a buffer that later calls share, grow and free)
+        try:
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            return None  # the two-pass kernels need no such scratch
     key = (idx, stream_ptr)
     buf = _ds_scratch.get(key)
     if buf is None or buf.numel() < nbytes:
@@ -187,9 +195,8 @@ def attention_backward_adapter(
     ``[B, H, T]`` fp32 (reference: kernel.py:1380) and, for the backward kernels that evaluate
     the scores once, room for the dS tiles (``kb_sa_bwd_workspace_bytes``, fp32:
     ``kb_sa_bwd_generic_workspace_bytes``; it grows with
-    ``(back_contexts + 1) * context_size``; one buffer per device and stream, kept between calls).
-    When that room exceeds ``_MAX_DS_SCRATCH_BYTES`` or a quarter of the device's memory, it is
-    withheld and the library runs its two-pass kernels, which need none.  ``do`` may arrive in another dtype or with any strides
+    ``(back_contexts + 1) * context_size``; see ``_ds_scratch_for``).  Where it is withheld the library
+    runs its two-pass kernels, which need none.  ``do`` may arrive in another dtype or with any strides
     (``tests/test_streaming_attention.py:98-112``): it is cast to
     ``q``'s dtype first.
     """
@@ -220,7 +227,7 @@ def attention_backward_adapter(
         workspace_bytes = lib.kb_sa_bwd_generic_workspace_bytes if q.dtype == torch.float32 else lib.kb_sa_bwd_workspace_bytes
         ws_bytes = int(workspace_bytes(
             B, H, T, D, _lib.dtype_code(q.dtype), _clamp_i32(context_size), _clamp_i32(back_contexts)))
-        ds_ws = _ds_scratch_for(q.device, torch.cuda.current_stream(q.device).cuda_stream, ws_bytes)
+        ds_ws = _ds_scratch_for(q.device, torch.cuda.current_stream(q.device).cuda_stream, ws_bytes, q.dtype)
     lens_keep, lens_ptr, lens_stride = _lens_arg(lens, q.device)
     p = _lib.SaBwdParams()
     p.q, p.k, p.v, p.o, p.d_o = (_lib.tensor4(t) for t in (q, k, v, o, do))

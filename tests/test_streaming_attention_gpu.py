@@ -426,3 +426,60 @@ def test_fp32_backward_scratch_belongs_to_the_graph_that_captured_it():
         graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_fp32_backward_holds_no_memory_and_bounds_its_scratch(monkeypatch):
+    """An fp32 backward leaves no scratch behind, takes none above its limit or where the allocation fails, and gives its
+    result either way; a 16-bit one inside a capture falls back in the same way."""
+    from kernels_b200.streaming_attention import kernel as K
+
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v, do = (torch.randn(2, 2, 500, 64, generator=g, device="cuda") for _ in range(4))
+
+    def grads(*tensors):
+        a, b, c, d = tensors
+        o, lse = torch.ops.alexdremov_streaming_attention.forward(a, b, c, None, 32, 4, 0.125, False, True, False, "ieee")
+        n0 = K._lib.launch_count()
+        out = torch.ops.alexdremov_streaming_attention.backward(a, b, c, None, o, lse, d, 32, 4, 0.125, False, False, "ieee")
+        return out, K._lib.launch_count() - n0
+
+    need = K._lib.load().kb_sa_bwd_generic_workspace_bytes(2, 2, 500, 64, K._lib.KB_F32, 32, 4)
+    kept = {i: b.data_ptr() for i, b in K._ds_scratch.items() if b is not None}
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    once, launches = grads(q, k, v, do)
+    held = torch.cuda.memory_allocated() - before
+    assert launches == 3 and need > 1 << 20
+    assert held <= 3 * (q.numel() * 4 + 512)  # dq, dk, dv and nothing else
+    assert {i: b.data_ptr() for i, b in K._ds_scratch.items() if b is not None} == kept
+
+    real_empty = torch.empty
+
+    def full(*a, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("no room (test)")
+        return real_empty(*a, **kw)
+
+    for limit, empty in ((need - 1, real_empty), (K._MAX_F32_DS_SCRATCH_BYTES, full)):
+        with monkeypatch.context() as m:
+            m.setattr(K, "_MAX_F32_DS_SCRATCH_BYTES", limit)
+            m.setattr(torch, "empty", empty)
+            twice, launches = grads(q, k, v, do)
+        assert launches == 2
+        for a, b in zip(once, twice):  # two orders of the same fp32 sums: the grid's bound for fp32 gradients
+            assert (a - b).abs().max() <= 5e-5
+
+    half = [t.half() for t in (q, k, v, do)]
+    want, _ = grads(*half)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side), monkeypatch.context() as m:
+        grads(*half)  # (whatever is looked up at a first call)
+        side.synchronize()
+        m.setattr(torch, "empty", full)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            got, _ = grads(*half)
+        graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert (a.float() - b.float()).abs().max() <= 1e-2  # the grid's bound for fp16 gradients
