@@ -285,10 +285,21 @@ def _setup_context(ctx, inputs, output):
     ctx.precision = precision
 
 
+def _rows_in_place(t: torch.Tensor) -> bool:
+    """Whether the kernels read ``t`` where it lies as fast as a dense copy: dense rows on 16-byte boundaries."""
+    per_vec = 16 // t.element_size()
+    *outer, inner = t.stride()
+    return inner == 1 and t.data_ptr() % 16 == 0 and all(s > 0 and s % per_vec == 0 for s in outer)
+
+
 def _backward(ctx, do, dlse):
     # Gradients through LSE are not supported (dlse is ignored), as in the reference
     # (kernel.py:1498-1523).
     q, k, v, o, lse, lens = ctx.saved_tensors
+    # A gradient may come expanded (``o.sum()``) or as every other element of something: a dense copy, which the
+    # compiled function makes of every gradient that is not dense, keeps it on the tcgen05 kernels.
+    if _lib.plain_call(do) and not do.is_contiguous() and not _rows_in_place(do):
+        do = do.contiguous()
     DQ, DK, DV = torch.ops.alexdremov_streaming_attention.backward(
         q=q, k=k, v=v, lens=lens, o=o, lse=lse, do=do,
         context_size=ctx.context_size, back_contexts=ctx.back_contexts, sm_scale=ctx.sm_scale,

@@ -483,3 +483,32 @@ def test_fp32_backward_holds_no_memory_and_bounds_its_scratch(monkeypatch):
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert (a.float() - b.float()).abs().max() <= 1e-2  # the grid's bound for fp16 gradients
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float16, 64), (torch.bfloat16, 128), (torch.float32, 64), (torch.float16, 32)])
+def test_gradients_of_any_layout_take_the_same_kernels(dtype, D):
+    """Expanded, strided, misaligned and transposed output gradients give the bits of a dense one and launch the same
+    kernels (the same number of them, and none of the slower ones: equal bits)."""
+    from kernels_b200 import _lib
+    from kernels_b200.streaming_attention import streaming_attention
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    B, H, T = 2, 3, 150
+    q, k, v = (torch.randn(B, H, T, D, generator=g, device="cuda").to(dtype).requires_grad_() for _ in range(3))
+    lens = torch.tensor([T, 77], dtype=torch.int32, device="cuda")
+    one = torch.randn(1, device="cuda", generator=g).to(dtype)
+    row = torch.randn(1, 1, 1, D, device="cuda", generator=g).to(dtype)
+    wide = torch.randn(B, H, T, 2 * D + 2, device="cuda", generator=g).to(dtype)
+    layouts = {
+        "expanded": one.expand(B, H, T, D), "one row": row.expand(B, H, T, D), "one head": wide[:, :1, :, :D].expand(B, H, T, D),
+        "every other": wide[..., : 2 * D : 2], "misaligned": wide[..., 1:D + 1], "rows off": wide[..., :D],
+        "transposed": torch.randn(B, T, H, D, device="cuda", generator=g).to(dtype).transpose(1, 2),
+    }
+    o = streaming_attention(q, k, v, lens, 24, 2)
+    for name, do in layouts.items():
+        n0 = _lib.launch_count()
+        want = torch.autograd.grad(o, (q, k, v), do.contiguous(), retain_graph=True)
+        n1 = _lib.launch_count()
+        got = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
+        assert _lib.launch_count() - n1 == n1 - n0, name
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), name
