@@ -389,8 +389,10 @@ def streaming_attention(
     # The compiled function is one operator call, so compiling it changes no result.  An ordinary call goes to the
     # operator directly: guards, the compiled wrapper and its autograd function took 300 of the 500 us of host time of
     # a forward + backward pass, more than the kernels of a small one.  Everything that looks inside (an outer
-    # compilation, transforms, hooks, modes) still meets the compiled function.
-    if _lib.plain_call(q, k, v):
+    # compilation, transforms, hooks, modes) still meets the compiled function, and so do numbers that are not Python's
+    # own: it refuses numpy's and zero-dimensional tensors, which the operator alone would take.
+    numbers = type(context_size) in (int, bool) and type(back_contexts) in (int, bool) and type(sm_scale) in (type(None), int, float)
+    if numbers and _lib.plain_call(q, k, v):
         attention = _streaming_attention_eager
     else:
         attention = _streaming_attention

@@ -512,3 +512,20 @@ def test_gradients_of_any_layout_take_the_same_kernels(dtype, D):
         got = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
         assert _lib.launch_count() - n1 == n1 - n0, name
         assert all(torch.equal(a, b) for a, b in zip(got, want)), name
+
+
+def test_numbers_that_are_not_pythons_own_are_refused():
+    """Chunk length, look-back and scale as numpy numbers or zero-dimensional tensors: refused on an ordinary call as
+    inside a compiled function."""
+    import numpy as np
+
+    from kernels_b200.streaming_attention import streaming_attention
+
+    q, k, v = (torch.randn(1, 2, 64, 64, device="cuda", dtype=torch.float16) for _ in range(3))
+    for args, kw in (((np.int64(16), 2), {}), ((16, np.int32(2)), {}), ((torch.tensor(16), 2), {}), ((16, 2), dict(sm_scale=np.float32(0.1))),
+                     ((16, 2), dict(sm_scale=torch.tensor(0.1))), ((16.0, 2), {})):
+        torch._dynamo.reset()
+        with pytest.raises(RuntimeError):
+            streaming_attention(q, k, v, None, *args, **kw)
+    torch._dynamo.reset()
+    assert torch.equal(streaming_attention(q, k, v, None, 16, 2, sm_scale=1), streaming_attention(q, k, v, None, 16, 2, sm_scale=1.0))
