@@ -198,13 +198,29 @@ def tensor4(t: torch.Tensor) -> Tensor4:
     return Tensor4(t.data_ptr(), strides[:4])
 
 
+# What torch itself asks on its hot paths.  These are not public: with a torch that lacks one, ``launch`` goes through the
+# public calls and no call counts as plain.
+try:
+    _current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+except AttributeError:
+    _current_device = _raw_stream = None
+try:
+    _tracing_state, _dispatch_modes = torch._C._get_tracing_state, torch._C._len_torch_dispatch_stack
+    _function_modes, _transforms_active = torch._C._len_torch_function_stack, torch._C._are_functorch_transforms_active
+    _saved_tensor_hooks, _forward_ad = torch._C._autograd._top_saved_tensors_default_hooks, torch.autograd.forward_ad
+    _forward_ad._current_level
+    _can_tell_plain = True
+except AttributeError:
+    _can_tell_plain = False
+
+
 def launch(entry, params, device: torch.device) -> int:
     """``entry(&params, stream)`` on ``device`` and its current stream; the status code.  The device is only switched
     where it is not current already, and the stream is asked for as the handle it is needed as: a few microseconds of
     calls that take about twenty."""
     index = device.index
-    if index == torch._C._cuda_getDevice():
-        return entry(C.byref(params), torch._C._cuda_getCurrentRawStream(index))
+    if _current_device is not None and index == _current_device():
+        return entry(C.byref(params), _raw_stream(index))
     with torch.cuda.device(device):
         return entry(C.byref(params), torch.cuda.current_stream(device).cuda_stream)
 
@@ -215,11 +231,12 @@ def plain_call(*tensors) -> bool:
     subclasses).  Entry points that have a shorter way for such calls ask this and leave everything else as it is."""
     return (
         not torch.compiler.is_compiling()
+        and _can_tell_plain
         and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda for t in tensors)
-        and torch._C._get_tracing_state() is None
-        and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-        and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
-        and torch._C._autograd._top_saved_tensors_default_hooks(True) is None
+        and _tracing_state() is None
+        and _dispatch_modes() == 0 and _function_modes() == 0
+        and not _transforms_active() and _forward_ad._current_level < 0
+        and _saved_tensor_hooks(True) is None
     )
 
 

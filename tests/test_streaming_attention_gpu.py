@@ -529,3 +529,90 @@ def test_numbers_that_are_not_pythons_own_are_refused():
             streaming_attention(q, k, v, None, *args, **kw)
     torch._dynamo.reset()
     assert torch.equal(streaming_attention(q, k, v, None, 16, 2, sm_scale=1), streaming_attention(q, k, v, None, 16, 2, sm_scale=1.0))
+
+
+def test_only_ordinary_calls_leave_the_compiled_function(monkeypatch):
+    """Which of the two ways a call takes: transforms, forward-mode AD, jit tracing, modes, subclasses and saved-tensor
+    hooks meet the compiled function; tensors, parameters, no_grad, inference mode, another stream and another thread
+    go to the operator directly, and nothing does where torch cannot say."""
+    import threading
+
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from kernels_b200 import _lib
+    from kernels_b200.streaming_attention import kernel as K
+
+    taken = []
+    for name in ("_streaming_attention", "_streaming_attention_eager"):
+        monkeypatch.setattr(K, name, lambda name=name, **kw: (taken.append(name), kw["q"] * 1)[1])
+    q, k, v = (torch.randn(2, 2, 64, 64, device="cuda", dtype=torch.float16) for _ in range(3))
+
+    def call(a=q, b=k, c=v):
+        return K.streaming_attention(a, b, c, None, 16, 1)
+
+    class Sub(torch.Tensor):
+        pass
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class FunctionMode(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    def dual():
+        with torch.autograd.forward_ad.dual_level():
+            call(torch.autograd.forward_ad.make_dual(q, torch.ones_like(q)))
+
+    def within(context):
+        def run():
+            with context:
+                call()
+        return run
+
+    def thread():
+        t = threading.Thread(target=call)
+        t.start()
+        t.join()
+
+    hooks = torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t)
+    looked_into = {
+        "vmap": lambda: torch.func.vmap(call)(q[None], k[None], v[None]),
+        "jvp": lambda: torch.func.jvp(call, (q,), (q,)),
+        "grad": lambda: torch.func.grad(lambda t: call(t).float().sum())(q),
+        "forward-mode AD": dual,
+        "jit.trace": lambda: torch.jit.trace(call, (q, k, v), check_trace=False),
+        "dispatch mode": within(Mode()), "function mode": within(FunctionMode()), "default device": within(torch.device("cuda")),
+        "subclass": lambda: call(q.as_subclass(Sub)), "hooks": within(hooks),
+    }
+    ordinary = {
+        "tensors": call, "parameter": lambda: call(torch.nn.Parameter(q)), "no_grad": within(torch.no_grad()),
+        "inference mode": within(torch.inference_mode()), "stream": within(torch.cuda.stream(torch.cuda.Stream())), "thread": thread,
+    }
+    for calls, way in ((looked_into, "_streaming_attention"), (ordinary, "_streaming_attention_eager")):
+        for what, run in calls.items():
+            taken.clear()
+            run()
+            assert taken and set(taken) == {way}, (what, taken)
+    monkeypatch.setattr(_lib, "_can_tell_plain", False)
+    taken.clear()
+    call()
+    assert taken == ["_streaming_attention"]
+
+
+def test_launch_without_the_private_calls(monkeypatch):
+    """The public way to the device and the stream gives the same result, on a side stream too."""
+    from kernels_b200 import _lib
+    from kernels_b200.softmax import softmax
+
+    x = torch.randn(3, 200, device="cuda")
+    want = softmax(x)
+    monkeypatch.setattr(_lib, "_current_device", None)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = softmax(x)
+    side.synchronize()
+    assert torch.equal(got, want)
