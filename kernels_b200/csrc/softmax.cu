@@ -119,22 +119,27 @@ __global__ void __launch_bounds__(THREADS, GROUP > 32 ? 1024 / THREADS : 2) soft
   }
   // exp(z - max) with one rounding: 2^(z log2e - max log2e).  The rounding of max log2e is a factor that the whole row
   // shares, and cancels as long as it stays near 1: up to |max| = 2^16 it lies within 2^(2^-8) of it, from 2^31 on it alone
-  // leaves fp32's range.  So a larger maximum (a row masked to the type's lowest value, an infinity) is subtracted first.
-  // In bf16 that takes no subtraction per element: all that is not the maximum lies 256 or more below it and counts as 0
-  // in any base, so base 2 does.  Finite fp16 values never come to that.  (bf16 [65536, 4096] 171 -> 172 us, fp32 [65536, 200]
-  // 15.8 -> 16.2; subtracting in every row instead: bf16 180 us.)
-  const bool far = !std::is_same<T, __half>::value && !(fabsf(mx) <= 65536.f);
-  const bool base2 = far && sizeof(T) == 2;
-  const float mul = base2 ? 1.f : kLog2e;
-  float shift = base2 ? mx : mx * kLog2e;
-  if (sizeof(T) == 4 && !RAGGED && far) {
+  // leaves fp32's range.  In the rare row with a larger maximum (masked to the type's lowest value, an infinity) the maximum
+  // is subtracted from every element first.  (A difference rounded to bf16 is 0 for the maximum itself and otherwise -256 or
+  // less, which counts as 0 in fp32.)  Finite fp16 values never come to that.
+  constexpr bool kFar = !std::is_same<T, __half>::value && !(RAGGED && sizeof(T) == 4);
+  if (kFar && __builtin_expect(!(fabsf(mx) <= 65536.f), 0)) {
 #pragma unroll
-    for (int i = 0; i < (kPacked ? 1 : NV); ++i)
+    for (int i = 0; i < NV; ++i) {
+      if constexpr (kPacked) {
+        __nv_bfloat162* w = reinterpret_cast<__nv_bfloat162*>(&raw[i]);
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[i][e] -= mx;
-    shift = 0.f;
+        for (int j = 0; j < E / 2; ++j) w[j] = __hsub2(w[j], __float2bfloat162_rn(mx));
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[i][e] -= mx;
+      }
+    }
+    ve -= mx;
+    mx = 0.f;
   }
-  auto exp_of = [&](float z) { return RAGGED && sizeof(T) == 4 ? expf(z - mx) : exp2f(fmaf(z, mul, -shift)); };
+  const float mx_l2 = mx * kLog2e;
+  auto exp_of = [&](float z) { return RAGGED && sizeof(T) == 4 ? expf(z - mx) : exp2f(fmaf(z, kLog2e, -mx_l2)); };
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
