@@ -616,3 +616,42 @@ def test_launch_without_the_private_calls(monkeypatch):
         got = softmax(x)
     side.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("D,layout", [(16, "dense"), (16, "odd"), (32, "dense"), (32, "strided"), (64, "odd"), (128, "strided"), (256, "dense"),
+                                      (256, "odd")])
+@pytest.mark.parametrize("T,c,back", [(1, 1, 0), (31, 7, 3), (65, 64, 1), (129, 200, 0), (200, 10, 5)])
+def test_16_bit_generic_tiles_edges_and_layouts(D, layout, T, c, back):
+    """The generic kernels' scalar loads in 16 bits, one row around the tiles (64, 32 for D = 256), against dense attention in
+    64 bits.  Rows past the last one count as zeros, whatever the last one holds: the padding is NaN there in q.  Bounds:
+    the fp16 ones of the grid."""
+    from kernels_b200.streaming_attention import streaming_attention
+
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+
+    def make():
+        if layout == "odd":
+            return torch.randn(2 * 3 * T * D + 1, generator=g, device="cuda").half()[1:].view(2, 3, T, D)
+        x = torch.randn(2, 3, T, 2 * D, generator=g, device="cuda").half()
+        return x[..., ::2] if layout == "strided" else x[..., :D].contiguous()
+
+    q, k, v, do = (make() for _ in range(4))
+    lens = torch.tensor([T, max(T - 1, 1)], dtype=torch.int32, device="cuda")
+    live = torch.arange(T, device="cuda")[None] < lens[:, None]
+    chunk = torch.arange(T, device="cuda") // c
+    diff = chunk[:, None] - chunk[None]
+    mask = ((diff >= 0) & (diff <= back))[None] & live[:, :, None] & live[:, None]
+    ref = [t.double().requires_grad_() for t in (q, k, v)]
+    scores = (ref[0] @ ref[1].mT * D**-0.5).masked_fill(~mask[:, None], -1e300)
+    want = (torch.softmax(scores, -1) @ ref[2]) * live[:, None, :, None]
+    want = [want.detach(), *torch.autograd.grad(want, ref, do.double() * live[:, None, :, None])]
+    if T > 1:
+        q[1, :, -1] = float("nan")  # a padding row
+    got_in = [t.requires_grad_() for t in (q, k, v)]
+    got = streaming_attention(*got_in, lens, c, back)
+    assert (got - want[0]).abs().max() <= 3e-3
+    # (dK of the padded batch entry would be 0 x NaN: its padding is zeroed again for the backward)
+    with torch.no_grad():
+        q.nan_to_num_(0.0)
+    for name, a, b in zip(("dq", "dk", "dv"), torch.autograd.grad(streaming_attention(*got_in, lens, c, back), got_in, do), want[1:]):
+        assert (a - b).abs().max() <= 1e-2, name
