@@ -1180,7 +1180,8 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.fd_c = kb_fastdiv_make(c);
   fa.scale_log2 = p.sm_scale * kLog2e;
   fa.sm_scale = p.sm_scale;
-  fa.item_rot = kb_item_rotation((int32_t)grid_main, n_tiles, p.lens || PACKED);
+  const int32_t most_places = c % (2 * kBK) ? 4 : mid && !PACKED ? 1 : 2;  // see kb_item_rotation
+  fa.item_rot = kb_item_rotation((int32_t)grid_main, n_tiles, p.lens || PACKED, most_places);
   fa.item_rot_dq = kb_item_rotation((int32_t)grid, n_tiles, p.lens || PACKED);
   fa.status = p.status;
   if (!(p.flags & KB_FLAG_BWD_SKIP_DKDV)) {

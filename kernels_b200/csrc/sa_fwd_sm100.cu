@@ -902,7 +902,7 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   const int64_t n_items = (int64_t)p.B * p.H * kb_cdiv_i32(Tq, kBM * kQTiles);
   if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
   const unsigned grid = (unsigned)(n_items < n_sm ? n_items : n_sm);  // persistent: one CTA per SM
-  a.item_rot = kb_item_rotation((int32_t)grid, kb_cdiv_i32(Tq, kBM * kQTiles), p.lens || p.cu_seqlens);
+  a.item_rot = fast ? 0 : kb_item_rotation((int32_t)grid, kb_cdiv_i32(Tq, kBM * kQTiles), p.lens || p.cu_seqlens);
   kern<<<grid, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
   KB_LAUNCH_CHECK("sa_fwd_sm100_kernel");
   return KB_OK;

@@ -93,11 +93,21 @@ KB_HD int32_t kb_fastdiv(int32_t n, const KbFastDiv& f) {
 // often padding, and with few places per CTA some CTAs get much more work than others (n = 4, G = 148: CTA 0 only the
 // first quarter of every sequence).  r > 0 makes G + r and n coprime, which spreads the places.
 //
-// Only where the lengths differ and a CTA would meet at most four places.  Measured (B200, r = 0 / r = 1): packed batch
-// of 256 sequences of 128-1024 rows, forward 951 / 843 us, main backward kernel 1286 / 1081, dQ 497 / 402; fp16 D=64
-// c=10 T=1353 (n = 6, three places) forward 261 / 235 us.  With eight and more places nothing is gained, and
+// Only where the lengths differ and a CTA would meet at most `most_places` places (1 to 4).  Measured (B200, r = 0 / r = 1):
+// packed batch of 256 sequences of 128-1024 rows, forward 951 / 843 us, main backward kernel 1286 / 1081, dQ 497 / 402;
+// fp16 D=64 c=10 T=1353 (n = 6, three places) forward 261 / 235 us.  With eight and more places nothing is gained, and
 // an odd r can cost: main kernel, bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r (with an even one
 // CTAs 2 m and 2 m + 1 always have the two key tiles of one chunk, which stream the same Q / dO tiles).
+//
+// The main backward kernel therefore shifts chunks that are whole pairs of key tiles (c a multiple of 256) only where a
+// CTA meets fewer places than four.  r = 0 / shifted, us, bf16 D=128, by the places met: padded, lengths T/2 to T: one (T=512)
+// 782 / 818, dQ 330 / 281; two (T=1024) 909 / 977, four (T=2048) 954 / 1035; c=512 T=768 (three) 928 / 1006.  Packed, T/8 to T:
+// one 1390 / 1145, two 1369 / 1340, four 1400 / 1470.  fp16 D=64 c=256, padded: one 334 / 289, two 409 / 385, four 451 /
+// 464.  Hence at most two, at most one for the padded head-dim-128 class.  (Other chunk lengths gain everywhere, but for
+// c=160 and 192 at T=512: 784 / 834, with dQ 361 / 297 and the forward 708 / 625.)
+//
+// The forward's straight-line instance takes no shift: bf16 D=128 c=256 ragged T=512 601 / 535 us, T=1024 679 / 616, but
+// T=2048 501 / 532; dense fp16 D=64 375 / 376.
 inline int32_t kb_gcd(int32_t a, int32_t b) {
   while (b) {
     const int32_t t = a % b;
@@ -106,9 +116,9 @@ inline int32_t kb_gcd(int32_t a, int32_t b) {
   }
   return a;
 }
-inline int32_t kb_item_rotation(int32_t ctas, int32_t items_per_seq, bool ragged) {
+inline int32_t kb_item_rotation(int32_t ctas, int32_t items_per_seq, bool ragged, int32_t most_places = 4) {
   const int32_t n = items_per_seq;
-  if (!ragged || ctas < 1 || n < 1 || n / kb_gcd(ctas, n) > 4) return 0;
+  if (!ragged || ctas < 1 || n < 1 || n / kb_gcd(ctas, n) > most_places) return 0;
   int32_t r = 0;
   while (kb_gcd(ctas + r, n) != 1) ++r;  // among n consecutive numbers one is coprime to n
   return r % ctas;
