@@ -320,20 +320,15 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           KB_FTR(0, g, 0);
           // order of issue = order of need: S wants K and Q, dP (issued a tile later) wants V and dO
           if (c.t == 0) {
-            // K and V are read by this CTA only and come from DRAM.  The long-item class asks for the tiles of the next
-            // tile's item in L2 (the one that opens here, unless it has a single tile): 1 617 us against 1 635 without
-            // (bf16 c=256 T=16384).  The other classes lose by it: fp16 D=64 c=10 379 us with, 359 without, c=128 258 /
-            // 246, packed 1 073 / 1 052.
+            // K and V are read by this CTA only and come from DRAM.  The long-item class asks for the opening item's tiles in
+            // L2 at once; V and the second half of K are loaded behind waits.  1 669 us against 1 720 without (bf16 c=256
+            // T=16384), packed c=256 1 793 / 1 800.  The other classes lose by it: fp16 D=64 c=10 379 us with, 359 without,
+            // c=128 258 / 246, packed c=64 1 073 / 1 052.
             if constexpr (MID) {
-              Cursor nx = c;
-              nx.t = nx.tiles() - 1;
-              cursor_next<PACKED>(a, nx, n_items, n_ktiles);
-              if (nx.valid) {
 #pragma unroll
-                for (int p = 0; p < kPanels; ++p) {
-                  tma_prefetch_l2_4d(&tm_k, p * 64, nx.it.row0 + nx.it.k0, nx.it.hk, PACKED ? 0 : nx.it.b);
-                  tma_prefetch_l2_4d(&tm_v, p * 64, nx.it.row0 + nx.it.k0, nx.it.hk, PACKED ? 0 : nx.it.b);
-                }
+              for (int p = 0; p < kPanels; ++p) {
+                tma_prefetch_l2_4d(&tm_k, p * 64, c.it.row0 + c.it.k0, c.it.hk, PACKED ? 0 : c.it.b);
+                tma_prefetch_l2_4d(&tm_v, p * 64, c.it.row0 + c.it.k0, c.it.hk, PACKED ? 0 : c.it.b);
               }
             }
             const int ks = n & 1;
