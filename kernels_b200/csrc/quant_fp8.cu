@@ -39,7 +39,7 @@ __device__ __forceinline__ uint32_t abs_bits_max(uint32_t m, T, uint32_t w) { re
 // x / scale rounded to nearest, with r = 1 / scale rounded to nearest: one Newton correction of x r by its exact
 // remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990: correctly
 // rounded where nothing underflows).  Here scale >= 1e-12 and quotients below 2^-11 become 0 whatever their last bit,
-// so the remainders that matter stay far above the smallest normal number; scale <= 2^120 keeps r normal.
+// so the remainders that matter stay far above the smallest normal number; scale <= 1e37 keeps r normal.
 __device__ __forceinline__ float div_by(float x, float scale, float r) {
   const float q = __fmul_rn(x, r);
   const float d = __fmaf_rn(__fmaf_rn(-q, scale, x), r, q);

@@ -22,7 +22,8 @@
 // lengths 1000-2000): forward 238 -> 145 us, dQ 336 -> 202 us, dK/dV 618 -> 260 us against 4 x 4 blocks of 256
 // threads with one product per instruction, scalar loads and a division per mask element; 31-35 TFLOP/s of the
 // blocks' arithmetic.  Tiles come in with cp.async where the rows
-// are fp32, 16-byte aligned and dense, the next one while the current block is still being worked on.
+// are fp32, 16-byte aligned and dense: in the forward and the dQ pass the next tile of an operand while the block still works
+// on the other; the dK/dV pass asks for Q and dO and waits for them (one buffer each).
 //
 // Backward: the dQ pass and the dK/dV pass each evaluate the scores and dP.  fp32 calls with a dS scratch evaluate them
 // once instead: delta, dK/dV (which saves its dS tiles), dQ = dS K (sa_bwd_dq_saved_generic_kernel).  Same case: 202 +

@@ -24,7 +24,8 @@ constexpr int kTwoPassStagesFirst = 3, kTwoPassStagesSecond = 2;
 constexpr int kMainKeys = 128, kMainQueries = 128, kMainStagesQ = 2, kMainStagesK = 2;
 constexpr int kDqQueries = 128, kDqKeys = 128, kDqStages = 3;
 
-// generic CUDA-core kernels: square tiles, no software pipeline
+// generic CUDA-core kernels: square tiles, one buffer per operand (the forward and the dQ pass refill it while the other
+// operand is in use; the dK/dV pass waits for its loads)
 constexpr int generic_tile(int D) { return D <= 128 ? 64 : 32; }
 constexpr int kGenericStages = 1;
 
