@@ -1,0 +1,153 @@
+// The work items of the persistent kernels, handed out while the kernel runs.
+//
+// The grid has one block per work item, one block fits an SM, and a running CTA takes over blocks that have not been
+// launched yet (clusterlaunchcontrol.try_cancel): it starts with the item of its own block index and asks for another
+// when it is about to run out.  So a CTA that meets padding or short items simply comes back sooner.  No counter in
+// global memory: nothing to clear before a launch, nothing that calls, streams or graph replays could share.
+//
+// One warp of the CTA, the TMA producer's, asks (ItemWriter).  It clears the outputs of items that lie wholly in the
+// padding itself and passes the live ones to the other roles through a ring of kItemSlots numbers in shared memory
+// (ItemReader).  (Padded items do not go through the ring: a role may look for the next live item before the current one
+// is complete, and would wait for ever behind a run of padded ones that fills the ring.)  It asks when it starts on the
+// last tile of an item: the answer takes less than the tile, and an item claimed earlier would wait at a CTA that is
+// still busy.
+#pragma once
+#include "sm100_ptx.cuh"
+
+namespace kb {
+namespace sm100 {
+
+constexpr int kItemSlots = 4;
+enum ItemWaitSite { kWaitItemAnswer = 121, kWaitItemEmpty, kWaitItemFull };
+
+struct alignas(16) ItemQueue {
+  uint32_t answer[4];
+  int4 entry[kItemSlots];  // item (-1: there are no more), and what its writer says about it
+  uint64_t answered, full[kItemSlots], empty[kItemSlots];
+};
+
+// `readers`: ItemReaders of the CTA.  Executed by one thread, before fence_mbar_init() and the CTA's first barrier.
+__device__ __forceinline__ void item_queue_init(ItemQueue& q, int readers) {
+  mbar_init(&q.answered, 1);
+  for (int i = 0; i < kItemSlots; ++i) {
+    mbar_init(&q.full[i], 1);
+    mbar_init(&q.empty[i], readers);
+  }
+}
+
+__device__ __forceinline__ void item_ask(ItemQueue* q) {
+  fence_proxy_async();  // the last answer was read through the generic proxy
+  mbar_expect_tx(&q->answered, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(q->answer)),
+               "r"(smem_u32(&q->answered))
+               : "memory");
+}
+// The block index in the answer, -1 if there was no block left to take over (after which none may be asked for).
+__device__ __forceinline__ int item_answer(const ItemQueue* q) {
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t.reg .b32 y, z, w;\n\t"
+      "ld.shared.b128 a, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, y, z, w}, a;\n\t}"
+      : "=r"(got), "=&r"(x)
+      : "r"(smem_u32(q->answer))
+      : "memory");
+  return got ? (int)x : -1;
+}
+// After a wait of the CTA gave up: the blocks not launched yet are taken over and dropped, so that the kernel ends with
+// the error code now and not after as many such waits as there are items left.  `answers`: answers taken so far.
+static __device__ __noinline__ void item_drop_rest(ItemQueue* q, int answers, bool asked) {
+  for (int item = 0; item >= 0; ++answers) {
+    if (!asked) item_ask(q);
+    asked = false;
+    for (uint32_t spins = 0; !mbar_try_wait(&q->answered, answers & 1);)
+      if (++spins >= kWaitLimitSpins) return;
+    item = item_answer(q);
+  }
+}
+
+// Used by a whole converged warp; item() is the same in all lanes, the rest is lane 0's.
+struct ItemWriter {
+  ItemQueue* q;
+  int answers, published, item_;  // answers taken, items passed on so far; the current item, -1 after the last one
+  bool asked, more, ok;          // a request is under way; no request has failed yet; no wait gave up
+  __device__ __forceinline__ explicit ItemWriter(ItemQueue& queue)
+      : q(&queue), answers(0), published(0), item_((int)blockIdx.x), asked(false), more(true), ok(true) {}
+  __device__ __forceinline__ int item() const { return item_; }
+  // Lane 0: ask for the next item ahead of next().
+  __device__ __forceinline__ void ask() {
+    if (!asked) item_ask(q);
+    asked = true;
+  }
+  // Lane 0: pass an item on to the readers.
+  __device__ __forceinline__ bool publish(int4 entry, const WaitCtx& ctx) {
+    const int n = published++, s = n % kItemSlots;
+    if (n >= kItemSlots && !mbar_wait(&q->empty[s], ((n / kItemSlots) - 1) & 1, ctx, kWaitItemEmpty)) return false;
+    q->entry[s] = entry;
+    mbar_arrive(&q->full[s]);
+    return true;
+  }
+  // The warp's next item; `go_on` (lane 0's counts): false ends the walk after an error.
+  __device__ __forceinline__ void next(bool go_on, const WaitCtx& ctx) {
+    int got = -1;
+    if ((threadIdx.x & 31) == 0) {
+      ok = go_on;
+      if (ok) {
+        ask();
+        ok = mbar_wait(&q->answered, answers & 1, ctx, kWaitItemAnswer);
+        if (ok) {
+          asked = false;
+          ++answers;
+          got = item_answer(q);
+          more = got >= 0;
+        }
+      }
+    }
+    item_ = __shfl_sync(0xffffffffu, got, 0);
+  }
+  // Lane 0, after the walk.
+  __device__ __forceinline__ void finish(const WaitCtx& ctx) {
+    if (ok) publish(make_int4(-1, 0, 0, 0), ctx);
+    if (more) item_drop_rest(q, answers, asked);
+  }
+};
+
+enum class Reader {
+  kThread,  // one thread
+  kWarp,    // a whole converged warp, all of whose lanes leave together if a wait gives up
+  kLead     // a warp of which only lane 0 has effects; the others follow it, each with waits of its own
+};
+template <Reader KIND>
+struct ItemReader {
+  ItemQueue* q;
+  int n;   // entries read so far
+  int4 e;  // the current one; its item is -1 after the last one (or after a wait that gave up)
+  __device__ __forceinline__ ItemReader(ItemQueue& queue, const WaitCtx& ctx) : q(&queue), n(0) { next(ctx); }
+  __device__ __forceinline__ int item() const { return e.x; }
+  __device__ __forceinline__ void next(const WaitCtx& ctx) {
+    const int s = n % kItemSlots;
+    bool ok = mbar_wait(&q->full[s], (n / kItemSlots) & 1, ctx, kWaitItemFull);
+    if (KIND == Reader::kWarp) ok = __all_sync(0xffffffffu, ok);
+    e = q->entry[s];
+    if (!ok) e.x = -1;
+    if (KIND == Reader::kWarp) __syncwarp();
+    if (KIND == Reader::kThread || (threadIdx.x & 31) == 0) mbar_arrive(&q->empty[s]);
+    ++n;
+  }
+};
+
+// Zeros into `rows` rows of BYTES bytes (at most 512), `stride` bytes apart, by a whole warp.
+template <int BYTES>
+__device__ __forceinline__ void warp_clear_rows(void* first, int64_t stride, int rows) {
+  constexpr int kLanes = BYTES / 16;
+  const int lane = threadIdx.x & 31;
+  uint8_t* p = static_cast<uint8_t*>(first) + (lane / kLanes) * stride + (lane % kLanes) * 16;
+#pragma unroll 4
+  for (int i = lane / kLanes; i < rows; i += 32 / kLanes, p += (32 / kLanes) * stride) *reinterpret_cast<uint4*>(p) = make_uint4(0, 0, 0, 0);
+}
+
+}  // namespace sm100
+}  // namespace kb

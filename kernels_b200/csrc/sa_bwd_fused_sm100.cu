@@ -158,7 +158,7 @@ struct Item {
 // The tiles of an item: for every query head of the key/value head's group (hq = 0 .. group - 1), the
 // query tiles of `qr` (tq = 0 ..); t is the running index over both.
 struct Cursor {
-  KbItemWalk<> walk;
+  KbItemWalk walk;
   int n, g, t, tq, hq, group;
   Item it;
   bool valid;
@@ -210,7 +210,7 @@ __device__ __forceinline__ void seek_live(const FusedArgs& a, Cursor& c, int n_i
 }
 template <bool PACKED>
 __device__ __forceinline__ Cursor cursor_first(const FusedArgs& a, int n_items, int n_ktiles) {
-  Cursor c{KbItemWalk<>(a.item_rot)};  // (everything after the walk starts as zero)
+  Cursor c{KbItemWalk(a.item_rot)};  // (everything after the walk starts as zero)
   c.group = a.group;
   seek_live<PACKED>(a, c, n_items, n_ktiles);
   return c;
@@ -451,7 +451,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       };
       // This thread keeps no cursor: all it needs of the schedule is how many tiles each live item has.
       // Tiles of the first live item from the walk's position on, 0 if there is none.
-      auto next_live = [&](KbItemWalk<>& walk) -> int {
+      auto next_live = [&](KbItemWalk& walk) -> int {
         for (; walk.item() < n_items; walk.next()) {
           const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles);
           if (it.qr.begin < it.qr.end) return (it.qr.end - it.qr.begin) * a.group;
@@ -459,7 +459,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         return 0;
       };
 
-      KbItemWalk<> walk(a.item_rot);
+      KbItemWalk walk(a.item_rot);
       int cnt = next_live(walk);  // tiles of the current item
       int n = 0, g = 0;           // live items, tiles so far
       bool ok = cnt > 0 && issue_s(0, 0, true) && issue_dp(0, 0, true, cnt == 1);
@@ -725,7 +725,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     int n = 0;
     bool ok = true;
-    for (KbItemWalk<> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
+    for (KbItemWalk walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
       const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles);
       const int kr = it.k0 + row;
       if (it.qr.begin >= it.qr.end) {
@@ -970,7 +970,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       prefetch_tensormap(&tm_k);
       int u = 0;
       bool ok = true;
-      for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
+      for (KbItemWalk walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
         const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
         for (int j = it.kr.begin; j < it.kr.end; ++j, ++u) {
           const int s = u % kDqStages;
@@ -990,7 +990,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       constexpr uint32_t idesc = make_idesc(BF16, kBQ, D, true, true);  // A = dS read MN-major (rows = keys), B = K MN-major
       int u = 0, m = 0;
       bool ok = true;
-      for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
+      for (KbItemWalk walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
         const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
         if (it.kr.begin >= it.kr.end) continue;
         const uint32_t acc = tmem + (m & 1) * 128;
@@ -1017,7 +1017,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
     int m = 0;
     bool ok = true;
-    for (KbItemWalk<> walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
+    for (KbItemWalk walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
       const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
       const int qi = it.qt * kBQ + row;
       if (it.kr.begin >= it.kr.end) {

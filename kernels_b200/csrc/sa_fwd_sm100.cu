@@ -5,12 +5,13 @@
 // q tiles use every K/V tile that is brought into shared memory, which halves the L2 traffic
 // per FLOP against one q tile per CTA.  Ten warps, three roles (K and V rings two deep; output rows leave through shared memory and TMA stores):
 //   warps 0-3 / 4-7  softmax of q tile A / B: thread r owns query row r of its tile (= TMEM lane
-//              r).  Walks its row of a 128 x 128 block of S in TMEM twice, 64 columns at a time (row
+//              r).  Walks its row of a 128 x 128 block of S in TMEM twice, 32 columns at a time (row
 //              maximum, then exponentials in packed fp32 arithmetic), keeps the running max / sum,
 //              writes P (16-bit) back over S, rescales O when the max moved by more than 2^8,
 //              writes O / LSE at the end;
-//   warp 8     TMA producer (one lane): Q once, then a ring of K tiles and a ring of V tiles;
-//   warp 9     MMA issuer (one lane): S = Q K^T (A, B from shared memory), O += P V
+//   warp 8     TMA producer (one lane): Q once, then a ring of K tiles and a ring of V tiles; takes the work
+//              items from the hardware's queue (item_queue.cuh) and clears the outputs of padded ones;
+//   warp 9     MMA issuer (a converged warp, one lane's instructions count): S = Q K^T (A, B from shared memory), O += P V
 //              (A = P from TMEM, B = V from shared memory, MN-major); owns the TMEM allocation.
 // MMA issue order per KV tile t:  PV_A(t-1)  S_A(t)  PV_B(t-1)  S_B(t).  While the softmax warps
 // of one q tile work on their S block the tensor pipe runs the other q tile's MMAs.  MMAs
@@ -19,9 +20,10 @@
 // TMEM columns: S_A at 0, S_B at 128 (fp32; P overlays the first 64 columns of each),
 // O_A at 256, O_B at 384.  One CTA per SM.
 //
-// The kernel is persistent: the grid is one CTA per SM and every CTA walks the work items
-// (batch, head, 256-row q block) in the order of KbItemWalk (schedule.h).  Barriers and
-// TMEM are set up once; the producer runs ahead into the next item (its Q is loaded as soon as
+// The kernel is persistent: one CTA fits an SM, and every CTA takes work items (batch, head, 256-row q block) until
+// there are none left (item_queue.cuh).  Handing them out statically left CTAs that met the long sequences of a ragged batch
+// behind: a simulation of the items' costs gives 1.06-1.30 times the mean for static orders, 1.01-1.05 for this one.
+// Barriers and TMEM are set up once; the producer runs ahead into the next item (its Q is loaded as soon as
 // the last S of the current item has been issued) and the softmax warps write the current
 // item's O while the MMAs of the next one already run, so the pipeline is not drained and
 // refilled per item.  Consecutive items are consecutive q blocks of one (batch, head): the CTAs
@@ -39,6 +41,7 @@
 #include "common.cuh"
 #include <type_traits>
 
+#include "item_queue.cuh"
 #include "sm100_ptx.cuh"
 #include "sm100_host.h"
 #include "tiles.h"
@@ -82,7 +85,6 @@ struct FwdArgs {
   // extent is 1, o_sb = lse_sb = 0) and T is the longest sequence.  NULL: the padded layout.
   const int32_t* cu;
   KbFastDiv fd_qblocks, fd_H, fd_c, fd_group;  // division by ceil(T / 256), H, c and H / H_kv (query heads per K/V head)
-  int32_t item_rot;  // see KbItemWalk
   float scale_log2;
   int32_t* status;
   // 8-bit (e4m3) inputs only: one dequantisation scale per tile of 128 rows of q [B, H, n128], k and v
@@ -102,6 +104,7 @@ struct alignas(1024) FwdSmem {
   uint8_t o_stage[kQTiles][kBM * 128];  // one 64-column panel of a q tile's output on its way to a TMA store
   uint64_t q_full[kQTiles], k_full[kStagesK], k_empty[kStagesK], v_full[kStagesV], v_empty[kStagesV];
   uint64_t q_empty[kQTiles], s_ready[kQTiles], p_ready[kQTiles], o_done[kQTiles], o_free[kQTiles];
+  ItemQueue items;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -109,105 +112,79 @@ struct alignas(1024) FwdSmem {
 enum WaitSite { kWaitQ = 1, kWaitQEmpty, kWaitOFree, kWaitKEmpty, kWaitVEmpty, kWaitKFull, kWaitVFull, kWaitSReady, kWaitPReady, kWaitEpilogue };
 constexpr int kErrSmemAlign = 11;
 
-// Which of the 32 columns from c0 on lie in the row's live interval [lo, hi).  WORD: as the bits of one word (half the
-// instructions per element); otherwise two compares per element.  Words everywhere but in the straight-line instance
-// for head dim 128, whose items are masked at sequence ends only and whose code the words make slower (bf16 c=256
-// T=16384 without lengths: 888 us with compares, 919 with words; 8-bit: 215 / 241; while
-// c=64 T=8192: 895 / 811 us, fp16 D=64 c=10: 340 / 270, dense D=64 with lengths: 434 / 399).
-template <bool WORD>
-struct LiveCols {
-  uint32_t word;
-  int c0, lo, hi;
-  __device__ __forceinline__ LiveCols(int c0_, int lo_, int hi_) : word(WORD ? live_word(c0_, lo_, hi_) : 0u), c0(c0_), lo(lo_), hi(hi_) {}
-  __device__ __forceinline__ bool all() const { return WORD ? word == ~0u : (lo <= c0 && c0 + 32 <= hi); }
-  __device__ __forceinline__ bool none() const { return WORD ? word == 0u : (c0 + 32 <= lo || c0 >= hi); }
-  __device__ __forceinline__ bool operator[](int i) const { return WORD ? (word & (1u << i)) != 0 : (c0 + i >= lo && c0 + i < hi); }
-};
+// The softmax warps walk their row of a 128 x 128 block twice, 32 columns at a time, the next 32 on their way out of TMEM
+// meanwhile.  The loops stay loops and there is one copy of the arithmetic with masks and one without: the code of a
+// block is what the MMA-issuing warp competes with for the instruction cache.  Both passes unrolled over the
+// row / as loops: bf16 D=128 c=64 806 / 682 us; the masked copy 64 columns wide / 32: packed c=64 649 / 569; one pass with all
+// 128 scores held against this at D=64: fp16 c=10 260 / 229.
 
-// One 128 x 128 block of scores for the thread's row, in two passes over the row in TMEM, 64 columns at a
-// time, so that at most 64 scores are live in registers (holding all 128 leaves the softmax warps no register to
-// spare at the 168 the launch gives them, and every spill sits on the kernel's critical chain).
-// Pass 1 (softmax_row_max): the row maximum of the masked scores.  kMasked = false is the fast path for blocks
-// in which every element of the warp's rows is live.
-template <bool kMasked, bool WORD>
-__device__ __forceinline__ float softmax_row_max(uint32_t t_s, int k0, int lo, int hi) {
+// The columns' scores have arrived (the compiler may not move their use above the wait).
+__device__ __forceinline__ void scores_arrived(uint32_t (&s)[32]) {
+  tmem_wait_ld();
+  asm volatile("" : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]), "+r"(s[7]), "+r"(s[8]),
+               "+r"(s[9]), "+r"(s[10]), "+r"(s[11]), "+r"(s[12]), "+r"(s[13]), "+r"(s[14]), "+r"(s[15]));
+  asm volatile("" : "+r"(s[16]), "+r"(s[17]), "+r"(s[18]), "+r"(s[19]), "+r"(s[20]), "+r"(s[21]), "+r"(s[22]), "+r"(s[23]), "+r"(s[24]),
+               "+r"(s[25]), "+r"(s[26]), "+r"(s[27]), "+r"(s[28]), "+r"(s[29]), "+r"(s[30]), "+r"(s[31]));
+}
+// -inf into the scores of the 32 columns from c on that are outside the row's live interval [lo, hi).  False, with the
+// scores as they were, if all of them are for every row of the warp.
+__device__ __forceinline__ bool mask_scores(uint32_t (&s)[32], int c, int lo, int hi) {
+  const uint32_t live = live_word(c, lo, hi);
+  if (__all_sync(0xffffffffu, live == 0u)) return false;
+  if (!__all_sync(0xffffffffu, live == ~0u)) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) s[i] = (live & (1u << i)) ? s[i] : 0xff800000u;
+  }
+  return true;
+}
+template <bool MASKED>
+__device__ __forceinline__ void max_scores(uint32_t (&s)[32], int c, int lo, int hi, float (&mx)[4]) {
+  if (MASKED && !mask_scores(s, c, lo, hi)) return;
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)  // 3-input max: two scores per instruction
+      mx[e] = fmax3(mx[e], __uint_as_float(s[i + 2 * e]), __uint_as_float(s[i + 2 * e + 1]));
+  }
+}
+// Pass 1: the row maximum of the masked scores.  Leaves the first 32 columns in `s` for pass 2.
+template <bool MASKED>
+__device__ __forceinline__ float softmax_row_max(uint32_t t_s, uint32_t (&s)[32], int k0, int lo, int hi) {
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    uint32_t s[64];
-    tmem_ld32(t_s + half * 64, reinterpret_cast<uint32_t(&)[32]>(s[0]));
-    tmem_ld32(t_s + half * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(s[32]));
-    tmem_wait_ld();
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      const int c0 = k0 + half * 64 + cc * 32;
-      // a 32-column group that is live for every row of the warp needs no select, one that is masked for every
-      // row contributes nothing (chunk boundaries that are multiples of 32 never leave a mixed group)
-      const LiveCols<WORD> live(c0, lo, hi);
-      const bool all_live = !kMasked || __all_sync(0xffffffffu, live.all());
-      const bool all_dead = kMasked && __all_sync(0xffffffffu, live.none());
-      if (all_dead) continue;
-      // 3-input max: two scores per instruction
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = cc * 32 + i + 2 * e;
-          float a = __uint_as_float(s[j]), b = __uint_as_float(s[j + 1]);
-          if (!all_live) {
-            a = live[i + 2 * e] ? a : -INFINITY;
-            b = live[i + 2 * e + 1] ? b : -INFINITY;
-          }
-          mx[e] = fmax3(mx[e], a, b);
-        }
-      }
-    }
+  tmem_ld32(t_s, s);
+  scores_arrived(s);
+#pragma unroll 1
+  for (int c = 0; c < kBN; c += 64) {
+    uint32_t u[32];
+    tmem_ld32(t_s + c + 32, u);
+    max_scores<MASKED>(s, k0 + c, lo, hi, mx);
+    scores_arrived(u);
+    tmem_ld32(t_s + ((c + 64) & (kBN - 1)), s);
+    max_scores<MASKED>(u, k0 + c + 32, lo, hi, mx);
+    scores_arrived(s);
   }
   return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
 }
-
-// Pass 2 (softmax_exp_half): P = 2^(S scale - m) for the 64 columns [64 half, 64 half + 64) of the row, 16-bit,
-// into TMEM over S (P of columns 32 j .. 32 j + 31 lands on columns 16 j .. 16 j + 15: the second half of P
-// overwrites only scores of the first half, which are in registers by then); the row sum goes into `sum`.
-// FP8: P is written as e4m3, four values per TMEM column (64 keys = 16 columns at 16 half), for the 8-bit P V.
-template <bool BF16, bool kMasked, bool FP8, bool WORD>
-__device__ __forceinline__ void softmax_exp_half(uint32_t t_s, int half, float scale, float m_used, int k0, int lo, int hi,
-                                                 float (&sum)[4]) {
-  const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
-  // packed fp32 arithmetic: one FMA and one add per PAIR of scores
-  const uint64_t scale2 = f2_pack(scale, scale), negm2 = f2_pack(-m_safe, -m_safe);
-  uint64_t sum01 = f2_pack(sum[0], sum[1]), sum23 = f2_pack(sum[2], sum[3]);
-  uint32_t s[64];
-  tmem_ld32(t_s + half * 64, reinterpret_cast<uint32_t(&)[32]>(s[0]));
-  tmem_ld32(t_s + half * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(s[32]));
-  tmem_wait_ld();
+// P = 2^(S scale - m) of 32 scores, 16-bit (FP8: e4m3, four to a column), into TMEM.
+struct SoftSum {
+  uint64_t s01, s23;
+};
+template <bool BF16, bool MASKED, bool FP8>
+__device__ __forceinline__ void exp_scores(uint32_t t_p, uint32_t (&s)[32], uint64_t scale2, uint64_t negm2, int c, int lo, int hi, SoftSum& sum) {
+  uint32_t pk[16];
+  float pf[FP8 ? 32 : 1];
+  if (MASKED && !mask_scores(s, c, lo, hi)) {
 #pragma unroll
-  for (int cc = 0; cc < 2; ++cc) {
-    const int c0 = k0 + half * 64 + cc * 32;
-    const LiveCols<WORD> live(c0, lo, hi);
-    const bool all_live = !kMasked || __all_sync(0xffffffffu, live.all());
-    const bool all_dead = kMasked && __all_sync(0xffffffffu, live.none());
-    uint32_t pk[16];
-    if (all_dead) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) pk[i] = 0u;
-      if (FP8) tmem_st8(t_s + (half * 2 + cc) * 8, reinterpret_cast<const uint32_t(&)[8]>(pk[0]));
-      else tmem_st16(t_s + (half * 2 + cc) * 16, pk);
-      continue;
-    }
-    float pf[FP8 ? 32 : 1];
+    for (int i = 0; i < 16; ++i) pk[i] = 0u;
+  } else {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      float s0 = __uint_as_float(s[cc * 32 + 2 * i]), s1 = __uint_as_float(s[cc * 32 + 2 * i + 1]);
-      if (!all_live) {
-        s0 = live[2 * i] ? s0 : -INFINITY;
-        s1 = live[2 * i + 1] ? s1 : -INFINITY;
-      }
-      const uint64_t x = f2_fma(f2_pack(s0, s1), scale2, negm2);
+      // packed fp32 arithmetic: one FMA and one add per PAIR of scores
+      const uint64_t x = f2_fma(f2_pack(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), scale2, negm2);
       float x0, x1;
       f2_unpack(x, x0, x1);
       const float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-      if (i & 1) sum23 = f2_add(sum23, f2_pack(p0, p1)); else sum01 = f2_add(sum01, f2_pack(p0, p1));
+      if (i & 1) sum.s23 = f2_add(sum.s23, f2_pack(p0, p1)); else sum.s01 = f2_add(sum.s01, f2_pack(p0, p1));
       if (FP8) {
         pf[2 * i] = p0;
         pf[2 * i + 1] = p1;
@@ -218,77 +195,34 @@ __device__ __forceinline__ void softmax_exp_half(uint32_t t_s, int half, float s
     if (FP8) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) pk[i] = pack_e4m3x4(pf[4 * i], pf[4 * i + 1], pf[4 * i + 2], pf[4 * i + 3]);
-      tmem_st8(t_s + (half * 2 + cc) * 8, reinterpret_cast<const uint32_t(&)[8]>(pk[0]));
-    } else {
-      tmem_st16(t_s + (half * 2 + cc) * 16, pk);
     }
   }
-  f2_unpack(sum01, sum[0], sum[1]);
-  f2_unpack(sum23, sum[2], sum[3]);
+  if (FP8) tmem_st8(t_p, reinterpret_cast<const uint32_t(&)[8]>(pk[0]));
+  else tmem_st16(t_p, pk);
+}
+// Pass 2: P into TMEM over S (P of columns 32 j .. 32 j + 31 lands on columns 16 j .. 16 j + 15, whose scores are in
+// registers by then); the row sum goes into `sum`.
+template <bool BF16, bool MASKED, bool FP8>
+__device__ __forceinline__ void softmax_exp(uint32_t t_s, uint32_t (&s)[32], uint64_t scale2, uint64_t negm2, int k0, int lo, int hi, SoftSum& sum) {
+  constexpr int kPack = FP8 ? 4 : 2;
+#pragma unroll 1
+  for (int c = 0; c < kBN; c += 64) {
+    uint32_t u[32];
+    tmem_ld32(t_s + c + 32, u);
+    exp_scores<BF16, MASKED, FP8>(t_s + c / kPack, s, scale2, negm2, k0 + c, lo, hi, sum);
+    scores_arrived(u);
+    if (c + 64 < kBN) tmem_ld32(t_s + c + 64, s);
+    exp_scores<BF16, MASKED, FP8>(t_s + (c + 32) / kPack, u, scale2, negm2, k0 + c + 32, lo, hi, sum);
+    scores_arrived(s);
+  }
 }
 
 // PACKED: one launch over a packed batch (FwdArgs::cu).  FP8: q, k, v are e4m3 with per-tile scales, both matmuls
 // run as kind::f8f6f4 (half the instructions), the output is 16-bit (BF16 selects which).
-// The same block in ONE pass for head dim 64, where the registers allow it (the epilogue holds 64 output columns,
-// not 128) and where it matters: with half the matmul work per block the softmax warps set the pace, and the
-// second walk over TMEM is time on their chain.  Loads the row's 128 scores once; returns the row maximum.
-template <bool kMasked>
-__device__ __forceinline__ float softmax_load_row_max(uint32_t t_s, uint32_t (&s)[kBN], bool (&dead)[kBN / 32], int k0, int lo, int hi) {
-#pragma unroll
-  for (int cc = 0; cc < kBN / 32; ++cc) tmem_ld32(t_s + cc * 32, reinterpret_cast<uint32_t(&)[32]>(s[cc * 32]));
-  tmem_wait_ld();
-  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-  for (int cc = 0; cc < kBN / 32; ++cc) {
-    const int c0 = k0 + cc * 32;
-    const LiveCols<true> live(c0, lo, hi);
-    const bool all_live = !kMasked || __all_sync(0xffffffffu, live.all());
-    dead[cc] = kMasked && __all_sync(0xffffffffu, live.none());
-    if (dead[cc]) continue;
-    if (!all_live) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) s[cc * 32 + i] = live[i] ? s[cc * 32 + i] : 0xff800000u;  // -inf
-    }
-#pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        mx[e] = fmax3(mx[e], __uint_as_float(s[cc * 32 + i + 2 * e]), __uint_as_float(s[cc * 32 + i + 2 * e + 1]));
-    }
-  }
-  return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-}
-// ... and P = 2^(S scale - m) from the registers, 16-bit, into TMEM over S; the row sum goes into `sum`.
-template <bool BF16, bool kMasked>
-__device__ __forceinline__ void softmax_exp_held(uint32_t t_s, const uint32_t (&s)[kBN], const bool (&dead)[kBN / 32], float scale,
-                                                 float m_used, float (&sum)[4]) {
-  const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
-#pragma unroll
-  for (int cc = 0; cc < kBN / 32; ++cc) {
-    uint32_t pk[16];
-    if (kMasked && dead[cc]) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) pk[i] = 0u;
-      tmem_st16(t_s + cc * 16, pk);
-      continue;
-    }
-    // scalar arithmetic here: with 128 scores held, the register pairs of the packed form do not fit
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float p0 = ex2_approx(fmaf(__uint_as_float(s[cc * 32 + 2 * i]), scale, -m_safe));
-      const float p1 = ex2_approx(fmaf(__uint_as_float(s[cc * 32 + 2 * i + 1]), scale, -m_safe));
-      sum[(2 * i) & 3] += p0;
-      sum[(2 * i + 1) & 3] += p1;
-      pk[i] = pack16x2<BF16>(p0, p1);
-    }
-    tmem_st16(t_s + cc * 16, pk);
-  }
-}
-
 // FAST: the instance for chunk lengths that are multiples of the work item's 256 rows, where the two q tiles of
 // every item lie in one chunk and walk the same key tiles: the MMA thread then runs such items through a
 // straight-line schedule (first / inner / last step written out, nothing worked out per step).  Other chunk
-// lengths are built without it (the extra code measured 1.5 % slower there).
+// lengths are built without it (the extra code measured 1.5 % slower there; c a multiple of 256 without it 865 -> 906 us, dense D=64 368 -> 392).
 template <int D, bool BF16, bool PACKED, bool FP8, bool FAST>
 __global__ void __launch_bounds__(kThreads, 1)
 sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -299,7 +233,6 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = a.T;
   const int n_qblocks = kb_cdiv_i32(T - a.q_start, kBM * kQTiles);
-  const int n_items = a.B * a.H * n_qblocks;
 
   if (smem_u32(smem_raw) & 1023u) {
     // swizzled operand tiles need a 1024-byte aligned base: report instead of computing garbage
@@ -359,6 +292,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_init(&sm.o_done[x], 1);
       mbar_init(&sm.o_free[x], kBM);
     }
+    item_queue_init(sm.items, 1 + kQTiles * 4);
     sm.abort_flag = 0;
     fence_mbar_init();
   }
@@ -382,47 +316,63 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       prefetch_tensormap(&tm_q);
       prefetch_tensormap(&tm_k);
       prefetch_tensormap(&tm_v);
-      int kc = 0, vc = 0;
-      int items_x[kQTiles] = {0, 0};  // items in which q tile x was live so far
-      bool ok = true;
-      for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
-        const Item it = decode(walk.item());
-        if (!it.act[0] && !it.act[1]) continue;
-        // a Q buffer is free once the last S of its q tile in the previous item has run
-        auto load_q = [&](int x) -> bool {
-          if (!it.act[x]) return true;
-          if (items_x[x] > 0 && !mbar_wait(&sm.q_empty[x], (items_x[x] - 1) & 1, ctx, kWaitQEmpty)) return false;
-          ++items_x[x];
-          mbar_expect_tx(&sm.q_full[x], kTileBytes);
-#pragma unroll
-          for (int p = 0; p < kPanels; ++p)
-            tma_load_4d(sm.q[x] + p * kPanelBytes, &tm_q, &sm.q_full[x], p * kPanelElems, it.row0 + it.q0 - a.q_start + x * kBM, it.h, PACKED ? 0 : it.b);
-          return true;
-        };
-        if (!load_q(0)) break;
-        const int h_kv = kb_fastdiv(it.h, a.fd_group);  // the K/V head this query head reads
-        for (int t = it.u_begin; t < it.u_end; ++t, ++kc, ++vc) {
-          const int sk = kc % kStagesK, sv = vc % kStagesV;
-          const int k0 = t * kBN;
-          if (kc >= kStagesK && !mbar_wait(&sm.k_empty[sk], ((kc / kStagesK) - 1) & 1, ctx, kWaitKEmpty)) { ok = false; break; }
-          mbar_expect_tx(&sm.k_full[sk], kTileBytes);
-#pragma unroll
-          for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.k[sk] + p * kPanelBytes, &tm_k, &sm.k_full[sk], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
-          // (order of need: Q of tile A and the first K, then Q of tile B)
-          if (t == it.u_begin && !load_q(1)) { ok = false; break; }
-          if (vc >= kStagesV && !mbar_wait(&sm.v_empty[sv], ((vc / kStagesV) - 1) & 1, ctx, kWaitVEmpty)) { ok = false; break; }
-          mbar_expect_tx(&sm.v_full[sv], kTileBytes);
-#pragma unroll
-          for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.v[sv] + p * kPanelBytes, &tm_v, &sm.v_full[sv], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
+    }
+    int kc = 0, vc = 0;
+    int items_x[kQTiles] = {0, 0};  // items in which q tile x was live so far
+    bool ok = true;
+    ItemWriter items(sm.items);
+    for (; items.item() >= 0; items.next(ok, ctx)) {
+      const Item it = decode(items.item());
+      if (!it.act[0]) {  // (tile B is never live without tile A)
+        // the q block lies wholly in the padding: its rows are zeros (a packed batch has no padding rows)
+        if (!PACKED) {
+          const int rows = kb_min_i32(kQTiles * kBM, T - it.q0), r0 = it.q0 - a.q_start;
+          warp_clear_rows<D * 2>(static_cast<uint16_t*>(a.o) + it.b * a.o_sb + it.h * a.o_sh + r0 * a.o_st, a.o_st * 2, rows);
+          if (a.lse)
+            for (int i = lane; i < rows; i += 32) a.lse[it.b * a.lse_sb + it.h * a.lse_sh + r0 + i] = 0.f;
         }
+        continue;
+      }
+      if (lane != 0) continue;
+      const int n_b = it.kr[1].end - it.kr[1].begin;
+      ok = items.publish(make_int4(items.item(), it.kr[0].end - it.kr[0].begin, n_b, n_b > 0 ? it.kr[1].begin - it.kr[0].begin : 0), ctx);
+      // a Q buffer is free once the last S of its q tile in the previous item has run
+      auto load_q = [&](int x) -> bool {
+        if (!it.act[x]) return true;
+        if (items_x[x] > 0 && !mbar_wait(&sm.q_empty[x], (items_x[x] - 1) & 1, ctx, kWaitQEmpty)) return false;
+        ++items_x[x];
+        mbar_expect_tx(&sm.q_full[x], kTileBytes);
+#pragma unroll
+        for (int p = 0; p < kPanels; ++p)
+          tma_load_4d(sm.q[x] + p * kPanelBytes, &tm_q, &sm.q_full[x], p * kPanelElems, it.row0 + it.q0 - a.q_start + x * kBM, it.h, PACKED ? 0 : it.b);
+        return true;
+      };
+      ok = ok && load_q(0);
+      const int h_kv = kb_fastdiv(it.h, a.fd_group);  // the K/V head this query head reads
+      for (int t = it.u_begin; ok && t < it.u_end; ++t, ++kc, ++vc) {
+        const int sk = kc % kStagesK, sv = vc % kStagesV;
+        const int k0 = t * kBN;
+        if (t == kb_max_i32(it.u_begin, it.u_end - 2)) items.ask();
+        if (kc >= kStagesK && !mbar_wait(&sm.k_empty[sk], ((kc / kStagesK) - 1) & 1, ctx, kWaitKEmpty)) { ok = false; break; }
+        mbar_expect_tx(&sm.k_full[sk], kTileBytes);
+#pragma unroll
+        for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.k[sk] + p * kPanelBytes, &tm_k, &sm.k_full[sk], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
+        // (order of need: Q of tile A and the first K, then Q of tile B)
+        if (t == it.u_begin && !load_q(1)) { ok = false; break; }
+        if (vc >= kStagesV && !mbar_wait(&sm.v_empty[sv], ((vc / kStagesV) - 1) & 1, ctx, kWaitVEmpty)) { ok = false; break; }
+        mbar_expect_tx(&sm.v_full[sv], kTileBytes);
+#pragma unroll
+        for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.v[sv] + p * kPanelBytes, &tm_v, &sm.v_full[sv], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
       }
     }
+    if (lane == 0) items.finish(ctx);
   } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    {
+      const bool lead = lane == 0;
       constexpr uint32_t idesc_qk = FP8 ? make_idesc_e4m3(kBM, kBN, false, false) : make_idesc(BF16, kBM, kBN, false, false);
       constexpr uint32_t idesc_pv = FP8 ? make_idesc_e4m3(kBM, D, false, true) : make_idesc(BF16, kBM, D, false, true);
-      int kbase = 0;                    // K (= V) tiles of earlier items
+      uint32_t kbase = 0;                    // K (= V) tiles of earlier items
       int tiles_x[kQTiles] = {0, 0};    // S / P blocks of q tile x so far
       int items_x[kQTiles] = {0, 0};    // items in which q tile x was live so far
       bool ok = true;
@@ -433,21 +383,20 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // FAST: the first S of tile A of an item is issued ahead, between the last P V of tile A and that of tile B of the
       // item before it, where its Q and K have landed by then (`ahead`): tile A's softmax warps go from one item to the
       // next without waiting for tile B's last block.  (Q has a barrier pair per q tile for this: a Q buffer is free
-      // after ITS tile's last S.)  bf16 D=128 c=256 T=16384: 865 -> 830 us, T=2048: 116 -> 109, 8-bit 217 -> 211, dense
-      // D=64 397 -> 378.  In the general schedule the same step measured 235 -> 270 us (fp16 D=64 c=10) and 846 -> 923
-      // (packed, c=64); the barrier pairs alone 240 -> 234 and 803 -> 779 (bf16 c=64 T=8192).
-      KbItemWalk<!FAST> walk(a.item_rot);
-      Item next;
-      auto seek = [&]() -> bool {  // the first live item from the walk's position on
-        for (; walk.item() < n_items; walk.next()) {
-          next = decode(walk.item());
-          if (next.act[0]) return true;  // (tile B is never live without tile A)
-        }
-        return false;
+      // after ITS tile's last S.)  bf16 D=128 c=256 T=16384: 865 -> 830 us, T=2048: 116 -> 109, 8-bit 217 -> 211.
+      ItemReader<Reader::kLead> items(sm.items, ctx);
+      // Of an item this thread needs how many key tiles each q tile walks (tile A at least one; tile B none if it lies in the
+      // padding), and how many key tiles after tile A's tile B's begin.
+      struct Walk {
+        int n0, n1, d;
+      } next;
+      auto seek = [&]() -> bool {
+        next.n0 = items.e.y, next.n1 = items.e.z, next.d = items.e.w;
+        return items.item() >= 0;
       };
       bool more = seek(), ahead = false;
       while (ok && more) {
-        const Item it = next;
+        const Walk it = next;
         KB_FACC(0);
         // Step s issues, per q tile x:  PV_x(s - 1) then S_x(s), each q tile walking its own key tiles in order.
         // When tile B's range starts d key tiles after tile A's (chunks shorter than the 256-row item: the two q
@@ -455,31 +404,30 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // 0 on their own first tile ("skewed": B works d key tiles ahead of A), so that every step carries both
         // q tiles and each one's softmax overlaps the other's MMAs; otherwise B starts at step d on the tile A is
         // on.  Either way a q tile sees its key tiles in the same order, so the results are the same bits.
-        const int n_x[kQTiles] = {it.act[0] ? it.kr[0].end - it.kr[0].begin : 0, it.act[1] ? it.kr[1].end - it.kr[1].begin : 0};
-        const int d = (it.act[0] && it.act[1]) ? it.kr[1].begin - it.kr[0].begin : 0;
-        const int first_x[kQTiles] = {0, d < kStagesK && d < kStagesV ? 0 : d};
-        const int n_steps = kb_max_i32(first_x[0] + n_x[0], first_x[1] + n_x[1]);
-        // the step at which q tile x visits key tile t (only meaningful for t inside its range)
-        auto step_of = [&](int x, int t) { return first_x[x] + t - it.kr[x].begin; };
+        // Key tiles are counted from tile A's first.
+        const int n_x[kQTiles] = {it.n0, it.n1}, begin_x[kQTiles] = {0, it.d};
+        const int first_x[kQTiles] = {0, it.d < kStagesK && it.d < kStagesV ? 0 : it.d};
+        const int n_steps = kb_max_i32(it.n0, first_x[1] + it.n1);
+        const int n_tiles = kb_max_i32(it.n0, it.d + it.n1);
         // q tile x is the last of the item to use key tile t (in a matmul of the kind issued at its step)
         auto last_user = [&](int x, int t) {
-          const int y = 1 - x;
-          if (!(it.act[y] && t >= it.kr[y].begin && t < it.kr[y].end)) return true;
-          const int sx = step_of(x, t), sy = step_of(y, t);
+          const int y = 1 - x, i = t - begin_x[y];
+          if (i < 0 || i >= n_x[y]) return true;
+          const int sx = first_x[x] + t - begin_x[x], sy = first_x[y] + i;
           return sx > sy || (sx == sy && x > y);
         };
         // O_x (+)= P_x V of the q tile's lx-th key tile, V being ring tile vi (counted over the CTA's life)
-        auto issue_pv = [&](auto first_c, auto last_c, int x, int vi, bool release_v) -> bool {
+        auto issue_pv = [&](auto first_c, auto last_c, int x, uint32_t vi, bool release_v) -> bool {
           constexpr bool kFirst = decltype(first_c)::value, kLast = decltype(last_c)::value;  // of the q tile's key tiles
-          const int sv = vi % kStagesV;
+          const uint32_t sv = vi % kStagesV;
           const int px = tiles_x[x] - 1;  // P block consumed now = last S block issued for x
           KB_FACC(2);
-          if (!mbar_wait(&sm.p_ready[x], px & 1, ctx, kWaitPReady)) return false;
+          if (!mbar_wait_short(&sm.p_ready[x], px & 1, ctx, kWaitPReady)) return false;
           KB_FACC(3 + x);
-          if (!mbar_wait(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull)) return false;
+          if (!release_v && (kFirst || kLast) && !mbar_wait_short(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull)) return false;
           KB_FACC(5);
           // the first P V of an item overwrites O: the softmax warps must have read the old one
-          if (kFirst && items_x[x] > 0 && !mbar_wait(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree)) return false;
+          if (kFirst && items_x[x] > 0 && !mbar_wait_short(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree)) return false;
           tc_fence_after();
           // short issue loops (four instructions per trip, descriptor low words stepped by adds): the
           // scalar work between two MMAs is what the tensor pipe waits for
@@ -488,27 +436,27 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             // 128 keys = four instructions of 32 keys: 8 packed columns of P, 32 rows (4096 bytes) of V each
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              mma_ts_lo_f8(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, !kFirst || i > 0);
+              mma_ts_lo_f8_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, !kFirst || i > 0);
           } else {
 #pragma unroll 1
             for (int h = 0; h < kBN / 64; ++h, p_col += 32, v_lo += 4 * (2048 >> 4)) {
 #pragma unroll
               for (int i = 0; i < 4; ++i)
-                mma_ts_lo(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, !kFirst || h > 0 || i > 0);
+                mma_ts_lo_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, !kFirst || h > 0 || i > 0);
             }
           }
-          if (release_v) mma_commit(&sm.v_empty[sv]);  // V is free once the last q tile that uses it has consumed it
-          if (kLast) mma_commit(&sm.o_done[x]);
+          if (release_v) mma_commit_if(lead, &sm.v_empty[sv]);  // V is free once the last q tile that uses it has consumed it
+          if (kLast) mma_commit_if(lead, &sm.o_done[x]);
           KB_FACC(6);
           return true;
         };
         // S_x = Q_x K^T, K being ring tile ki; `first` / `last` of the q tile's key tiles
-        auto issue_s = [&](int x, int ki, bool release_k, bool first, bool last) -> bool {
-          const int sk = ki % kStagesK;
+        auto issue_s = [&](int x, uint32_t ki, bool release_k, bool first, bool last, bool waited = false) -> bool {
+          const uint32_t sk = ki % kStagesK;
           KB_FACC(2);
-          if (first && !mbar_wait(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) return false;
+          if (first && !mbar_wait_short(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) return false;
           KB_FACC(1);
-          if (!mbar_wait(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) return false;
+          if (x == 0 && !waited && !mbar_wait_short(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) return false;
           KB_FACC(7);
           tc_fence_after();
           uint32_t q_lo = desc_lo_kmajor(smem_u32(sm.q[x])), k_lo = desc_lo_kmajor(smem_u32(sm.k[sk]));
@@ -516,13 +464,13 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           for (int h = 0; h < kPanels; ++h, q_lo += kPanelBytes >> 4, k_lo += kPanelBytes >> 4) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {  // 32 bytes of every row per instruction: 16 16-bit or 32 8-bit elements
-              if (FP8) mma_ss_lo_f8(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
-              else mma_ss_lo(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+              if (FP8) mma_ss_lo_f8_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+              else mma_ss_lo_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
             }
           }
-          if (release_k) mma_commit(&sm.k_empty[sk]);
-          if (last) mma_commit(&sm.q_empty[x]);
-          mma_commit(&sm.s_ready[x]);
+          if (release_k) mma_commit_if(lead, &sm.k_empty[sk]);
+          if (last) mma_commit_if(lead, &sm.q_empty[x]);
+          mma_commit_if(lead, &sm.s_ready[x]);
           ++tiles_x[x];
           KB_FACC(8);
           return true;
@@ -530,26 +478,26 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const bool was_ahead = ahead;
         ahead = false;
         auto look_ahead = [&] {  // for the next live item; FAST: while the thread would wait for the last P of tile A
-          walk.next();
+          items.next(ctx);
           more = seek();
         };
         // After the last P V of tile A and before that of tile B, the first S of tile A of that item
         auto issue_ahead = [&]() -> bool {
-          const int ki = kbase + (it.u_end - it.u_begin);
+          const uint32_t ki = kbase + n_tiles;
           ahead = more && mbar_test(&sm.q_full[0], (items_x[0] + 1) & 1) && mbar_test(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1);
           if (!ahead) return true;
           ++items_x[0];  // (the S belongs to the next item's count)
-          const bool b_too = next.act[1] && next.kr[1].begin == next.kr[0].begin;  // tile B uses the key tile as well
-          const bool done = issue_s(0, ki, !b_too, true, next.kr[0].end - next.kr[0].begin == 1);
+          const bool b_too = next.n1 > 0 && next.d == 0;  // tile B uses the key tile as well
+          const bool done = issue_s(0, ki, !b_too, true, next.n0 == 1);
           --items_x[0];
           return done;
         };
-        if (FAST && it.act[0] && it.act[1] && d == 0 && n_x[0] == n_x[1]) {
+        if (FAST && it.d == 0 && it.n0 == it.n1) {
           // Both q tiles on the same key tiles at the same steps: ring tile kbase + i is the i-th key tile of both,
           // tile B its last user.  First, inner and last step are written out.
           using Yes = std::true_type;
           using No = std::false_type;
-          const int n = n_x[0];
+          const int n = it.n0;
           ok = (was_ahead || issue_s(0, kbase, false, true, n == 1)) && issue_s(1, kbase, true, true, n == 1);
           if (n == 1) {
             look_ahead();
@@ -557,8 +505,12 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           } else {
             ok = ok && issue_pv(Yes{}, No{}, 0, kbase, false) && issue_s(0, kbase + 1, false, false, n == 2) &&
                  issue_pv(Yes{}, No{}, 1, kbase, true) && issue_s(1, kbase + 1, true, false, n == 2);
+#pragma unroll 1
             for (int step = 2; ok && step < n; ++step) {
-              ok = issue_pv(No{}, No{}, 0, kbase + step - 1, false) && issue_s(0, kbase + step, false, false, step == n - 1) &&
+              const uint32_t ki = kbase + step, vi = ki - 1;
+              ok = mbar_wait_short(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1, ctx, kWaitKFull) &&
+                   mbar_wait_short(&sm.v_full[vi % kStagesV], (vi / kStagesV) & 1, ctx, kWaitVFull);
+              ok = ok && issue_pv(No{}, No{}, 0, kbase + step - 1, false) && issue_s(0, kbase + step, false, false, step == n - 1, true) &&
                    issue_pv(No{}, No{}, 1, kbase + step - 1, true) && issue_s(1, kbase + step, true, false, step == n - 1);
             }
             look_ahead();
@@ -566,23 +518,25 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
         } else {
           // (the same two issue sequences, written out: through the lambdas this path measured 3-4 % slower)
+#pragma unroll 1
           for (int step = 0; ok && step <= n_steps; ++step) {
   #pragma unroll
             for (int x = 0; x < kQTiles; ++x) {
               if (FAST && x == 0 && step == n_steps) look_ahead();
-              const bool pv_live = it.act[x] && step - 1 >= first_x[x] && step - 1 < first_x[x] + n_x[x];
-              const bool s_live = it.act[x] && step >= first_x[x] && step < first_x[x] + n_x[x];
+              const bool pv_live = step - 1 >= first_x[x] && step - 1 < first_x[x] + n_x[x];
+              const bool s_live = step >= first_x[x] && step < first_x[x] + n_x[x];
               if (pv_live) {
                 const int lx = step - 1 - first_x[x];  // index within this q tile's range
-                const int u = it.kr[x].begin + lx, vi = kbase + (u - it.u_begin), sv = vi % kStagesV;
+                const int u = begin_x[x] + lx;
+                const uint32_t vi = kbase + u, sv = vi % kStagesV;
                 const int px = tiles_x[x] - 1;  // P block consumed now = last S block issued for x
                 KB_FACC(2);
-                if (!mbar_wait(&sm.p_ready[x], px & 1, ctx, kWaitPReady)) { ok = false; break; }
+                if (!mbar_wait_short(&sm.p_ready[x], px & 1, ctx, kWaitPReady)) { ok = false; break; }
                 KB_FACC(3 + x);
-                if (!mbar_wait(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull)) { ok = false; break; }
+                if (!mbar_wait_short(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull)) { ok = false; break; }
                 KB_FACC(5);
                 // the first P V of an item overwrites O: the softmax warps must have read the old one
-                if (lx == 0 && items_x[x] > 0 && !mbar_wait(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree)) { ok = false; break; }
+                if (lx == 0 && items_x[x] > 0 && !mbar_wait_short(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree)) { ok = false; break; }
                 tc_fence_after();
                 // short issue loops (four instructions per trip, descriptor low words stepped by adds): the
                 // scalar work between two MMAs is what the tensor pipe waits for
@@ -591,28 +545,28 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                   // 128 keys = four instructions of 32 keys: 8 packed columns of P, 32 rows (4096 bytes) of V each
   #pragma unroll
                   for (int i = 0; i < 4; ++i)
-                    mma_ts_lo_f8(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, lx > 0 || i > 0);
+                    mma_ts_lo_f8_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, lx > 0 || i > 0);
                 } else {
   #pragma unroll 1
                   for (int h = 0; h < kBN / 64; ++h, p_col += 32, v_lo += 4 * (2048 >> 4)) {
   #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                      mma_ts_lo(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, lx > 0 || h > 0 || i > 0);
+                      mma_ts_lo_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, lx > 0 || h > 0 || i > 0);
                   }
                 }
                 // V_u is free once the last q tile that uses it has consumed it
-                if (last_user(x, u)) mma_commit(&sm.v_empty[sv]);
-                if (u == it.kr[x].end - 1) mma_commit(&sm.o_done[x]);
+                if (last_user(x, u)) mma_commit_if(lead, &sm.v_empty[sv]);
+                if (lx == n_x[x] - 1) mma_commit_if(lead, &sm.o_done[x]);
                 KB_FACC(6);
               }
               if (FAST && x == 0 && step == n_steps && !issue_ahead()) { ok = false; break; }
               if (s_live && !(x == 0 && step == 0 && was_ahead)) {
-                const int t = it.kr[x].begin + (step - first_x[x]);
-                const int ki = kbase + (t - it.u_begin), sk = ki % kStagesK;
+                const int t = begin_x[x] + (step - first_x[x]);
+                const uint32_t ki = kbase + t, sk = ki % kStagesK;
                 KB_FACC(2);
-                if (step == first_x[x] && !mbar_wait(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) { ok = false; break; }
+                if (step == first_x[x] && !mbar_wait_short(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) { ok = false; break; }
                 KB_FACC(1);
-                if (!mbar_wait(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) { ok = false; break; }
+                if (!mbar_wait_short(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) { ok = false; break; }
                 KB_FACC(7);
                 tc_fence_after();
                 uint32_t q_lo = desc_lo_kmajor(smem_u32(sm.q[x])), k_lo = desc_lo_kmajor(smem_u32(sm.k[sk]));
@@ -620,13 +574,13 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 for (int h = 0; h < kPanels; ++h, q_lo += kPanelBytes >> 4, k_lo += kPanelBytes >> 4) {
   #pragma unroll
                   for (int i = 0; i < 4; ++i) {  // 32 bytes of every row per instruction: 16 16-bit or 32 8-bit elements
-                    if (FP8) mma_ss_lo_f8(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
-                    else mma_ss_lo(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+                    if (FP8) mma_ss_lo_f8_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+                    else mma_ss_lo_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
                   }
                 }
-                if (last_user(x, t)) mma_commit(&sm.k_empty[sk]);
-                if (t == it.kr[x].end - 1) mma_commit(&sm.q_empty[x]);
-                mma_commit(&sm.s_ready[x]);
+                if (last_user(x, t)) mma_commit_if(lead, &sm.k_empty[sk]);
+                if (step - first_x[x] == n_x[x] - 1) mma_commit_if(lead, &sm.q_empty[x]);
+                mma_commit_if(lead, &sm.s_ready[x]);
                 ++tiles_x[x];
                 KB_FACC(8);
               }
@@ -634,9 +588,9 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
         }
         if (!FAST) look_ahead();
-        kbase += it.u_end - it.u_begin;
+        kbase += n_tiles;
 #pragma unroll
-        for (int x = 0; x < kQTiles; ++x) items_x[x] += it.act[x] ? 1 : 0;
+        for (int x = 0; x < kQTiles; ++x) items_x[x] += n_x[x] > 0 ? 1 : 0;
       }
 #ifdef KB_TRACE_FWD
       if (blockIdx.x == 60)
@@ -650,25 +604,23 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t t_s = t_lane + kColS + x * 128, t_o = t_lane + kColO + x * 128;
     const float scale_base = a.scale_log2;
-    int tiles = 0, items = 0;  // S blocks / live items of this q tile so far
+    int tiles = 0, live_items = 0;  // S blocks / live items of this q tile so far
     bool ok = true;
 #ifdef KB_TRACE_FWD
     long long acc_t[8] = {0};
     long long tl = clock64();
 #endif
-    for (KbItemWalk<!FAST> walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
-      const Item it = decode(walk.item());
+    for (ItemReader<Reader::kWarp> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
+      const Item it = decode(items.item());
       const int qi = it.q0 + x * kBM + row;
       const int orow = it.row0 + qi - a.q_start;  // this thread's row of o and lse
       uint16_t* o_row = static_cast<uint16_t*>(a.o) + it.b * a.o_sb + it.h * a.o_sh + orow * a.o_st;
       float* lse_row = a.lse ? a.lse + it.b * a.lse_sb + it.h * a.lse_sh + orow : nullptr;
       if (!it.act[x]) {
-        // this q tile lies wholly in the padding: its rows are zeros
-        if (qi < (PACKED ? it.len : T)) {  // a packed batch has no padding rows
-          uint4* dst = reinterpret_cast<uint4*>(o_row);
-#pragma unroll
-          for (int i = 0; i < D * 2 / 16; ++i) dst[i] = make_uint4(0, 0, 0, 0);
-          if (lse_row) *lse_row = 0.f;
+        // this q tile lies wholly in the padding: its rows are zeros (a packed batch has no padding rows)
+        if (!PACKED) {
+          warp_clear_rows<D * 2>(o_row - lane * a.o_st, a.o_st * 2, kb_min_i32(32, T - (qi - lane)));
+          if (qi < T && lse_row) *lse_row = 0.f;
         }
         continue;
       }
@@ -710,17 +662,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         KB_FACC(1);
         const bool warp_full = __all_sync(0xffffffffu, lo <= k0 && k0 + kBN <= hi);
-        constexpr bool kWord = !FAST;
-        constexpr bool kHold = (D == 64) && !FP8;  // one pass with the row's scores held in registers
-        uint32_t s_held[kHold ? kBN : 1];
-        bool dead_held[kBN / 32];
-        float row_max;
-        if (kHold) {
-          row_max = warp_full ? softmax_load_row_max<false>(t_s, reinterpret_cast<uint32_t(&)[kBN]>(s_held), dead_held, k0, lo, hi)
-                              : softmax_load_row_max<true>(t_s, reinterpret_cast<uint32_t(&)[kBN]>(s_held), dead_held, k0, lo, hi);
-        } else {
-          row_max = warp_full ? softmax_row_max<false, kWord>(t_s, k0, lo, hi) : softmax_row_max<true, kWord>(t_s, k0, lo, hi);
-        }
+        uint32_t sc[32];
+        const float row_max = warp_full ? softmax_row_max<false>(t_s, sc, k0, lo, hi) : softmax_row_max<true>(t_s, sc, k0, lo, hi);
         const float m_new = fmaxf(m_used, row_max * scale);
         // lazy rescale: keep the old reference maximum unless the new one is larger by more than the threshold
         const bool need = m_new > m_used + (FP8 ? kRescaleThresholdFp8 : kRescaleThreshold);
@@ -732,17 +675,17 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
         KB_FACC(2);
         KB_FACC(3);
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
         const float m_exp = m_used - p_off;  // 2^(s scale - m_exp) = p * 2^p_off
-        if (kHold) {
-          if (warp_full) softmax_exp_held<BF16, false>(t_s, reinterpret_cast<const uint32_t(&)[kBN]>(s_held), dead_held, scale, m_exp, sum);
-          else softmax_exp_held<BF16, true>(t_s, reinterpret_cast<const uint32_t(&)[kBN]>(s_held), dead_held, scale, m_exp, sum);
-        } else {
-          if (warp_full) softmax_exp_half<BF16, false, FP8, kWord>(t_s, 0, scale, m_exp, k0, lo, hi, sum);
-          else softmax_exp_half<BF16, true, FP8, kWord>(t_s, 0, scale, m_exp, k0, lo, hi, sum);
-          if (warp_full) softmax_exp_half<BF16, false, FP8, kWord>(t_s, 1, scale, m_exp, k0, lo, hi, sum);
-          else softmax_exp_half<BF16, true, FP8, kWord>(t_s, 1, scale, m_exp, k0, lo, hi, sum);
-        }
+        const float m_safe = (m_exp == -INFINITY) ? 0.f : m_exp;
+        const uint64_t scale2 = f2_pack(scale, scale), negm2 = f2_pack(-m_safe, -m_safe);
+        SoftSum sum2;
+        sum2.s01 = sum2.s23 = f2_pack(0.f, 0.f);
+        if (warp_full) softmax_exp<BF16, false, FP8>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
+        else softmax_exp<BF16, true, FP8>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
+        float sum4[4];
+        f2_unpack(sum2.s01, sum4[0], sum4[1]);
+        f2_unpack(sum2.s23, sum4[2], sum4[3]);
+        const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
         // the rescale of O comes after the exponentials: the row's scores are dead by now, which keeps the
         // registers of the two from being live together
         if (lx > 0 && __any_sync(0xffffffffu, need)) {
@@ -760,17 +703,16 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive(&sm.p_ready[x]);
-        if (FP8) l += ((sum[0] + sum[1]) + (sum[2] + sum[3])) * ex2_approx(-p_off);
-        else l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        l += FP8 ? sum * ex2_approx(-p_off) : sum;
         KB_FACC(4);
       }
       if (!ok) break;
       KB_FACC(0);
 
-      ok = __all_sync(0xffffffffu, mbar_wait(&sm.o_done[x], items & 1, ctx, kWaitEpilogue));
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.o_done[x], live_items & 1, ctx, kWaitEpilogue));
       if (!ok) break;
       KB_FACC(5);
-      ++items;
+      ++live_items;
       tc_fence_after();
       // pull the whole O row out of TMEM, release the accumulator to the next item, then store
       uint32_t r[D];
@@ -831,7 +773,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (row == 0) tma_store_wait_all();
 #ifdef KB_TRACE_FWD
     if (blockIdx.x == 60 && threadIdx.x == 0)
-      for (int i = 0; i < 8; ++i) g_fwtrace[16 + i] = acc_t[i];
+      for (int i = 0; i < 8; ++i) g_fwtrace[16 + i] = i < 7 ? acc_t[i] : tiles;
 #endif
   }
 
@@ -863,8 +805,8 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   auto kern = fast ? sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, true> : sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, false>;
   constexpr size_t smem = sizeof(FwdSmem<D>);
   static_assert(sizeof(FwdSmem<D>) <= 232448, "forward shared memory exceeds the 227 KB a CTA may have");
-  int dev = 0, n_sm = 0;
-  if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
+  int dev = 0;
+  KB_CUDA_TRY(cudaGetDevice(&dev));
   static std::atomic<bool> smem_opted_in[kMaxDevices], smem_opted_in_fast[kMaxDevices];
   KB_CUDA_TRY(opt_in_smem_once(kern, smem, dev, fast ? smem_opted_in_fast : smem_opted_in));
   FwdArgs a;
@@ -901,9 +843,7 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   a.Hk = H_kv;
   const int64_t n_items = (int64_t)p.B * p.H * kb_cdiv_i32(Tq, kBM * kQTiles);
   if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
-  const unsigned grid = (unsigned)(n_items < n_sm ? n_items : n_sm);  // persistent: one CTA per SM
-  a.item_rot = fast ? 0 : kb_item_rotation((int32_t)grid, kb_cdiv_i32(Tq, kBM * kQTiles), p.lens || p.cu_seqlens);
-  kern<<<grid, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
+  kern<<<(unsigned)n_items, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
   KB_LAUNCH_CHECK("sa_fwd_sm100_kernel");
   return KB_OK;
 }

@@ -86,7 +86,8 @@ KB_HD int32_t kb_fastdiv(int32_t n, const KbFastDiv& f) {
   return (int32_t)((hi + (uint32_t)n) >> f.shift);
 }
 
-// The order in which the CTAs of a persistent kernel take the work items.  Wave w hands out the items
+// The order in which the CTAs of the main backward kernel take the work items (the others take them as they become free,
+// item_queue.cuh).  Wave w hands out the items
 // [w G, (w + 1) G) (G = CTAs): neighbouring items run at the same time and share their K / V rows in L2.  Inside a
 // wave CTA x takes number (x + w r) mod G.  An item's place in its sequence is item mod n (n = items per sequence and
 // head); with r = 0 a CTA meets only n / gcd(G, n) of the places.  Where sequences differ in length the late places are
@@ -94,20 +95,16 @@ KB_HD int32_t kb_fastdiv(int32_t n, const KbFastDiv& f) {
 // first quarter of every sequence).  r > 0 makes G + r and n coprime, which spreads the places.
 //
 // Only where the lengths differ and a CTA would meet at most `most_places` places (1 to 4).  Measured (B200, r = 0 / r = 1):
-// packed batch of 256 sequences of 128-1024 rows, forward 951 / 843 us, main backward kernel 1286 / 1081, dQ 497 / 402;
-// fp16 D=64 c=10 T=1353 (n = 6, three places) forward 261 / 235 us.  With eight and more places nothing is gained, and
-// an odd r can cost: main kernel, bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r (with an even one
+// packed batch of 256 sequences of 128-1024 rows 1286 / 1081 us.  With eight and more places nothing is gained, and
+// an odd r can cost: bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r (with an even one
 // CTAs 2 m and 2 m + 1 always have the two key tiles of one chunk, which stream the same Q / dO tiles).
 //
-// The main backward kernel therefore shifts chunks that are whole pairs of key tiles (c a multiple of 256) only where a
+// Chunks that are whole pairs of key tiles (c a multiple of 256) are therefore shifted only where a
 // CTA meets fewer places than four.  r = 0 / shifted, us, bf16 D=128, by the places met: padded, lengths T/2 to T: one (T=512)
-// 782 / 818, dQ 330 / 281; two (T=1024) 909 / 977, four (T=2048) 954 / 1035; c=512 T=768 (three) 928 / 1006.  Packed, T/8 to T:
+// 782 / 818; two (T=1024) 909 / 977, four (T=2048) 954 / 1035; c=512 T=768 (three) 928 / 1006.  Packed, T/8 to T:
 // one 1390 / 1145, two 1369 / 1340, four 1400 / 1470.  fp16 D=64 c=256, padded: one 334 / 289, two 409 / 385, four 451 /
 // 464.  Hence at most two, at most one for the padded head-dim-128 class.  (Other chunk lengths gain everywhere, but for
-// c=160 and 192 at T=512: 784 / 834, with dQ 361 / 297 and the forward 708 / 625.)
-//
-// The forward's straight-line instance takes no shift: bf16 D=128 c=256 ragged T=512 601 / 535 us, T=1024 679 / 616, but
-// T=2048 501 / 532; dense fp16 D=64 375 / 376.
+// c=160 and 192 at T=512: 784 / 834.)
 inline int32_t kb_gcd(int32_t a, int32_t b) {
   while (b) {
     const int32_t t = a % b;
@@ -124,15 +121,12 @@ inline int32_t kb_item_rotation(int32_t ctas, int32_t items_per_seq, bool ragged
   return r % ctas;
 }
 #if defined(__CUDACC__)
-// ROT = false: r = 0 known at compile time.
-template <bool ROT = true>
 struct KbItemWalk {
   int32_t base, off, rot;
   __device__ __forceinline__ explicit KbItemWalk(int32_t rotation) : base(0), off((int32_t)blockIdx.x), rot(rotation) {}
   __device__ __forceinline__ int32_t item() const { return base + off; }  // the walk ends at the first item() >= n_items
   __device__ __forceinline__ void next() {
     base += (int32_t)gridDim.x;
-    if (!ROT) return;
     off += rot;
     if (off >= (int32_t)gridDim.x) off -= (int32_t)gridDim.x;
   }

@@ -64,6 +64,8 @@ def _run_case(B, H, T, D, c, back, dtype, lens_mode, noncontiguous, seed=20, che
         lens = _tricky_lens(B, T, c, back, rng)
     elif lens_mode == "random":
         lens = torch.from_numpy(rng.randint(1, T + 1, B).astype(np.int32))
+    elif torch.is_tensor(lens_mode):
+        lens = lens_mode
 
     ref_out, ref_dq, ref_dk, ref_dv = SO.oracle_fwd_bwd(q, k, v, dout, c, back, lens)
     res_mask = torch.ones(B, 1, T, 1, dtype=torch.bool)
@@ -176,6 +178,14 @@ def test_long_sequence_class_with_several_work_items_per_cta(D):
     """Chunks of 256 rows, 320 forward and 640 backward work items: more than one per CTA, through the kernel
     instances whose MMA threads run the specialised issue sequences, against the oracle."""
     _run_case(2, 40, 1024, D, 256, 2, torch.bfloat16, "random", False)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("c, back", [(10, 9), (128, 1), (256, 2)])
+def test_long_runs_of_padded_work_items(D, c, back):
+    """More work items than CTAs, and between the live ones runs of up to 72 (132 in the backward) that lie wholly in the
+    padding: a CTA takes many of them in a row, their outputs are zeros, the next live item is found."""
+    _run_case(6, 12, 1300, D, c, back, torch.bfloat16, torch.tensor([1300, 0, 1, 0, 700, 129], dtype=torch.int32), False)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=str)
