@@ -49,6 +49,7 @@
 #include "common.cuh"
 #include <type_traits>
 
+#include "item_queue.cuh"
 #include "sm100_ptx.cuh"
 #include "sm100_host.h"
 #include "tiles.h"
@@ -106,7 +107,7 @@ struct FusedArgs {
   const int32_t* cu;
   int32_t total, n_ptiles;
   KbFastDiv fd_tiles, fd_H, fd_Hk, fd_group, fd_c;  // division by ceil(T / 128), H, Hk, group and c
-  int32_t item_rot, item_rot_dq;  // main / dQ kernel, see KbItemWalk
+  int32_t item_rot;  // main kernel, see KbItemWalk
   float scale_log2, sm_scale;
   int32_t* status;
 };
@@ -890,8 +891,9 @@ __global__ void __launch_bounds__(256) sa_bwd_delta_kernel(const DeltaArgs a) {
 }
 
 // ---- dQ = sm_scale * sum_j dS_j^T K_j over the saved dS tiles ----
-// Persistent, one CTA per SM, six warps: warps 0-3 epilogue (thread = query row = TMEM lane),
-// warp 4 producer (one lane: a 32 KB bulk copy of dS and a TMA tile of K per stage, three stages),
+// Persistent, one CTA per SM, which takes work items until there are none left (item_queue.cuh; a static order / this one:
+// packed batch of 256 sequences of 128-1024 rows 415 / 345 us, bf16 c=64 T=8192 439 / 428, c=256 T=16384 609 / 605).  Six warps: warps 0-3 epilogue (thread = query row = TMEM lane),
+// warp 4 producer (a 32 KB bulk copy of dS and a TMA tile of K per stage, three stages),
 // warp 5 MMA issuer (one lane) and TMEM owner.  The accumulator is double buffered in TMEM so that
 // the MMAs of the next item run while the epilogue warps convert and store the finished one.
 constexpr int kDqStages = tiles::kDqStages;
@@ -905,6 +907,7 @@ struct alignas(1024) DqSmem {
   uint8_t k[kDqStages][kBK * D * 2];
   uint8_t out[kBQ * D * 2];
   uint64_t full[kDqStages], empty[kDqStages], acc_done[2], acc_free[2];
+  ItemQueue items;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -934,7 +937,6 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = a.T;
   const int n_tiles_t = kb_cdiv_i32(T, kBQ);  // query tiles = key tiles per sequence
-  const int n_items = a.B * a.H * n_tiles_t;
 
   if (smem_u32(smem_raw) & 1023u) {
     if (threadIdx.x == 0 && a.status) {
@@ -952,6 +954,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       mbar_init(&sm.acc_done[i], 1);
       mbar_init(&sm.acc_free[i], 128);
     }
+    item_queue_init(sm.items, 1 + 4);  // MMA; epilogue warps
     sm.abort_flag = 0;
     fence_mbar_init();
   }
@@ -966,36 +969,44 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 
   // u counts the (query tile, key tile) pairs of this CTA so far, m its items with at least one pair
   if (warp == kDqProducerWarp) {
-    if (lane == 0) {
-      prefetch_tensormap(&tm_k);
-      int u = 0;
-      bool ok = true;
-      for (KbItemWalk walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
-        const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
-        for (int j = it.kr.begin; j < it.kr.end; ++j, ++u) {
-          const int s = u % kDqStages;
-          if (u >= kDqStages && !mbar_wait<kRelaxedNs>(&sm.empty[s], ((u / kDqStages) - 1) & 1, ctx, kWDqEmpty)) { ok = false; break; }
-          // the slot this query tile has in key tile j's list: both schedules name the same pairs
-          const KbTileRange qr = kb_bwd_q_range_fd(j * kBK, kBQ, kBK, it.len, a.c, a.back, a.fd_c);
-          mbar_expect_tx(&sm.full[s], kDsTileBytes + kTileBytes);
-          bulk_load(sm.ds[s], ds_slot<PACKED>(a, it.b, it.row0, it.h, j, n_tiles_t, it.qt - qr.begin), kDsTileBytes, &sm.full[s]);
+    if (lane == 0) prefetch_tensormap(&tm_k);
+    int u = 0;
+    bool ok = true;
+    ItemWriter items(sm.items);
+    for (; items.item() >= 0; items.next(ok, ctx)) {
+      const DqItem it = decode_dq_item<PACKED>(a, items.item(), n_tiles_t);
+      if (it.kr.begin >= it.kr.end) {
+        // the whole query tile lies in the padding: its gradient is zero.  A packed batch has no padding rows.
+        const int q0 = it.qt * kBQ;
+        if (!PACKED)
+          warp_clear_rows<D * 2>(static_cast<uint16_t*>(a.dq) + it.b * a.dq_sb + it.h * a.dq_sh + q0 * a.dq_st, a.dq_st * 2, kb_min_i32(kBQ, T - q0));
+        continue;
+      }
+      if (lane != 0) continue;
+      ok = items.publish(make_int4(items.item(), it.kr.end - it.kr.begin, 0, 0), ctx);
+      for (int j = it.kr.begin; ok && j < it.kr.end; ++j, ++u) {
+        const int s = u % kDqStages;
+        if (j == it.kr.end - 1) items.ask();
+        if (u >= kDqStages && !mbar_wait<kRelaxedNs>(&sm.empty[s], ((u / kDqStages) - 1) & 1, ctx, kWDqEmpty)) { ok = false; break; }
+        // the slot this query tile has in key tile j's list: both schedules name the same pairs
+        const KbTileRange qr = kb_bwd_q_range_fd(j * kBK, kBQ, kBK, it.len, a.c, a.back, a.fd_c);
+        mbar_expect_tx(&sm.full[s], kDsTileBytes + kTileBytes);
+        bulk_load(sm.ds[s], ds_slot<PACKED>(a, it.b, it.row0, it.h, j, n_tiles_t, it.qt - qr.begin), kDsTileBytes, &sm.full[s]);
 #pragma unroll
-          for (int p = 0; p < kPanels; ++p)
-            tma_load_4d(sm.k[s] + p * kPanelBytes, &tm_k, &sm.full[s], p * 64, it.row0 + j * kBK, kb_fastdiv(it.h, a.fd_group), PACKED ? 0 : it.b);
-        }
+        for (int p = 0; p < kPanels; ++p)
+          tma_load_4d(sm.k[s] + p * kPanelBytes, &tm_k, &sm.full[s], p * 64, it.row0 + j * kBK, kb_fastdiv(it.h, a.fd_group), PACKED ? 0 : it.b);
       }
     }
+    if (lane == 0) items.finish(ctx);
   } else if (warp == kDqMmaWarp) {
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc(BF16, kBQ, D, true, true);  // A = dS read MN-major (rows = keys), B = K MN-major
       int u = 0, m = 0;
       bool ok = true;
-      for (KbItemWalk walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
-        const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
-        if (it.kr.begin >= it.kr.end) continue;
+      for (ItemReader<Reader::kThread> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
         const uint32_t acc = tmem + (m & 1) * 128;
         if (m >= 2 && !mbar_wait(&sm.acc_free[m & 1], ((m >> 1) - 1) & 1, ctx, kWDqAccFree)) break;
-        for (int j = it.kr.begin; j < it.kr.end; ++j, ++u) {
+        for (int j = 0; j < items.e.y; ++j, ++u) {
           const int s = u % kDqStages;
           if (!mbar_wait(&sm.full[s], (u / kDqStages) & 1, ctx, kWDqFull)) { ok = false; break; }
           tc_fence_after();
@@ -1004,7 +1015,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
           for (int h = 0; h < kBK / 64; ++h, ds_lo += 4 * (2048 >> 4), k_lo += 4 * (2048 >> 4)) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              mma_ss_lo(acc, ds_lo + i * (2048 >> 4), k_lo + i * (2048 >> 4), idesc, j > it.kr.begin || h > 0 || i > 0);
+              mma_ss_lo(acc, ds_lo + i * (2048 >> 4), k_lo + i * (2048 >> 4), idesc, j > 0 || h > 0 || i > 0);
           }
           mma_commit(&sm.empty[s]);
         }
@@ -1017,19 +1028,9 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
     int m = 0;
     bool ok = true;
-    for (KbItemWalk walk(a.item_rot_dq); ok && walk.item() < n_items; walk.next()) {
-      const DqItem it = decode_dq_item<PACKED>(a, walk.item(), n_tiles_t);
+    for (ItemReader<Reader::kWarp> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
+      const DqItem it = decode_dq_item<PACKED>(a, items.item(), n_tiles_t);
       const int qi = it.qt * kBQ + row;
-      if (it.kr.begin >= it.kr.end) {
-        // the whole query tile lies in the padding: its gradient is zero (rare; plain stores); a packed batch
-        // has no padding rows
-        if (!PACKED && qi < T) {
-          uint4* dq_row = reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.dq) + it.b * a.dq_sb + it.h * a.dq_sh + qi * a.dq_st);
-#pragma unroll
-          for (int i = 0; i < D * 2 / 16; ++i) dq_row[i] = make_uint4(0, 0, 0, 0);
-        }
-        continue;
-      }
       // packed batch, last query tile of a sequence: the rows below belong to the next sequence, so no box
       // store; every thread writes its own row
       const bool partial = PACKED && it.qt * kBQ + kBQ > it.len;
@@ -1103,7 +1104,6 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
   int dev = 0, n_sm = 0;
   if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
-  const unsigned grid = (unsigned)(n_items < n_sm ? n_items : n_sm);  // persistent: one CTA per SM (dQ kernel)
   const int64_t n_items_main = (int64_t)p.B * Hk * n_tiles;
   const unsigned grid_main = (unsigned)(n_items_main < n_sm ? n_items_main : n_sm);
 
@@ -1177,14 +1177,13 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.sm_scale = p.sm_scale;
   const int32_t most_places = c % (2 * kBK) ? 4 : mid && !PACKED ? 1 : 2;  // see kb_item_rotation
   fa.item_rot = kb_item_rotation((int32_t)grid_main, n_tiles, p.lens || PACKED, most_places);
-  fa.item_rot_dq = kb_item_rotation((int32_t)grid, n_tiles, p.lens || PACKED);
   fa.status = p.status;
   if (!(p.flags & KB_FLAG_BWD_SKIP_DKDV)) {
     main_kern<<<grid_main, kThreads, sizeof(FusedSmem<D>), s>>>(tm_k, tm_v, tm_q, tm_do, tm_dk, tm_dv, fa);
     KB_LAUNCH_CHECK("sa_bwd_fused_kernel");
   }
   if (!(p.flags & KB_FLAG_BWD_SKIP_DQ)) {
-    dq_kern<<<grid, kDqThreads, sizeof(DqSmem<D>), s>>>(tm_k, tm_dq, fa);
+    dq_kern<<<(unsigned)n_items, kDqThreads, sizeof(DqSmem<D>), s>>>(tm_k, tm_dq, fa);
     KB_LAUNCH_CHECK("sa_bwd_dq_kernel");
   }
   return KB_OK;
