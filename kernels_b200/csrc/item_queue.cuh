@@ -115,12 +115,8 @@ struct ItemWriter {
   }
 };
 
-enum class Reader {
-  kThread,  // one thread
-  kWarp,    // a whole converged warp, all of whose lanes leave together if a wait gives up
-  kLead     // a warp of which only lane 0 has effects; the others follow it, each with waits of its own
-};
-template <Reader KIND>
+// WARP: the reader is a whole converged warp, all of whose lanes leave together if a wait gives up; else one thread.
+template <bool WARP>
 struct ItemReader {
   ItemQueue* q;
   int n;   // entries read so far
@@ -130,11 +126,11 @@ struct ItemReader {
   __device__ __forceinline__ void next(const WaitCtx& ctx) {
     const int s = n % kItemSlots;
     bool ok = mbar_wait(&q->full[s], (n / kItemSlots) & 1, ctx, kWaitItemFull);
-    if (KIND == Reader::kWarp) ok = __all_sync(0xffffffffu, ok);
+    if (WARP) ok = __all_sync(0xffffffffu, ok);
     e = q->entry[s];
     if (!ok) e.x = -1;
-    if (KIND == Reader::kWarp) __syncwarp();
-    if (KIND == Reader::kThread || (threadIdx.x & 31) == 0) mbar_arrive(&q->empty[s]);
+    if (WARP) __syncwarp();
+    if (!WARP || (threadIdx.x & 31) == 0) mbar_arrive(&q->empty[s]);
     ++n;
   }
 };

@@ -392,7 +392,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         }
         mbar_arrive(&sm.stats_full[g & 1]);
       }
-    } else if (warp == kMmaWarp && lane == 0) {
+    } else if (warp == kMmaWarp && elect_one()) {
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t idesc_z = make_idesc(BF16, kBK, kBQ, false, false);  // S, dP
       constexpr uint32_t idesc_acc = make_idesc(BF16, kBK, D, false, true);   // dV, dK (A in TMEM)
@@ -999,11 +999,11 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     }
     if (lane == 0) items.finish(ctx);
   } else if (warp == kDqMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(BF16, kBQ, D, true, true);  // A = dS read MN-major (rows = keys), B = K MN-major
       int u = 0, m = 0;
       bool ok = true;
-      for (ItemReader<Reader::kThread> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
+      for (ItemReader<false> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
         const uint32_t acc = tmem + (m & 1) * 128;
         if (m >= 2 && !mbar_wait(&sm.acc_free[m & 1], ((m >> 1) - 1) & 1, ctx, kWDqAccFree)) break;
         for (int j = 0; j < items.e.y; ++j, ++u) {
@@ -1028,7 +1028,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
     int m = 0;
     bool ok = true;
-    for (ItemReader<Reader::kWarp> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
+    for (ItemReader<true> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
       const DqItem it = decode_dq_item<PACKED>(a, items.item(), n_tiles_t);
       const int qi = it.qt * kBQ + row;
       // packed batch, last query tile of a sequence: the rows below belong to the next sequence, so no box

@@ -11,7 +11,7 @@
 //              writes O / LSE at the end;
 //   warp 8     TMA producer (one lane): Q once, then a ring of K tiles and a ring of V tiles; takes the work
 //              items from the hardware's queue (item_queue.cuh) and clears the outputs of padded ones;
-//   warp 9     MMA issuer (a converged warp, one lane's instructions count): S = Q K^T (A, B from shared memory), O += P V
+//   warp 9     MMA issuer (a converged warp that elects a lane for every group of MMAs): S = Q K^T (A, B from shared memory), O += P V
 //              (A = P from TMEM, B = V from shared memory, MN-major); owns the TMEM allocation.
 // MMA issue order per KV tile t:  PV_A(t-1)  S_A(t)  PV_B(t-1)  S_B(t).  While the softmax warps
 // of one q tile work on their S block the tensor pipe runs the other q tile's MMAs.  MMAs
@@ -369,7 +369,6 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issuer ------------------------------
     {
-      const bool lead = lane == 0;
       constexpr uint32_t idesc_qk = FP8 ? make_idesc_e4m3(kBM, kBN, false, false) : make_idesc(BF16, kBM, kBN, false, false);
       constexpr uint32_t idesc_pv = FP8 ? make_idesc_e4m3(kBM, D, false, true) : make_idesc(BF16, kBM, D, false, true);
       uint32_t kbase = 0;                    // K (= V) tiles of earlier items
@@ -384,7 +383,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // item before it, where its Q and K have landed by then (`ahead`): tile A's softmax warps go from one item to the
       // next without waiting for tile B's last block.  (Q has a barrier pair per q tile for this: a Q buffer is free
       // after ITS tile's last S.)  bf16 D=128 c=256 T=16384: 865 -> 830 us, T=2048: 116 -> 109, 8-bit 217 -> 211.
-      ItemReader<Reader::kLead> items(sm.items, ctx);
+      ItemReader<true> items(sm.items, ctx);
       // Of an item this thread needs how many key tiles each q tile walks (tile A at least one; tile B none if it lies in the
       // padding), and how many key tiles after tile A's tile B's begin.
       struct Walk {
@@ -422,31 +421,34 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           const uint32_t sv = vi % kStagesV;
           const int px = tiles_x[x] - 1;  // P block consumed now = last S block issued for x
           KB_FACC(2);
-          if (!mbar_wait_short(&sm.p_ready[x], px & 1, ctx, kWaitPReady)) return false;
+          bool got = mbar_wait_short(&sm.p_ready[x], px & 1, ctx, kWaitPReady);
           KB_FACC(3 + x);
-          if (!release_v && (kFirst || kLast) && !mbar_wait_short(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull)) return false;
+          if (!release_v && (kFirst || kLast)) got = mbar_wait_short(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull) && got;
           KB_FACC(5);
           // the first P V of an item overwrites O: the softmax warps must have read the old one
-          if (kFirst && items_x[x] > 0 && !mbar_wait_short(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree)) return false;
+          if (kFirst && items_x[x] > 0) got = mbar_wait_short(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree) && got;
+          if (!__all_sync(0xffffffffu, got)) return false;
           tc_fence_after();
-          // short issue loops (four instructions per trip, descriptor low words stepped by adds): the
-          // scalar work between two MMAs is what the tensor pipe waits for
-          uint32_t p_col = tmem + kColS + x * 128, v_lo = desc_lo_mnmajor(smem_u32(sm.v[sv]), kPanelBytes);
-          if (FP8) {
-            // 128 keys = four instructions of 32 keys: 8 packed columns of P, 32 rows (4096 bytes) of V each
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              mma_ts_lo_f8_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, !kFirst || i > 0);
-          } else {
-#pragma unroll 1
-            for (int h = 0; h < kBN / 64; ++h, p_col += 32, v_lo += 4 * (2048 >> 4)) {
+          if (elect_one()) {
+            // short issue loops (four instructions per trip, descriptor low words stepped by adds): the
+            // scalar work between two MMAs is what the tensor pipe waits for
+            uint32_t p_col = tmem + kColS + x * 128, v_lo = desc_lo_mnmajor(smem_u32(sm.v[sv]), kPanelBytes);
+            if (FP8) {
+              // 128 keys = four instructions of 32 keys: 8 packed columns of P, 32 rows (4096 bytes) of V each
 #pragma unroll
               for (int i = 0; i < 4; ++i)
-                mma_ts_lo_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, !kFirst || h > 0 || i > 0);
+                mma_ts_lo_f8(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, !kFirst || i > 0);
+            } else {
+#pragma unroll 1
+              for (int h = 0; h < kBN / 64; ++h, p_col += 32, v_lo += 4 * (2048 >> 4)) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  mma_ts_lo(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, !kFirst || h > 0 || i > 0);
+              }
             }
+            if (release_v) mma_commit(&sm.v_empty[sv]);  // V is free once the last q tile that uses it has consumed it
+            if (kLast) mma_commit(&sm.o_done[x]);
           }
-          if (release_v) mma_commit_if(lead, &sm.v_empty[sv]);  // V is free once the last q tile that uses it has consumed it
-          if (kLast) mma_commit_if(lead, &sm.o_done[x]);
           KB_FACC(6);
           return true;
         };
@@ -454,23 +456,26 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         auto issue_s = [&](int x, uint32_t ki, bool release_k, bool first, bool last, bool waited = false) -> bool {
           const uint32_t sk = ki % kStagesK;
           KB_FACC(2);
-          if (first && !mbar_wait_short(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) return false;
+          bool got = !first || mbar_wait_short(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ);
           KB_FACC(1);
-          if (x == 0 && !waited && !mbar_wait_short(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) return false;
+          if (x == 0 && !waited) got = mbar_wait_short(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull) && got;
           KB_FACC(7);
+          if ((first || (x == 0 && !waited)) && !__all_sync(0xffffffffu, got)) return false;
           tc_fence_after();
-          uint32_t q_lo = desc_lo_kmajor(smem_u32(sm.q[x])), k_lo = desc_lo_kmajor(smem_u32(sm.k[sk]));
+          if (elect_one()) {
+            uint32_t q_lo = desc_lo_kmajor(smem_u32(sm.q[x])), k_lo = desc_lo_kmajor(smem_u32(sm.k[sk]));
 #pragma unroll 1
-          for (int h = 0; h < kPanels; ++h, q_lo += kPanelBytes >> 4, k_lo += kPanelBytes >> 4) {
+            for (int h = 0; h < kPanels; ++h, q_lo += kPanelBytes >> 4, k_lo += kPanelBytes >> 4) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {  // 32 bytes of every row per instruction: 16 16-bit or 32 8-bit elements
-              if (FP8) mma_ss_lo_f8_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
-              else mma_ss_lo_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+              for (int i = 0; i < 4; ++i) {  // 32 bytes of every row per instruction: 16 16-bit or 32 8-bit elements
+                if (FP8) mma_ss_lo_f8(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+                else mma_ss_lo(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+              }
             }
+            if (release_k) mma_commit(&sm.k_empty[sk]);
+            if (last) mma_commit(&sm.q_empty[x]);
+            mma_commit(&sm.s_ready[x]);
           }
-          if (release_k) mma_commit_if(lead, &sm.k_empty[sk]);
-          if (last) mma_commit_if(lead, &sm.q_empty[x]);
-          mma_commit_if(lead, &sm.s_ready[x]);
           ++tiles_x[x];
           KB_FACC(8);
           return true;
@@ -484,7 +489,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // After the last P V of tile A and before that of tile B, the first S of tile A of that item
         auto issue_ahead = [&]() -> bool {
           const uint32_t ki = kbase + n_tiles;
-          ahead = more && mbar_test(&sm.q_full[0], (items_x[0] + 1) & 1) && mbar_test(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1);
+          ahead = more && __all_sync(0xffffffffu, mbar_test(&sm.q_full[0], (items_x[0] + 1) & 1) && mbar_test(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1));
           if (!ahead) return true;
           ++items_x[0];  // (the S belongs to the next item's count)
           const bool b_too = next.n1 > 0 && next.d == 0;  // tile B uses the key tile as well
@@ -508,8 +513,10 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll 1
             for (int step = 2; ok && step < n; ++step) {
               const uint32_t ki = kbase + step, vi = ki - 1;
-              ok = mbar_wait_short(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1, ctx, kWaitKFull) &&
-                   mbar_wait_short(&sm.v_full[vi % kStagesV], (vi / kStagesV) & 1, ctx, kWaitVFull);
+              // (the waits for K and V come before the one for P, off the chain P -> P V -> S -> P)
+              const bool k_in = mbar_wait_short(&sm.k_full[ki % kStagesK], (ki / kStagesK) & 1, ctx, kWaitKFull);
+              const bool v_in = mbar_wait_short(&sm.v_full[vi % kStagesV], (vi / kStagesV) & 1, ctx, kWaitVFull);
+              ok = __all_sync(0xffffffffu, k_in && v_in);
               ok = ok && issue_pv(No{}, No{}, 0, kbase + step - 1, false) && issue_s(0, kbase + step, false, false, step == n - 1, true) &&
                    issue_pv(No{}, No{}, 1, kbase + step - 1, true) && issue_s(1, kbase + step, true, false, step == n - 1);
             }
@@ -531,32 +538,35 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const uint32_t vi = kbase + u, sv = vi % kStagesV;
                 const int px = tiles_x[x] - 1;  // P block consumed now = last S block issued for x
                 KB_FACC(2);
-                if (!mbar_wait_short(&sm.p_ready[x], px & 1, ctx, kWaitPReady)) { ok = false; break; }
+                bool got = mbar_wait_short(&sm.p_ready[x], px & 1, ctx, kWaitPReady);
                 KB_FACC(3 + x);
-                if (!mbar_wait_short(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull)) { ok = false; break; }
+                got = mbar_wait_short(&sm.v_full[sv], (vi / kStagesV) & 1, ctx, kWaitVFull) && got;
                 KB_FACC(5);
                 // the first P V of an item overwrites O: the softmax warps must have read the old one
-                if (lx == 0 && items_x[x] > 0 && !mbar_wait_short(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree)) { ok = false; break; }
+                if (lx == 0 && items_x[x] > 0) got = mbar_wait_short(&sm.o_free[x], (items_x[x] - 1) & 1, ctx, kWaitOFree) && got;
+                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
                 tc_fence_after();
-                // short issue loops (four instructions per trip, descriptor low words stepped by adds): the
-                // scalar work between two MMAs is what the tensor pipe waits for
-                uint32_t p_col = tmem + kColS + x * 128, v_lo = desc_lo_mnmajor(smem_u32(sm.v[sv]), kPanelBytes);
-                if (FP8) {
-                  // 128 keys = four instructions of 32 keys: 8 packed columns of P, 32 rows (4096 bytes) of V each
-  #pragma unroll
-                  for (int i = 0; i < 4; ++i)
-                    mma_ts_lo_f8_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, lx > 0 || i > 0);
-                } else {
-  #pragma unroll 1
-                  for (int h = 0; h < kBN / 64; ++h, p_col += 32, v_lo += 4 * (2048 >> 4)) {
-  #pragma unroll
+                if (elect_one()) {
+                  // short issue loops (four instructions per trip, descriptor low words stepped by adds): the
+                  // scalar work between two MMAs is what the tensor pipe waits for
+                  uint32_t p_col = tmem + kColS + x * 128, v_lo = desc_lo_mnmajor(smem_u32(sm.v[sv]), kPanelBytes);
+                  if (FP8) {
+                    // 128 keys = four instructions of 32 keys: 8 packed columns of P, 32 rows (4096 bytes) of V each
+#pragma unroll
                     for (int i = 0; i < 4; ++i)
-                      mma_ts_lo_if(lead, tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, lx > 0 || h > 0 || i > 0);
+                      mma_ts_lo_f8(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (4096 >> 4), idesc_pv, lx > 0 || i > 0);
+                  } else {
+#pragma unroll 1
+                    for (int h = 0; h < kBN / 64; ++h, p_col += 32, v_lo += 4 * (2048 >> 4)) {
+#pragma unroll
+                      for (int i = 0; i < 4; ++i)
+                        mma_ts_lo(tmem + kColO + x * 128, p_col + 8 * i, v_lo + i * (2048 >> 4), idesc_pv, lx > 0 || h > 0 || i > 0);
+                    }
                   }
+                  // V_u is free once the last q tile that uses it has consumed it
+                  if (last_user(x, u)) mma_commit(&sm.v_empty[sv]);
+                  if (lx == n_x[x] - 1) mma_commit(&sm.o_done[x]);
                 }
-                // V_u is free once the last q tile that uses it has consumed it
-                if (last_user(x, u)) mma_commit_if(lead, &sm.v_empty[sv]);
-                if (lx == n_x[x] - 1) mma_commit_if(lead, &sm.o_done[x]);
                 KB_FACC(6);
               }
               if (FAST && x == 0 && step == n_steps && !issue_ahead()) { ok = false; break; }
@@ -564,23 +574,26 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const int t = begin_x[x] + (step - first_x[x]);
                 const uint32_t ki = kbase + t, sk = ki % kStagesK;
                 KB_FACC(2);
-                if (step == first_x[x] && !mbar_wait_short(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ)) { ok = false; break; }
+                bool got = step != first_x[x] || mbar_wait_short(&sm.q_full[x], items_x[x] & 1, ctx, kWaitQ);
                 KB_FACC(1);
-                if (!mbar_wait_short(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull)) { ok = false; break; }
+                got = mbar_wait_short(&sm.k_full[sk], (ki / kStagesK) & 1, ctx, kWaitKFull) && got;
                 KB_FACC(7);
+                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
                 tc_fence_after();
-                uint32_t q_lo = desc_lo_kmajor(smem_u32(sm.q[x])), k_lo = desc_lo_kmajor(smem_u32(sm.k[sk]));
-  #pragma unroll 1
-                for (int h = 0; h < kPanels; ++h, q_lo += kPanelBytes >> 4, k_lo += kPanelBytes >> 4) {
-  #pragma unroll
-                  for (int i = 0; i < 4; ++i) {  // 32 bytes of every row per instruction: 16 16-bit or 32 8-bit elements
-                    if (FP8) mma_ss_lo_f8_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
-                    else mma_ss_lo_if(lead, tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+                if (elect_one()) {
+                  uint32_t q_lo = desc_lo_kmajor(smem_u32(sm.q[x])), k_lo = desc_lo_kmajor(smem_u32(sm.k[sk]));
+#pragma unroll 1
+                  for (int h = 0; h < kPanels; ++h, q_lo += kPanelBytes >> 4, k_lo += kPanelBytes >> 4) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {  // 32 bytes of every row per instruction: 16 16-bit or 32 8-bit elements
+                      if (FP8) mma_ss_lo_f8(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+                      else mma_ss_lo(tmem + kColS + x * 128, q_lo + 2 * i, k_lo + 2 * i, idesc_qk, h > 0 || i > 0);
+                    }
                   }
+                  if (last_user(x, t)) mma_commit(&sm.k_empty[sk]);
+                  if (step - first_x[x] == n_x[x] - 1) mma_commit(&sm.q_empty[x]);
+                  mma_commit(&sm.s_ready[x]);
                 }
-                if (last_user(x, t)) mma_commit_if(lead, &sm.k_empty[sk]);
-                if (step - first_x[x] == n_x[x] - 1) mma_commit_if(lead, &sm.q_empty[x]);
-                mma_commit_if(lead, &sm.s_ready[x]);
                 ++tiles_x[x];
                 KB_FACC(8);
               }
@@ -610,7 +623,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     long long acc_t[8] = {0};
     long long tl = clock64();
 #endif
-    for (ItemReader<Reader::kWarp> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
+    for (ItemReader<true> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
       const Item it = decode(items.item());
       const int qi = it.q0 + x * kBM + row;
       const int orow = it.row0 + qi - a.q_start;  // this thread's row of o and lse
