@@ -9,8 +9,8 @@
 // padding itself and passes the live ones to the other roles through a ring of kItemSlots numbers in shared memory
 // (ItemReader).  (Padded items do not go through the ring: a role may look for the next live item before the current one
 // is complete, and would wait for ever behind a run of padded ones that fills the ring.)  It asks when it starts on the
-// last tile of an item: the answer takes less than the tile, and an item claimed earlier would wait at a CTA that is
-// still busy.
+// last tiles of an item: the answer takes 350 clocks, and an item claimed earlier would wait at a CTA that is still busy.
+// Or (n_fixed) it takes the items in turn with the grid's other CTAs; sa_bwd_fused_sm100.cu says where that is better.
 #pragma once
 #include "sm100_ptx.cuh"
 
@@ -72,14 +72,15 @@ static __device__ __noinline__ void item_drop_rest(ItemQueue* q, int answers, bo
 // Used by a whole converged warp; item() is the same in all lanes, the rest is lane 0's.
 struct ItemWriter {
   ItemQueue* q;
+  int n_fixed;                    // > 0: the CTAs of the grid take these items in turn, nothing is asked for
   int answers, published, item_;  // answers taken, items passed on so far; the current item, -1 after the last one
   bool asked, more, ok;          // a request is under way; no request has failed yet; no wait gave up
-  __device__ __forceinline__ explicit ItemWriter(ItemQueue& queue)
-      : q(&queue), answers(0), published(0), item_((int)blockIdx.x), asked(false), more(true), ok(true) {}
+  __device__ __forceinline__ explicit ItemWriter(ItemQueue& queue, int fixed = 0)
+      : q(&queue), n_fixed(fixed), answers(0), published(0), item_((int)blockIdx.x), asked(false), more(fixed == 0), ok(true) {}
   __device__ __forceinline__ int item() const { return item_; }
   // Lane 0: ask for the next item ahead of next().
   __device__ __forceinline__ void ask() {
-    if (!asked) item_ask(q);
+    if (!asked && n_fixed == 0) item_ask(q);
     asked = true;
   }
   // Lane 0: pass an item on to the readers.
@@ -95,7 +96,10 @@ struct ItemWriter {
     int got = -1;
     if ((threadIdx.x & 31) == 0) {
       ok = go_on;
-      if (ok) {
+      if (ok && n_fixed > 0) {
+        got = item_ + (int)gridDim.x;
+        if (got >= n_fixed) got = -1;
+      } else if (ok) {
         ask();
         ok = mbar_wait(&q->answered, answers & 1, ctx, kWaitItemAnswer);
         if (ok) {

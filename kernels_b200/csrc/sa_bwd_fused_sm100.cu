@@ -4,7 +4,8 @@
 //
 // Three launches:
 //   1. delta   delta = rowsum(O * dO) per row;
-//   2. main    persistent, one CTA per SM.  A work item is one tile of 128 key rows of one
+//   2. main    persistent, one CTA per SM, which takes work items until there are none left
+//              (item_queue.cuh).  A work item is one tile of 128 key rows of one
 //              (batch, head); the CTA keeps K and V of the item in shared memory and streams the
 //              128-row Q / dO tiles of the transposed schedule (schedule.h).  Per tile pair
 //                  S  = K Q^T            dP = V dO^T                 (keys x queries, into TMEM)
@@ -25,7 +26,7 @@
 //               of every tile.  Phase 1 turns S into P (16-bit, back into TMEM over S); phase 2
 //               turns dP into dS (16-bit, into TMEM over dP and into shared memory);
 //   warps 8-11  epilogue: end of item, dV and dK TMEM -> 16-bit -> shared memory -> TMA store;
-//   warp 12     TMA producer (one lane);
+//   warp 12     TMA producer (one lane); takes the work items, clears the outputs of padded ones;
 //   warp 13     MMA issuer (one lane), owner of the TMEM allocation;
 //   warp 14     one lane sends each dS tile to the scratch buffer;
 //   warp 15     per-tile staging of lse / delta into shared memory (whole warp; a role of its own so that the
@@ -107,7 +108,7 @@ struct FusedArgs {
   const int32_t* cu;
   int32_t total, n_ptiles;
   KbFastDiv fd_tiles, fd_H, fd_Hk, fd_group, fd_c;  // division by ceil(T / 128), H, Hk, group and c
-  int32_t item_rot;  // main kernel, see KbItemWalk
+  int32_t n_fixed;  // > 0: the main kernel's CTAs take the items in turn (see ItemWriter)
   float scale_log2, sm_scale;
   int32_t* status;
 };
@@ -137,6 +138,7 @@ struct alignas(1024) FusedSmem {
   alignas(16) float delta_s[2][kBQ];  // -delta
   uint64_t k_full[2], k_free[2], v_full, v_empty, q_full[2], q_empty[2], do_full, do_empty;
   uint64_t s_ready, p_ready, dp_ready, ds_ready[2], ds_free, stats_full[2], dv_done, dk_done, dv_free, dk_free;
+  ItemQueue items;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -149,7 +151,7 @@ enum WaitSite {
 constexpr int kErrSmemAlign = 71;
 
 // One work item of the main kernel and the position of a tile in the CTA's tile sequence.  Every
-// role walks the same sequence with its own cursor: `n` counts the live items so far, `g` the tiles
+// role walks the same sequence with its own cursor (ITEMS: where it takes the items from, item_queue.cuh): `n` counts the live items so far, `g` the tiles
 // so far; barrier phases are derived from them.
 struct Item {
   int b, hk, kt, k0, len;  // hk: key/value head
@@ -158,8 +160,9 @@ struct Item {
 };
 // The tiles of an item: for every query head of the key/value head's group (hq = 0 .. group - 1), the
 // query tiles of `qr` (tq = 0 ..); t is the running index over both.
+template <typename ITEMS>
 struct Cursor {
-  KbItemWalk walk;
+  ITEMS items;
   int n, g, t, tq, hq, group;
   Item it;
   bool valid;
@@ -197,37 +200,36 @@ __device__ __forceinline__ Item decode_item(const FusedArgs& a, int item, int n_
 // row0 and is b-th in the batch; floor(row0 / 128) + b + kt is unique per (b, kt) and below
 // floor(total / 128) + B + 1 (a sequence ends at most one tile later than its rows alone would need).
 __device__ __forceinline__ int ptile_id(int row0, int b, int kt) { return (row0 >> 7) + b + kt; }
-// first live item from the walk's position on
-template <bool PACKED>
-__device__ __forceinline__ void seek_live(const FusedArgs& a, Cursor& c, int n_items, int n_ktiles) {
-  c.valid = false;
-  for (; c.walk.item() < n_items; c.walk.next()) {
-    c.it = decode_item<PACKED>(a, c.walk.item(), n_ktiles);
-    if (c.it.qr.begin < c.it.qr.end) {
-      c.valid = true;
-      return;
-    }
-  }
+template <bool PACKED, typename ITEMS>
+__device__ __forceinline__ void cursor_open(const FusedArgs& a, Cursor<ITEMS>& c, int n_ktiles) {
+  c.valid = c.items.item() >= 0;
+  if (c.valid) c.it = decode_item<PACKED>(a, c.items.item(), n_ktiles);
 }
-template <bool PACKED>
-__device__ __forceinline__ Cursor cursor_first(const FusedArgs& a, int n_items, int n_ktiles) {
-  Cursor c{KbItemWalk(a.item_rot)};  // (everything after the walk starts as zero)
+template <bool PACKED, typename ITEMS>
+__device__ __forceinline__ Cursor<ITEMS> cursor_first(const FusedArgs& a, const ITEMS& items, int n_ktiles) {
+  Cursor<ITEMS> c{items};  // (everything after the items starts as zero)
   c.group = a.group;
-  seek_live<PACKED>(a, c, n_items, n_ktiles);
+  cursor_open<PACKED>(a, c, n_ktiles);
   return c;
 }
-template <bool PACKED>
-__device__ __forceinline__ void cursor_next(const FusedArgs& a, Cursor& c, int n_items, int n_ktiles) {
+// the next tile of the item; false after the last one
+template <typename ITEMS>
+__device__ __forceinline__ bool cursor_next_tile(Cursor<ITEMS>& c) {
   ++c.g;
   ++c.t;
-  if (++c.tq < c.q_tiles()) return;
+  if (++c.tq < c.q_tiles()) return true;
   c.tq = 0;
-  if (++c.hq < c.group) return;
+  if (++c.hq < c.group) return true;
   c.hq = 0;
   c.t = 0;
   ++c.n;
-  c.walk.next();
-  seek_live<PACKED>(a, c, n_items, n_ktiles);
+  return false;
+}
+template <bool PACKED, typename ITEMS>
+__device__ __forceinline__ void cursor_next(const FusedArgs& a, Cursor<ITEMS>& c, int n_ktiles, const WaitCtx& ctx) {
+  if (cursor_next_tile(c)) return;
+  c.items.next(ctx);
+  cursor_open<PACKED>(a, c, n_ktiles);
 }
 // `h` is the QUERY head, `row0` the sequence's first row (packed batch only)
 template <bool PACKED>
@@ -253,7 +255,6 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = a.T;
   const int n_ktiles = kb_cdiv_i32(T, kBK);
-  const int n_items = a.B * a.Hk * n_ktiles;
 
   if (smem_u32(smem_raw) & 1023u) {
     // swizzled operand tiles need a 1024-byte aligned base: report instead of computing garbage
@@ -285,6 +286,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     mbar_init(&sm.dk_done, 1);
     mbar_init(&sm.dv_free, kEpiThreads);
     mbar_init(&sm.dk_free, kEpiThreads);
+    item_queue_init(sm.items, 3 + kComputeThreads / 32 + kEpiThreads / 32);  // stats, MMA, copy-out; compute; epilogue
     sm.abort_flag = 0;
     fence_mbar_init();
   }
@@ -314,13 +316,27 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         prefetch_tensormap(&tm_do);
       }
       bool ok = true;
-      for (Cursor c = cursor_first<PACKED>(a, n_items, n_ktiles); ok && c.valid; cursor_next<PACKED>(a, c, n_items, n_ktiles)) {
-        const int g = c.g, n = c.n;
-        const int q0 = c.q0(), hq = c.head();
-        if (lane == 0) {
+      auto c = cursor_first<PACKED>(a, ItemWriter(sm.items, a.n_fixed), n_ktiles);
+      for (; c.valid; c.items.next(ok, ctx), cursor_open<PACKED>(a, c, n_ktiles)) {
+        if (c.it.qr.begin >= c.it.qr.end) {
+          // the whole key tile lies in the padding: its gradients are zeros.  A packed batch has no padding rows.
+          if (!PACKED) {
+            const int64_t off = c.it.b * a.dkv_sb + c.it.hk * a.dkv_sh + c.it.k0 * a.dkv_st;  // one head per key/value head
+            const int rows = kb_min_i32(kBK, T - c.it.k0);
+            warp_clear_rows<D * 2>(static_cast<uint16_t*>(a.dv) + off, a.dkv_st * 2, rows);
+            warp_clear_rows<D * 2>(static_cast<uint16_t*>(a.dk) + off, a.dkv_st * 2, rows);
+          }
+          continue;
+        }
+        if (lane != 0) continue;
+        ok = c.items.publish(make_int4(c.items.item(), c.tiles(), 0, 0), ctx);
+        do {
+          const int g = c.g, n = c.n;
+          const int q0 = c.q0(), hq = c.head();
+          if (c.last()) c.items.ask();
           KB_FTR(0, g, 0);
           // order of issue = order of need: S wants K and Q, dP (issued a tile later) wants V and dO
-          if (c.t == 0) {
+          if (ok && c.t == 0) {
             // K and V are read by this CTA only and come from DRAM.  The long-item class asks for the opening item's tiles in
             // L2 at once; V and the second half of K are loaded behind waits.  1 669 us against 1 720 without (bf16 c=256
             // T=16384), packed c=256 1 793 / 1 800.  The other classes lose by it: fp16 D=64 c=10 379 us with, 359 without,
@@ -367,15 +383,16 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
               tma_load_4d(sm.d_o + p * kPanelBytes, &tm_do, &sm.do_full, p * 64, c.it.row0 + q0, hq, PACKED ? 0 : c.it.b);
           }
           KB_FTR(0, g, 2);
-        }
+        } while (cursor_next_tile(c) && ok);
       }
+      if (lane == 0) c.items.finish(ctx);
     } else if (warp == kStatsWarp) {
       // ------------------------------ lse / delta staging ------------------------------
       // lse and delta of the tile's query rows, two slots deep: slot g & 1 was last read while dS(g - 2) was
       // formed.  The P phase of tile g needs them the moment S(g) completes.  The loop is kept short: two 64-bit
       // multiplies per element in it cost the kernel 15 %.
       bool ok = true;
-      for (Cursor c = cursor_first<PACKED>(a, n_items, n_ktiles); ok && c.valid; cursor_next<PACKED>(a, c, n_items, n_ktiles)) {
+      for (auto c = cursor_first<PACKED>(a, ItemReader<true>(sm.items, ctx), n_ktiles); ok && c.valid; cursor_next<PACKED>(a, c, n_ktiles, ctx)) {
         const int g = c.g;
         const int q0 = c.q0(), hq = c.head();
         if (g >= 2) ok = mbar_wait<kRelaxedNs>(&sm.ds_ready[g & 1], ((g >> 1) - 1) & 1, ctx, kWStatsSlot);
@@ -450,18 +467,12 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             mma_ts_lo(tmem + acc_col, a + 8 * i, b_lo + i * (2048 >> 4), idesc_acc, !first_tile || p > 0 || i > 0);
         }
       };
-      // This thread keeps no cursor: all it needs of the schedule is how many tiles each live item has.
-      // Tiles of the first live item from the walk's position on, 0 if there is none.
-      auto next_live = [&](KbItemWalk& walk) -> int {
-        for (; walk.item() < n_items; walk.next()) {
-          const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles);
-          if (it.qr.begin < it.qr.end) return (it.qr.end - it.qr.begin) * a.group;
-        }
-        return 0;
-      };
+      // This thread keeps no cursor: all it needs of the schedule is how many tiles each item has.
+      // Tiles of the current item, 0 if there is none.
+      ItemReader<false> items(sm.items, ctx);
+      auto item_tiles = [&]() -> int { return items.item() < 0 ? 0 : items.e.y; };
 
-      KbItemWalk walk(a.item_rot);
-      int cnt = next_live(walk);  // tiles of the current item
+      int cnt = item_tiles();  // tiles of the current item
       int n = 0, g = 0;           // live items, tiles so far
       bool ok = cnt > 0 && issue_s(0, 0, true) && issue_dp(0, 0, true, cnt == 1);
       KB_ACC(11);
@@ -490,8 +501,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           // S(g+1): of this item, or the first of the next live one.  (Looking for the next item before the wait for
           // P instead, off the chain, as the other classes' loop below does, measured 1 % slower in this one.)
           if (last) {
-            walk.next();
-            cnt_next = next_live(walk);
+            items.next(ctx);
+            cnt_next = item_tiles();
           }
           const bool more = !last || cnt_next > 0;
           if (more && !issue_s(last ? n + 1 : n, g + 1, last)) return false;
@@ -538,8 +549,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             // The look for the next live item (a decode per candidate) is done here, before the wait for P: from
             // that wait to the issue of S(g+1) the thread is on the kernel's critical chain.
             if (last) {
-              walk.next();
-              cnt_next = next_live(walk);
+              items.next(ctx);
+              cnt_next = item_tiles();
             }
             const bool more = !last || cnt_next > 0;
             const int n_next = last ? n + 1 : n;                           // item of tile g + 1
@@ -590,7 +601,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 #endif
     } else if (warp == kSpillWarp && lane == 0) {
       // ------------------------------ dS tiles to the scratch buffer ------------------------------
-      for (Cursor c = cursor_first<PACKED>(a, n_items, n_ktiles); c.valid; cursor_next<PACKED>(a, c, n_items, n_ktiles)) {
+      for (auto c = cursor_first<PACKED>(a, ItemReader<false>(sm.items, ctx), n_ktiles); c.valid; cursor_next<PACKED>(a, c, n_ktiles, ctx)) {
         if (!mbar_wait<kRelaxedNs>(&sm.ds_ready[c.g & 1], (c.g >> 1) & 1, ctx, kWSpill)) break;
         bulk_store(ds_slot<PACKED>(a, c.it.b, c.it.row0, c.head(), c.it.kt, n_ktiles, c.tq), sm.ds, kDsTileBytes);
         tma_store_commit();
@@ -614,7 +625,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint64_t scale2 = f2_pack(a.scale_log2, a.scale_log2);
     int lo = 0, hi = 0;  // live query columns of this key row: [lo, hi)
     bool ok = true;
-    for (Cursor c = cursor_first<PACKED>(a, n_items, n_ktiles); ok && c.valid; cursor_next<PACKED>(a, c, n_items, n_ktiles)) {
+    for (auto c = cursor_first<PACKED>(a, ItemReader<true>(sm.items, ctx), n_ktiles); ok && c.valid; cursor_next<PACKED>(a, c, n_ktiles, ctx)) {
       const int g = c.g;
       if (c.t == 0) {
         const int xi = c.it.k0 + row;
@@ -735,24 +746,9 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     int n = 0;
     bool ok = true;
-    for (KbItemWalk walk(a.item_rot); ok && walk.item() < n_items; walk.next()) {
-      const Item it = decode_item<PACKED>(a, walk.item(), n_ktiles);
+    for (ItemReader<true> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
+      const Item it = decode_item<PACKED>(a, items.item(), n_ktiles);
       const int kr = it.k0 + row;
-      if (it.qr.begin >= it.qr.end) {
-        // the whole key tile lies in the padding: its gradients are zeros (rare; plain stores).  A packed
-        // batch has no padding rows: a tile past the sequence's end owns nothing.
-        if (!PACKED && kr < T) {
-          const int64_t off = it.b * a.dkv_sb + it.hk * a.dkv_sh + kr * a.dkv_st;  // one head per key/value head
-          uint4* dv_row = reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.dv) + off);
-          uint4* dk_row = reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.dk) + off);
-#pragma unroll
-          for (int i = 0; i < D * 2 / 16; ++i) {
-            dv_row[i] = make_uint4(0, 0, 0, 0);
-            dk_row[i] = make_uint4(0, 0, 0, 0);
-          }
-        }
-        continue;
-      }
       uint8_t* stage = sm.k[n & 1];
       // Packed batch, last key tile of a sequence: the rows below it belong to the next sequence, so the tile
       // cannot leave as a box store; every thread writes its own row (one such tile per sequence and head).
@@ -1114,7 +1110,6 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   int dev = 0, n_sm = 0;
   if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
   const int64_t n_items_main = (int64_t)p.B * Hk * n_tiles;
-  const unsigned grid_main = (unsigned)(n_items_main < n_sm ? n_items_main : n_sm);
 
   // the class of long items of fully live tiles gets the main kernel with the second copy of the issue sequence
   const bool mid = D == 128 && c >= 128;
@@ -1184,8 +1179,14 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.fd_c = kb_fastdiv_make(c);
   fa.scale_log2 = p.sm_scale * kLog2e;
   fa.sm_scale = p.sm_scale;
-  const int32_t most_places = c % (2 * kBK) ? 4 : mid && !PACKED ? 1 : 2;  // see kb_item_rotation
-  fa.item_rot = kb_item_rotation((int32_t)grid_main, n_tiles, p.lens || PACKED, most_places);
+  // Where every sequence is as long and chunks are whole pairs of key tiles, CTAs 2 m and 2 m + 1 of the fixed order always
+  // work on the two key tiles of one chunk, which stream the same Q / dO tiles.  Fixed / taken as CTAs become free, us, bf16
+  // D=128: c=256 T=16384 1567 / 1650, T=8192 577 / 604, T=2048 542 / 563, T=1000 518 / 508; c=512 T=2048 842 / 861, T=1000
+  // 585 / 623, T=600 538 / 506.  Elsewhere the second: c=64 T=8192 290 / 254, c=128 420 / 382, c=200 T=1000 620 / 551,
+  // c=300 T=2048 787 / 742, fp16 D=64 c=256 T=1000 472 / 415; with lengths c=256 too (T=2048, in the fixed order 656 / 566).
+  const bool fixed = D == 128 && c % (2 * kBK) == 0 && !p.lens && !PACKED;
+  fa.n_fixed = fixed ? (int32_t)n_items_main : 0;
+  const unsigned grid_main = (unsigned)(fixed && n_items_main > n_sm ? n_sm : n_items_main);
   fa.status = p.status;
   if (!(p.flags & KB_FLAG_BWD_SKIP_DKDV)) {
     main_kern<<<grid_main, kThreads, sizeof(FusedSmem<D>), s>>>(tm_k, tm_v, tm_q, tm_do, tm_dk, tm_dv, fa);

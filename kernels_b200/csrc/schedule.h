@@ -86,53 +86,6 @@ KB_HD int32_t kb_fastdiv(int32_t n, const KbFastDiv& f) {
   return (int32_t)((hi + (uint32_t)n) >> f.shift);
 }
 
-// The order in which the CTAs of the main backward kernel take the work items (the others take them as they become free,
-// item_queue.cuh).  Wave w hands out the items
-// [w G, (w + 1) G) (G = CTAs): neighbouring items run at the same time and share their K / V rows in L2.  Inside a
-// wave CTA x takes number (x + w r) mod G.  An item's place in its sequence is item mod n (n = items per sequence and
-// head); with r = 0 a CTA meets only n / gcd(G, n) of the places.  Where sequences differ in length the late places are
-// often padding, and with few places per CTA some CTAs get much more work than others (n = 4, G = 148: CTA 0 only the
-// first quarter of every sequence).  r > 0 makes G + r and n coprime, which spreads the places.
-//
-// Only where the lengths differ and a CTA would meet at most `most_places` places (1 to 4).  Measured (B200, r = 0 / r = 1):
-// packed batch of 256 sequences of 128-1024 rows 1286 / 1081 us.  With eight and more places nothing is gained, and
-// an odd r can cost: bf16 D=128 c=256 T=16384: 1680 us with even r, 1890-1980 with odd r (with an even one
-// CTAs 2 m and 2 m + 1 always have the two key tiles of one chunk, which stream the same Q / dO tiles).
-//
-// Chunks that are whole pairs of key tiles (c a multiple of 256) are therefore shifted only where a
-// CTA meets fewer places than four.  r = 0 / shifted, us, bf16 D=128, by the places met: padded, lengths T/2 to T: one (T=512)
-// 782 / 818; two (T=1024) 909 / 977, four (T=2048) 954 / 1035; c=512 T=768 (three) 928 / 1006.  Packed, T/8 to T:
-// one 1390 / 1145, two 1369 / 1340, four 1400 / 1470.  fp16 D=64 c=256, padded: one 334 / 289, two 409 / 385, four 451 /
-// 464.  Hence at most two, at most one for the padded head-dim-128 class.  (Other chunk lengths gain everywhere, but for
-// c=160 and 192 at T=512: 784 / 834.)
-inline int32_t kb_gcd(int32_t a, int32_t b) {
-  while (b) {
-    const int32_t t = a % b;
-    a = b;
-    b = t;
-  }
-  return a;
-}
-inline int32_t kb_item_rotation(int32_t ctas, int32_t items_per_seq, bool ragged, int32_t most_places = 4) {
-  const int32_t n = items_per_seq;
-  if (!ragged || ctas < 1 || n < 1 || n / kb_gcd(ctas, n) > most_places) return 0;
-  int32_t r = 0;
-  while (kb_gcd(ctas + r, n) != 1) ++r;  // among n consecutive numbers one is coprime to n
-  return r % ctas;
-}
-#if defined(__CUDACC__)
-struct KbItemWalk {
-  int32_t base, off, rot;
-  __device__ __forceinline__ explicit KbItemWalk(int32_t rotation) : base(0), off((int32_t)blockIdx.x), rot(rotation) {}
-  __device__ __forceinline__ int32_t item() const { return base + off; }  // the walk ends at the first item() >= n_items
-  __device__ __forceinline__ void next() {
-    base += (int32_t)gridDim.x;
-    off += rot;
-    if (off >= (int32_t)gridDim.x) off -= (int32_t)gridDim.x;
-  }
-};
-#endif
-
 // The two tile ranges above with the divisions by the chunk length done by kb_fastdiv (same
 // results; the persistent kernels call these).
 KB_HD KbTileRange kb_fwd_kv_range_fd(int32_t q0, int32_t tile_q, int32_t tile_k, int32_t len, int32_t c,
