@@ -8,8 +8,8 @@
 // One warp of the CTA, the TMA producer's, asks (ItemWriter).  It clears the outputs of items that lie wholly in the
 // padding itself and passes the live ones to the other roles through a ring of kItemSlots numbers in shared memory
 // (ItemReader).  (Padded items do not go through the ring: a role may look for the next live item before the current one
-// is complete, and would wait for ever behind a run of padded ones that fills the ring.)  It asks when it starts on the
-// last tiles of an item: the answer takes 350 clocks, and an item claimed earlier would wait at a CTA that is still busy.
+// is complete, and would wait for ever behind a run of padded ones that fills the ring.)  It asks when it has
+// issued the loads of an item's last tiles: the answer takes 350 clocks, and an item claimed earlier would wait at a CTA that is still busy.
 // Or (n_fixed) it takes the items in turn with the grid's other CTAs; sa_bwd_fused_sm100.cu says where that is better.
 #pragma once
 #include "sm100_ptx.cuh"
@@ -36,7 +36,6 @@ __device__ __forceinline__ void item_queue_init(ItemQueue& q, int readers) {
 }
 
 __device__ __forceinline__ void item_ask(ItemQueue* q) {
-  fence_proxy_async();  // the last answer was read through the generic proxy
   mbar_expect_tx(&q->answered, 16);
   asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
                    smem_u32(q->answer)),
@@ -55,6 +54,7 @@ __device__ __forceinline__ int item_answer(const ItemQueue* q) {
       : "=r"(got), "=&r"(x)
       : "r"(smem_u32(q->answer))
       : "memory");
+  fence_proxy_async();  // (the next answer is written through the async proxy)
   return got ? (int)x : -1;
 }
 // After a wait of the CTA gave up: the blocks not launched yet are taken over and dropped, so that the kernel ends with

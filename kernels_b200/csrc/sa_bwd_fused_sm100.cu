@@ -333,7 +333,6 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         do {
           const int g = c.g, n = c.n;
           const int q0 = c.q0(), hq = c.head();
-          if (c.last()) c.items.ask();
           KB_FTR(0, g, 0);
           // order of issue = order of need: S wants K and Q, dP (issued a tile later) wants V and dO
           if (ok && c.t == 0) {
@@ -383,6 +382,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
               tma_load_4d(sm.d_o + p * kPanelBytes, &tm_do, &sm.do_full, p * 64, c.it.row0 + q0, hq, PACKED ? 0 : c.it.b);
           }
           KB_FTR(0, g, 2);
+          if (c.t >= c.tiles() - 2) c.items.ask();
         } while (cursor_next_tile(c) && ok);
       }
       if (lane == 0) c.items.finish(ctx);
@@ -991,7 +991,6 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       ok = items.publish(make_int4(items.item(), it.kr.end - it.kr.begin, 0, 0), ctx);
       for (int j = it.kr.begin; ok && j < it.kr.end; ++j, ++u) {
         const int s = u % kDqStages;
-        if (j == it.kr.end - 1) items.ask();
         if (u >= kDqStages && !mbar_wait<kRelaxedNs>(&sm.empty[s], ((u / kDqStages) - 1) & 1, ctx, kWDqEmpty)) { ok = false; break; }
         // the slot this query tile has in key tile j's list: both schedules name the same pairs
         const KbTileRange qr = kb_bwd_q_range_fd(j * kBK, kBQ, kBK, it.len, a.c, a.back, a.fd_c);
@@ -1000,6 +999,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 #pragma unroll
         for (int p = 0; p < kPanels; ++p)
           tma_load_4d(sm.k[s] + p * kPanelBytes, &tm_k, &sm.full[s], p * 64, it.row0 + j * kBK, kb_fastdiv(it.h, a.fd_group), PACKED ? 0 : it.b);
+        if (j >= it.kr.end - 2) items.ask();
       }
     }
     if (lane == 0) items.finish(ctx);

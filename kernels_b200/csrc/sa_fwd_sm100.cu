@@ -151,6 +151,21 @@ __device__ __forceinline__ void max_scores(uint32_t (&s)[32], int c, int lo, int
 template <bool MASKED>
 __device__ __forceinline__ float softmax_row_max(uint32_t t_s, uint32_t (&s)[32], int k0, int lo, int hi) {
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (!MASKED) {
+    // (without masks the registers have room for the whole row)
+    uint32_t u[3][32];
+    tmem_ld32(t_s, s);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) tmem_ld32(t_s + 32 + 32 * i, u[i]);
+    scores_arrived(s);
+    max_scores<false>(s, 0, 0, 0, mx);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      scores_arrived(u[i]);
+      max_scores<false>(u[i], 0, 0, 0, mx);
+    }
+    return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+  }
   tmem_ld32(t_s, s);
   scores_arrived(s);
 #pragma unroll 1
@@ -352,7 +367,6 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int t = it.u_begin; ok && t < it.u_end; ++t, ++kc, ++vc) {
         const int sk = kc % kStagesK, sv = vc % kStagesV;
         const int k0 = t * kBN;
-        if (t == kb_max_i32(it.u_begin, it.u_end - 2)) items.ask();
         if (kc >= kStagesK && !mbar_wait(&sm.k_empty[sk], ((kc / kStagesK) - 1) & 1, ctx, kWaitKEmpty)) { ok = false; break; }
         mbar_expect_tx(&sm.k_full[sk], kTileBytes);
 #pragma unroll
@@ -363,6 +377,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         mbar_expect_tx(&sm.v_full[sv], kTileBytes);
 #pragma unroll
         for (int p = 0; p < kPanels; ++p) tma_load_4d(sm.v[sv] + p * kPanelBytes, &tm_v, &sm.v_full[sv], p * kPanelElems, it.row0 + k0, h_kv, PACKED ? 0 : it.b);
+        if (t == kb_max_i32(it.u_begin, it.u_end - 2)) items.ask();
       }
     }
     if (lane == 0) items.finish(ctx);
