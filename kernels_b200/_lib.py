@@ -207,11 +207,19 @@ except AttributeError:
 try:
     _tracing_state, _dispatch_modes = torch._C._get_tracing_state, torch._C._len_torch_dispatch_stack
     _function_modes, _transforms_active = torch._C._len_torch_function_stack, torch._C._are_functorch_transforms_active
+    _has_storage = torch._C._has_storage  # (batched gradients come as tensors without one; no transform announces them)
     _saved_tensor_hooks, _forward_ad = torch._C._autograd._top_saved_tensors_default_hooks, torch.autograd.forward_ad
     _forward_ad._current_level
     _can_tell_plain = True
 except AttributeError:
     _can_tell_plain = False
+
+
+def stream_handle(device: torch.device) -> int:
+    """The handle of the device's current stream."""
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def launch(entry, params, device: torch.device) -> int:
@@ -228,11 +236,11 @@ def launch(entry, params, device: torch.device) -> int:
 def plain_call(*tensors) -> bool:
     """Whether a call on these tensors is ordinary eager execution on a GPU: nothing traces, transforms or intercepts
     it (compilation, jit tracing, functorch transforms, forward-mode AD, saved-tensor hooks, dispatch or function modes, tensor
-    subclasses).  Entry points that have a shorter way for such calls ask this and leave everything else as it is."""
+    subclasses, tensors without storage).  Entry points that have a shorter way for such calls ask this and leave everything else as it is."""
     return (
         not torch.compiler.is_compiling()
         and _can_tell_plain
-        and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda for t in tensors)
+        and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and _has_storage(t) for t in tensors)
         and _tracing_state() is None
         and _dispatch_modes() == 0 and _function_modes() == 0
         and not _transforms_active() and _forward_ad._current_level < 0

@@ -111,20 +111,7 @@ def _clamp_i32(x: int) -> int:
     return int(min(max(int(x), -(2**31)), 2**31 - 1))
 
 
-@torch.library.custom_op("alexdremov_streaming_attention::forward", mutates_args=(), device_types=("cuda",))
-def attention_forward_adapter(
-    q: torch.Tensor,
-    k: torch.Tensor,
-    v: torch.Tensor,
-    lens: Optional[torch.Tensor],
-    context_size: int,
-    back_contexts: int,
-    sm_scale: float,
-    autotune: bool,
-    return_lse: bool,
-    prescale_qk: bool,
-    precision: str,
-) -> tuple[torch.Tensor, torch.Tensor]:
+def _forward(q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision):
     """Forward op body: allocate ``O`` (and ``LSE``) and launch ``kb_sa_fwd``.
 
     ``autotune`` is accepted and ignored: tile shapes come from the committed sm_100a table
@@ -164,6 +151,23 @@ def attention_forward_adapter(
     return O, LSE
 
 
+@torch.library.custom_op("alexdremov_streaming_attention::forward", mutates_args=(), device_types=("cuda",))
+def attention_forward_adapter(
+    q: torch.Tensor,
+    k: torch.Tensor,
+    v: torch.Tensor,
+    lens: Optional[torch.Tensor],
+    context_size: int,
+    back_contexts: int,
+    sm_scale: float,
+    autotune: bool,
+    return_lse: bool,
+    prescale_qk: bool,
+    precision: str,
+) -> tuple[torch.Tensor, torch.Tensor]:
+    return _forward(q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision)
+
+
 @torch.library.register_fake("alexdremov_streaming_attention::forward")
 def attention_forward_adapter_abstract(
     q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision
@@ -173,22 +177,7 @@ def attention_forward_adapter_abstract(
     return out, lse
 
 
-@torch.library.custom_op("alexdremov_streaming_attention::backward", mutates_args=(), device_types=("cuda",))
-def attention_backward_adapter(
-    q: torch.Tensor,
-    k: torch.Tensor,
-    v: torch.Tensor,
-    lens: Optional[torch.Tensor],
-    o: torch.Tensor,
-    lse: torch.Tensor,
-    do: torch.Tensor,
-    context_size: int,
-    back_contexts: int,
-    sm_scale: float,
-    autotune: bool,
-    prescale_qk: bool,
-    precision: str,
-) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+def _gradients(q, k, v, lens, o, lse, do, context_size, back_contexts, sm_scale, autotune, prescale_qk, precision):
     """Backward op body: ``(dQ, dK, dV)`` through ``kb_sa_bwd``.
 
     Scratch is allocated here and handed to the library: ``delta = rowsum(O * dO)`` as
@@ -209,7 +198,7 @@ def attention_backward_adapter(
     if lse.numel() == 0 and q.numel() != 0:
         # The forward was called directly with return_lse=False although a gradient is wanted
         # (the public wrapper never does that): rebuild the log-sum-exp with one more forward.
-        _, lse = attention_forward_adapter(
+        _, lse = _forward(
             q.detach(), k.detach(), v.detach(), lens, context_size, back_contexts, sm_scale, autotune, True,
             prescale_qk, precision)
     if lse.dtype != torch.float32 or not lse.is_contiguous():
@@ -227,7 +216,7 @@ def attention_backward_adapter(
         workspace_bytes = lib.kb_sa_bwd_generic_workspace_bytes if q.dtype == torch.float32 else lib.kb_sa_bwd_workspace_bytes
         ws_bytes = int(workspace_bytes(
             B, H, T, D, _lib.dtype_code(q.dtype), _clamp_i32(context_size), _clamp_i32(back_contexts)))
-        ds_ws = _ds_scratch_for(q.device, torch.cuda.current_stream(q.device).cuda_stream, ws_bytes, q.dtype)
+        ds_ws = _ds_scratch_for(q.device, _lib.stream_handle(q.device), ws_bytes, q.dtype)
     lens_keep, lens_ptr, lens_stride = _lens_arg(lens, q.device)
     p = _lib.SaBwdParams()
     p.q, p.k, p.v, p.o, p.d_o = (_lib.tensor4(t) for t in (q, k, v, o, do))
@@ -260,6 +249,25 @@ def attention_backward_adapter(
     _lib.check(rc, "kb_sa_bwd")
     del lens_keep
     return DQ, DK, DV
+
+
+@torch.library.custom_op("alexdremov_streaming_attention::backward", mutates_args=(), device_types=("cuda",))
+def attention_backward_adapter(
+    q: torch.Tensor,
+    k: torch.Tensor,
+    v: torch.Tensor,
+    lens: Optional[torch.Tensor],
+    o: torch.Tensor,
+    lse: torch.Tensor,
+    do: torch.Tensor,
+    context_size: int,
+    back_contexts: int,
+    sm_scale: float,
+    autotune: bool,
+    prescale_qk: bool,
+    precision: str,
+) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    return _gradients(q, k, v, lens, o, lse, do, context_size, back_contexts, sm_scale, autotune, prescale_qk, precision)
 
 
 @torch.library.register_fake("alexdremov_streaming_attention::backward")
@@ -335,7 +343,7 @@ def streaming_attention_reference(q, k, v, context_size, back_contexts, lens, sc
     return out, res_mask, sparsity_fraction
 
 
-def _streaming_attention_eager(
+def _streaming_attention_op(
     q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision
 ):
     requires_grad = any(t.requires_grad for t in (q, k, v))
@@ -350,7 +358,40 @@ def _streaming_attention_eager(
     return O
 
 
-_streaming_attention = torch.compile(_streaming_attention_eager, fullgraph=True, dynamic=True)
+class _StreamingAttention(torch.autograd.Function):
+    """The operators' bodies and their autograd wiring without the dispatcher, for ordinary eager calls."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, lens, context_size, back_contexts, sm_scale, autotune, prescale_qk, precision):
+        O, LSE = _forward(q, k, v, lens, context_size, back_contexts, sm_scale, autotune, True, prescale_qk, precision)
+        ctx.save_for_backward(q, k, v, O, LSE, lens)
+        ctx.args = (context_size, back_contexts, sm_scale, autotune, prescale_qk, precision)
+        return O, LSE
+
+    @staticmethod
+    def backward(ctx, do, dlse):  # (no gradient through LSE, as above)
+        q, k, v, o, lse, lens = ctx.saved_tensors
+        # A transform or a mode around the backward pass meets the operator, and so does a pass that is to be
+        # differentiated again: the operator has no gradient and says so.
+        gradients = torch.ops.alexdremov_streaming_attention.backward
+        if not torch.is_grad_enabled() and _lib.plain_call(do):
+            if not do.is_contiguous() and not _rows_in_place(do):
+                do = do.contiguous()  # see _backward
+            gradients = _gradients
+        return (*gradients(q, k, v, lens, o, lse, do, *ctx.args), None, None, None, None, None, None, None)
+
+
+def _streaming_attention_eager(
+    q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision
+):
+    if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
+        O, LSE = _StreamingAttention.apply(q, k, v, lens, context_size, back_contexts, sm_scale, autotune, prescale_qk, precision)
+    else:
+        O, LSE = _forward(q, k, v, lens, context_size, back_contexts, sm_scale, autotune, return_lse, prescale_qk, precision)
+    return (O, LSE) if return_lse else O
+
+
+_streaming_attention = torch.compile(_streaming_attention_op, fullgraph=True, dynamic=True)
 
 
 def streaming_attention(
@@ -387,10 +428,11 @@ def streaming_attention(
     (kernel.py:1599-1652).
     """
     # The compiled function is one operator call, so compiling it changes no result.  An ordinary call goes to the
-    # operator directly: guards, the compiled wrapper and its autograd function took 300 of the 500 us of host time of
-    # a forward + backward pass, more than the kernels of a small one.  Everything that looks inside (an outer
-    # compilation, transforms, hooks, modes) still meets the compiled function, and so do numbers that are not Python's
-    # own: it refuses numpy's and zero-dimensional tensors, which the operator alone would take.
+    # operator's body directly, through an autograd function of its own: of the 500 us of host time of a forward +
+    # backward pass guards, the compiled wrapper and its autograd function took 200, the dispatcher and the
+    # operators' own autograd wrappers 100 of the rest, where the kernels of a small one take 55.  Everything
+    # that looks inside (an outer compilation, transforms, hooks, modes) still meets the compiled function, and so do numbers
+    # that are not Python's own: it refuses numpy's and zero-dimensional tensors, which the body alone would take.
     numbers = type(context_size) in (int, bool) and type(back_contexts) in (int, bool) and type(sm_scale) in (type(None), int, float)
     if numbers and _lib.plain_call(q, k, v):
         attention = _streaming_attention_eager

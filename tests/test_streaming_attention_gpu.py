@@ -541,6 +541,41 @@ def test_numbers_that_are_not_pythons_own_are_refused():
     assert torch.equal(streaming_attention(q, k, v, None, 16, 2, sm_scale=1), streaming_attention(q, k, v, None, 16, 2, sm_scale=1.0))
 
 
+@pytest.mark.parametrize("dtype, D", [(torch.float32, 32), (torch.bfloat16, 64)], ids=str)
+def test_backward_of_ordinary_calls(dtype, D):
+    """Through the direct route: a second differentiation is refused, also where the output gradient needs none; batched
+    output gradients and a mode around the backward pass give the gradients of ordinary passes; no graph without need."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    q, k, v = (torch.randn(2, 2, 70, D, device="cuda", dtype=dtype).requires_grad_() for _ in range(3))
+    do = torch.randn(2, 2, 2, 70, D, device="cuda", dtype=dtype)
+
+    def grads(g, **kw):
+        return torch.autograd.grad(_api()(q, k, v, None, 16, 1), (q, k, v), g, **kw)
+
+    once = [grads(g) for g in do]
+    dq, _, _ = grads(do[0], create_graph=True)
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad((dq.float() * q.float()).sum(), q)
+    for got, a, b in zip(grads(do, is_grads_batched=True), *once):
+        assert torch.equal(got, torch.stack([a, b]))
+
+    seen = []
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    o = _api()(q, k, v, None, 16, 1)
+    with Mode():
+        moded = torch.autograd.grad(o, (q, k, v), do[0])
+    assert all(torch.equal(a, b) for a, b in zip(moded, once[0])) and any("alexdremov_streaming_attention.backward" in s for s in seen)
+    with torch.no_grad():
+        assert _api()(q, k, v, None, 16, 1).grad_fn is None
+    assert _api()(q.detach(), k.detach(), v.detach(), None, 16, 1).grad_fn is None
+
+
 def test_only_ordinary_calls_leave_the_compiled_function(monkeypatch):
     """Which of the two ways a call takes: transforms, forward-mode AD, jit tracing, modes, subclasses and saved-tensor
     hooks meet the compiled function; tensors, parameters, no_grad, inference mode, another stream and another thread
