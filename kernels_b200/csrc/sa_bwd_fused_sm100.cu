@@ -40,7 +40,7 @@
 // S, dP and P of the next one are under way.  Nothing but the lse / delta rows is moved by thread
 // loads or stores: such traffic shares the path the MMAs fetch their operands through and was
 // measured to slow them down severely.
-// Shared memory at D = 128: K 2 x 32 KB, V 32, Q 2 x 32, dO 32, dS 32 = 224 KB.  The K buffer of a
+// Shared memory at D = 128: K 2 x 32 KB, V 32, Q 2 x 32, dO 32, dS 32 = 224 KB (D = 64: a second dO buffer).  The K buffer of a
 // finished item stages its dV / dK on their way out before the K of the item after next lands in it.
 //
 // Reference semantics: src/streaming_attention/kernel.py:453-514 (delta), 639-773 and 941-1023
@@ -127,16 +127,22 @@ inline int32_t fused_slots(int32_t T, int32_t c, int32_t back) {
 // its rows alone would need.
 inline int32_t packed_tiles(int32_t total, int32_t B) { return total / kBK + B + 1; }
 
+// dO tiles in shared memory.  With one, dO(g + 1) sets out when dV(g) is complete and dP(g + 1) waits for it: 350 to 640
+// of a tile's 4 300 to 6 000 clocks.  Head dim 64 has room for two (one / two, us: fp16 c=10 T=1353 300 / 298, c=37 T=1000
+// 208 / 191, c=128 T=4096 206 / 204, c=200 T=3000 181 / 174, packed c=50 393 / 385); head dim 128 has none left.
+template <int D>
+constexpr int kDoStages = D == 64 ? 2 : 1;
+
 template <int D>
 struct alignas(1024) FusedSmem {
   uint8_t k[2][kBK * 128 * 2];  // 32 KB each whatever D is: they double as staging for dV / dK
   uint8_t v[kBK * D * 2];
   uint8_t q[2][kBQ * D * 2];
-  uint8_t d_o[kBQ * D * 2];
+  uint8_t d_o[kDoStages<D>][kBQ * D * 2];
   uint8_t ds[kDsTileBytes];  // rows = keys, 64 queries per 128-byte row, two panels
   alignas(16) float lse_s[2][kBQ];    // -lse
   alignas(16) float delta_s[2][kBQ];  // -delta
-  uint64_t k_full[2], k_free[2], v_full, v_empty, q_full[2], q_empty[2], do_full, do_empty;
+  uint64_t k_full[2], k_free[2], v_full, v_empty, q_full[2], q_empty[2], do_full[kDoStages<D>], do_empty[kDoStages<D>];
   uint64_t s_ready, p_ready, dp_ready, ds_ready[2], ds_free, stats_full[2], dv_done, dk_done, dv_free, dk_free;
   ItemQueue items;
   uint32_t tmem_base;
@@ -276,8 +282,10 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     }
     mbar_init(&sm.v_full, 1);
     mbar_init(&sm.v_empty, 1);
-    mbar_init(&sm.do_full, 1);
-    mbar_init(&sm.do_empty, 1);
+    for (int i = 0; i < kDoStages<D>; ++i) {
+      mbar_init(&sm.do_full[i], 1);
+      mbar_init(&sm.do_empty[i], 1);
+    }
     mbar_init(&sm.s_ready, 1);
     mbar_init(&sm.p_ready, kComputeThreads);
     mbar_init(&sm.dp_ready, 1);
@@ -374,12 +382,13 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 tma_load_4d(sm.v + p * kPanelBytes, &tm_v, &sm.v_full, p * 64, c.it.row0 + c.it.k0, c.it.hk, PACKED ? 0 : c.it.b);
             }
           }
-          if (ok && g >= 1) ok = mbar_wait<kRelaxedNs>(&sm.do_empty, (g - 1) & 1, ctx, kWDoEmpty);
+          const int ds = g % kDoStages<D>;
+          if (ok && g >= kDoStages<D>) ok = mbar_wait<kRelaxedNs>(&sm.do_empty[ds], ((g / kDoStages<D>) - 1) & 1, ctx, kWDoEmpty);
           if (ok) {
-            mbar_expect_tx(&sm.do_full, kTileBytes);
+            mbar_expect_tx(&sm.do_full[ds], kTileBytes);
 #pragma unroll
             for (int p = 0; p < kPanels; ++p)
-              tma_load_4d(sm.d_o + p * kPanelBytes, &tm_do, &sm.do_full, p * 64, c.it.row0 + q0, hq, PACKED ? 0 : c.it.b);
+              tma_load_4d(sm.d_o[ds] + p * kPanelBytes, &tm_do, &sm.do_full[ds], p * 64, c.it.row0 + q0, hq, PACKED ? 0 : c.it.b);
           }
           KB_FTR(0, g, 2);
           if (c.t >= c.tiles() - 2) c.items.ask();
@@ -413,7 +422,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t idesc_z = make_idesc(BF16, kBK, kBQ, false, false);  // S, dP
       constexpr uint32_t idesc_acc = make_idesc(BF16, kBK, D, false, true);   // dV, dK (A in TMEM)
-      const uint32_t v_addr = smem_u32(sm.v), do_addr = smem_u32(sm.d_o);
+      const uint32_t v_addr = smem_u32(sm.v);
 #ifdef KB_TRACE_FUSED
       long long acc_t[12] = {0};
       long long tl = clock64();
@@ -443,10 +452,10 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       // dP of tile g (item n) = V dO^T;  `last`: the tile closes its item
       auto issue_dp = [&](int n, int g, bool new_item, bool last) -> bool {
         if (new_item && !mbar_wait(&sm.v_full, n & 1, ctx, kWVFull)) return false;
-        if (!mbar_wait(&sm.do_full, g & 1, ctx, kWDoFull)) return false;
+        if (!mbar_wait(&sm.do_full[g % kDoStages<D>], (g / kDoStages<D>) & 1, ctx, kWDoFull)) return false;
         KB_ACC(10);  // waits for V, dO (counted apart from the issue of dP)
         tc_fence_after();
-        uint32_t v_lo = desc_lo_kmajor(v_addr), do_lo = desc_lo_kmajor(do_addr);
+        uint32_t v_lo = desc_lo_kmajor(v_addr), do_lo = desc_lo_kmajor(smem_u32(sm.d_o[g % kDoStages<D>]));
 #pragma unroll 1
         for (int p = 0; p < D / 64; ++p, v_lo += kPanelBytes >> 4, do_lo += kPanelBytes >> 4) {
 #pragma unroll
@@ -493,8 +502,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           KB_FTR(1, g, 1);
           KB_ACC(2);  // wait dv_free
           tc_fence_after();
-          issue_acc(kColDV, kColS, do_addr, first);
-          mma_commit(&sm.do_empty);
+          issue_acc(kColDV, kColS, smem_u32(sm.d_o[g % kDoStages<D>]), first);
+          mma_commit(&sm.do_empty[g % kDoStages<D>]);
           if (last) mma_commit(&sm.dv_done);  // the epilogue warps start on dV while dK(last) still runs
           KB_FTR(1, g, 2);
           KB_ACC(3);  // issue dV
@@ -565,8 +574,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             KB_FTR(1, g, 1);
             KB_ACC(2);  // wait dv_free
             tc_fence_after();
-            issue_acc(kColDV, kColS, do_addr, first);
-            mma_commit(&sm.do_empty);
+            issue_acc(kColDV, kColS, smem_u32(sm.d_o[g % kDoStages<D>]), first);
+            mma_commit(&sm.do_empty[g % kDoStages<D>]);
             if (last) mma_commit(&sm.dv_done);  // the epilogue warps start on dV while dK(last) still runs
             KB_FTR(1, g, 2);
             KB_ACC(3);  // issue dV
