@@ -419,6 +419,12 @@ KB_API int kb_sa_tile_config(int32_t dtype, int32_t D, int32_t context_size, uin
  * abort flag), and the abort flag (1 expected).  Read both after synchronising the stream.
  */
 KB_API int kb_selftest_wait_timeout(int32_t* status, int32_t* seen, void* stream);
+/*
+ * The same for warps that meet at barriers without a time limit: two of four see a wait give up, the other two find
+ * their item; all four have to leave.  `seen` (8 device-visible int32): the items each warp worked on (1 expected), and
+ * the last item each found (5, 5, 7, 7 expected).  `status` stays as it is.
+ */
+KB_API int kb_selftest_reader_group(int32_t* status, int32_t* seen, void* stream);
 
 /* number of kernels the library launched since it was loaded (all entry points) */
 KB_API int64_t kb_launch_count(void);

@@ -139,6 +139,27 @@ struct ItemReader {
   }
 };
 
+// Four warps that read the same items and meet at named barriers.  A wait that gives up does so in one warp: another
+// role has raised the abort flag, this warp's poll saw it, and a sibling's wait may still have succeeded.  A named barrier
+// has no time limit, so the four leave together or not at all: before the barriers of an item they agree that each of them
+// got there, and a warp that leaves its loop without that vote (no item for it: the end, or a wait that gave up) votes
+// against.  Every warp's last vote is therefore a no of one of them, or, at the end, of all.
+struct ReaderGroup {
+  static constexpr int kThreads = 128;
+  uint32_t barrier;
+  bool apart;  // the group has voted no
+  __device__ __forceinline__ explicit ReaderGroup(uint32_t named_barrier) : barrier(named_barrier), apart(false) {}
+  // Once per item, before its first named barrier: whether all four go on.
+  __device__ __forceinline__ bool agree(bool ok) {
+    apart = !named_barrier_and(barrier, kThreads, ok);
+    return !apart;
+  }
+  // After the loop over the items.
+  __device__ __forceinline__ void leave() {
+    if (!apart) named_barrier_and(barrier, kThreads, false);
+  }
+};
+
 // Zeros into `rows` rows of BYTES bytes (at most 512), `stride` bytes apart, by a whole warp.
 template <int BYTES>
 __device__ __forceinline__ void warp_clear_rows(void* first, int64_t stride, int rows) {

@@ -755,6 +755,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     int n = 0;
     bool ok = true;
+    ReaderGroup group(1);
     for (ItemReader<true> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
       const Item it = decode_item<PACKED>(a, items.item(), n_ktiles);
       const int kr = it.k0 + row;
@@ -768,7 +769,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         const float mul = which ? a.sm_scale : 1.f;
         // dV is complete after the item's last dV MMA (every S that reads the K buffer ran before it),
         // dK one matmul later.  All four warps must take the same exit: they meet at named barriers.
-        ok = named_barrier_and(1, kEpiThreads, mbar_wait<kRelaxedNs>(which ? &sm.dk_done : &sm.dv_done, n & 1, ctx, kWAccDone));
+        ok = group.agree(mbar_wait<kRelaxedNs>(which ? &sm.dk_done : &sm.dv_done, n & 1, ctx, kWAccDone));
         if (!ok) break;
         if (etid == 0) KB_FTR(3, n, which);
         tc_fence_after();
@@ -815,6 +816,7 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       if (!ok) break;
       ++n;
     }
+    group.leave();
     if (etid == 0) tma_store_wait_all();
   }
 
@@ -1042,6 +1044,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
     int m = 0;
     bool ok = true;
+    ReaderGroup group(1);
     for (ItemReader<true> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
       const DqItem it = decode_dq_item<PACKED>(a, items.item(), n_tiles_t);
       const int qi = it.qt * kBQ + row;
@@ -1049,7 +1052,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       // store; every thread writes its own row
       const bool partial = PACKED && it.qt * kBQ + kBQ > it.len;
       // all four warps must take the same exit: they meet at named barriers below
-      ok = named_barrier_and(1, 128, mbar_wait<kRelaxedNs>(&sm.acc_done[m & 1], (m >> 1) & 1, ctx, kWDqAccDone));
+      ok = group.agree(mbar_wait<kRelaxedNs>(&sm.acc_done[m & 1], (m >> 1) & 1, ctx, kWDqAccDone));
       if (!ok) break;
       tc_fence_after();
 #pragma unroll
@@ -1090,6 +1093,7 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
       named_barrier_sync(1, 128);  // the staging tile may be overwritten
       ++m;
     }
+    group.leave();
     if (threadIdx.x == 0) tma_store_wait_all();
   }
 

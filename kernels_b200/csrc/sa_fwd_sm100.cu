@@ -638,6 +638,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     long long acc_t[8] = {0};
     long long tl = clock64();
 #endif
+    ReaderGroup group(1 + x);
     for (ItemReader<true> items(sm.items, ctx); ok && items.item() >= 0; items.next(ctx)) {
       const Item it = decode(items.item());
       const int qi = it.q0 + x * kBM + row;
@@ -737,7 +738,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (!ok) break;
       KB_FACC(0);
 
-      ok = __all_sync(0xffffffffu, mbar_wait(&sm.o_done[x], live_items & 1, ctx, kWaitEpilogue));
+      if (row == 0) tma_store_wait_read();  // the store that used the staging buffer last has read it
+      ok = group.agree(mbar_wait(&sm.o_done[x], live_items & 1, ctx, kWaitEpilogue));
       if (!ok) break;
       KB_FACC(5);
       ++live_items;
@@ -775,8 +777,10 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       } else {
 #pragma unroll
       for (int p = 0; p < kOutPanels; ++p) {
-        if (row == 0) tma_store_wait_read();  // the store that used the buffer last has read it
-        named_barrier_sync(1 + x, kBM);
+        if (p > 0) {  // (the first panel's is at the wait for O)
+          if (row == 0) tma_store_wait_read();  // the store that used the buffer last has read it
+          named_barrier_sync(1 + x, kBM);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int e = p * 64 + 8 * j;
@@ -798,6 +802,7 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (qi < (PACKED ? it.len : T) && lse_row) *lse_row = valid ? m_used + log2f(l) : 0.f;
       KB_FACC(6);
     }
+    group.leave();
     if (row == 0) tma_store_wait_all();
 #ifdef KB_TRACE_FWD
     if (blockIdx.x == 60 && threadIdx.x == 0)

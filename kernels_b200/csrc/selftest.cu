@@ -9,7 +9,13 @@
 // a limit of 1 024 polls (well under a millisecond) instead of the kernels' 2^22.  Nothing faults and
 // nothing hangs: the wait runs out, the second warp sees the abort flag the first one raised, the kernel
 // returns and the context stays usable.
+//
+// kb_selftest_reader_group: the case in which only some of the warps that meet at named barriers see a wait give up.
+// Two of four reader warps wait for an item that has not been published when the abort flag goes up; the other two look
+// only after the first two have left, and find the item there.  All four must end their loops (ReaderGroup), so the
+// kernel returns.  Every spin in it is bounded.
 #include "common.cuh"
+#include "item_queue.cuh"
 #include "sm100_ptx.cuh"
 
 namespace kb {
@@ -45,6 +51,54 @@ __global__ void __launch_bounds__(64) wait_timeout_selftest_kernel(int32_t* stat
   if (threadIdx.x == 0) seen[2] = abort_flag;
 }
 
+// Warps 0-3 read, thread 128 writes.  seen[w]: the number of items warp w worked on; seen[4 + w]: the last item it found.
+__global__ void __launch_bounds__(160) reader_group_selftest_kernel(int32_t* status, int32_t* seen) {
+  __shared__ ItemQueue queue;
+  __shared__ int abort_flag, gone;
+  if (threadIdx.x == 0) {
+    item_queue_init(queue, 4);
+    abort_flag = gone = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const WaitCtx ctx{&abort_flag, status};
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto wait_for = [&](volatile int* word, int value) {  // (at most a few milliseconds)
+    for (int spins = 0; *word < value && spins < 10000; ++spins) __nanosleep(200);
+  };
+  if (warp == 4) {
+    if (lane == 0) {
+      ItemWriter items(queue, 1);  // (a fixed walk: nothing is asked of the hardware)
+      items.publish(make_int4(5, 0, 0, 0), ctx);
+      wait_for(&gone, 4);  // every warp has worked on item 5
+      *ctx.abort_flag = 1;
+      wait_for(&gone, 6);  // warps 0 and 1 have given up the wait for the next one
+      items.publish(make_int4(7, 0, 0, 0), ctx);
+      atomicAdd(&gone, 1);
+    }
+  } else {
+    ReaderGroup group(1);
+    int done = 0, found = -1;
+    bool ok = true;
+    for (ItemReader<true> items(queue, ctx); ok && items.item() >= 0; items.next(ctx)) {
+      found = items.item();
+      ok = group.agree(true);
+      if (!ok) break;
+      ++done;
+      named_barrier_sync(1, 128);
+      if (lane == 0) atomicAdd(&gone, 1);
+      if (warp >= 2) wait_for(&gone, 7);
+    }
+    if (warp < 2 && lane == 0) atomicAdd(&gone, 1);
+    group.leave();
+    if (lane == 0) {
+      seen[warp] = done;
+      seen[4 + warp] = found;
+    }
+  }
+  __syncthreads();
+}
+
 }  // namespace
 }  // namespace kb
 
@@ -52,5 +106,12 @@ extern "C" int kb_selftest_wait_timeout(int32_t* status, int32_t* seen, void* st
   if (!status || !seen) return KB_ERR_BAD_ARGUMENT;
   kb::wait_timeout_selftest_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(status, seen);
   KB_LAUNCH_CHECK("wait_timeout_selftest_kernel");
+  return KB_OK;
+}
+
+extern "C" int kb_selftest_reader_group(int32_t* status, int32_t* seen, void* stream) {
+  if (!status || !seen) return KB_ERR_BAD_ARGUMENT;
+  kb::reader_group_selftest_kernel<<<1, 160, 0, static_cast<cudaStream_t>(stream)>>>(status, seen);
+  KB_LAUNCH_CHECK("reader_group_selftest_kernel");
   return KB_OK;
 }

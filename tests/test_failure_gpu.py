@@ -42,6 +42,21 @@ def test_bounded_wait_gives_up_and_reports():
     _lib.check_device_status()
 
 
+def test_warps_that_share_barriers_leave_together():
+    """A wait gives up in two of four warps that meet at named barriers, the other two find their item: the kernel ends."""
+    lib = _lib.load()
+    dev = torch.device("cuda", 0)
+    status = _lib.status_words()
+    status.zero_()
+    seen = torch.full((8,), -1, dtype=torch.int32).pin_memory()
+    stream = torch.cuda.current_stream(dev)
+    _lib.check(lib.kb_selftest_reader_group(status.data_ptr(), seen.data_ptr(), stream.cuda_stream), "kb_selftest_reader_group")
+    stream.synchronize()
+    assert seen.tolist() == [1, 1, 1, 1, 5, 5, 7, 7]
+    assert status.tolist() == [0, 0, 0, 0]
+
+
 def test_selftest_rejects_null_pointers():
     lib = _lib.load()
     assert lib.kb_selftest_wait_timeout(None, None, None) == 1
+    assert lib.kb_selftest_reader_group(None, None, None) == 1
