@@ -148,10 +148,14 @@ __device__ __forceinline__ void max_scores(uint32_t (&s)[32], int c, int lo, int
   }
 }
 // Pass 1: the row maximum of the masked scores.  Leaves the first 32 columns in `s` for pass 2.
-template <bool MASKED>
+// LONG: the straight-line instance of 8-bit inputs.  Its matmuls take half the instructions, which leaves the instruction
+// cache room: pass 2 without masks is unrolled, and pass 1 loops (the whole row held beside a tile's scales spills).
+// B=2 H=32 T=8192 c=256, us: 204.9 as in the other instances, 206.5 with pass 1 as a loop, 202.2 with pass 2
+// unrolled, 200.9 with both; c=64 the other way round, 176 and, unrolled, 183.
+template <bool MASKED, bool LONG>
 __device__ __forceinline__ float softmax_row_max(uint32_t t_s, uint32_t (&s)[32], int k0, int lo, int hi) {
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  if (!MASKED) {
+  if (!MASKED && !LONG) {
     // (without masks the registers have room for the whole row)
     uint32_t u[3][32];
     tmem_ld32(t_s, s);
@@ -217,10 +221,10 @@ __device__ __forceinline__ void exp_scores(uint32_t t_p, uint32_t (&s)[32], uint
 }
 // Pass 2: P into TMEM over S (P of columns 32 j .. 32 j + 31 lands on columns 16 j .. 16 j + 15, whose scores are in
 // registers by then); the row sum goes into `sum`.
-template <bool BF16, bool MASKED, bool FP8>
+template <bool BF16, bool MASKED, bool FP8, bool LONG>
 __device__ __forceinline__ void softmax_exp(uint32_t t_s, uint32_t (&s)[32], uint64_t scale2, uint64_t negm2, int k0, int lo, int hi, SoftSum& sum) {
   constexpr int kPack = FP8 ? 4 : 2;
-#pragma unroll 1
+#pragma unroll (LONG && !MASKED ? 2 : 1)
   for (int c = 0; c < kBN; c += 64) {
     uint32_t u[32];
     tmem_ld32(t_s + c + 32, u);
@@ -691,8 +695,9 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         KB_FACC(1);
         const bool warp_full = __all_sync(0xffffffffu, lo <= k0 && k0 + kBN <= hi);
+        constexpr bool kLong = FP8 && FAST;
         uint32_t sc[32];
-        const float row_max = warp_full ? softmax_row_max<false>(t_s, sc, k0, lo, hi) : softmax_row_max<true>(t_s, sc, k0, lo, hi);
+        const float row_max = warp_full ? softmax_row_max<false, kLong>(t_s, sc, k0, lo, hi) : softmax_row_max<true, kLong>(t_s, sc, k0, lo, hi);
         const float m_new = fmaxf(m_used, row_max * scale);
         // lazy rescale: keep the old reference maximum unless the new one is larger by more than the threshold
         const bool need = m_new > m_used + (FP8 ? kRescaleThresholdFp8 : kRescaleThreshold);
@@ -709,8 +714,8 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint64_t scale2 = f2_pack(scale, scale), negm2 = f2_pack(-m_safe, -m_safe);
         SoftSum sum2;
         sum2.s01 = sum2.s23 = f2_pack(0.f, 0.f);
-        if (warp_full) softmax_exp<BF16, false, FP8>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
-        else softmax_exp<BF16, true, FP8>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
+        if (warp_full) softmax_exp<BF16, false, FP8, kLong>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
+        else softmax_exp<BF16, true, FP8, kLong>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
         float sum4[4];
         f2_unpack(sum2.s01, sum4[0], sum4[1]);
         f2_unpack(sum2.s23, sum4[2], sum4[3]);
