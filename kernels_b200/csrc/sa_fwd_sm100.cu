@@ -38,6 +38,8 @@
 // P cast to the input type before P V, LSE = m + log2(l)).
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include <type_traits>
 
@@ -236,13 +238,55 @@ __device__ __forceinline__ void softmax_exp(uint32_t t_s, uint32_t (&s)[32], uin
   }
 }
 
+// The same in one walk with the row's 128 scores held in registers (`dead`: groups of 32 columns that are masked for every
+// row of the warp).  Head dim 64, whose epilogue leaves the registers for it and whose softmax sets the pace: a second walk
+// through TMEM is time on the chain S -> softmax -> P V.  But it is straight code, with masks and without, which the
+// MMA warp loses its instructions to, and it costs an item more; `launch` says which calls take it.
+template <bool MASKED>
+__device__ __forceinline__ float softmax_row_max_held(uint32_t t_s, uint32_t (&s)[4][32], bool (&dead)[4], int k0, int lo, int hi) {
+  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) tmem_ld32(t_s + 32 * j, s[j]);
+  tmem_wait_ld();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    dead[j] = MASKED && !mask_scores(s[j], k0 + 32 * j, lo, hi);
+    if (!dead[j]) max_scores<false>(s[j], 0, 0, 0, mx);
+  }
+  return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+}
+template <bool BF16, bool MASKED>
+__device__ __forceinline__ float softmax_exp_held(uint32_t t_s, uint32_t (&s)[4][32], const bool (&dead)[4], float scale, float m) {
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t pk[16];
+    if (MASKED && dead[j]) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) pk[i] = 0u;
+    } else {
+      // scalar arithmetic: with 128 scores held, the register pairs of the packed form do not fit
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float p0 = ex2_approx(fmaf(__uint_as_float(s[j][2 * i]), scale, -m));
+        const float p1 = ex2_approx(fmaf(__uint_as_float(s[j][2 * i + 1]), scale, -m));
+        sum[(2 * i) & 3] += p0;
+        sum[(2 * i + 1) & 3] += p1;
+        pk[i] = pack16x2<BF16>(p0, p1);
+      }
+    }
+    tmem_st16(t_s + 16 * j, pk);
+  }
+  return (sum[0] + sum[1]) + (sum[2] + sum[3]);
+}
+
 // PACKED: one launch over a packed batch (FwdArgs::cu).  FP8: q, k, v are e4m3 with per-tile scales, both matmuls
 // run as kind::f8f6f4 (half the instructions), the output is 16-bit (BF16 selects which).
 // FAST: the instance for chunk lengths that are multiples of the work item's 256 rows, where the two q tiles of
 // every item lie in one chunk and walk the same key tiles: the MMA thread then runs such items through a
 // straight-line schedule (first / inner / last step written out, nothing worked out per step).  Other chunk
 // lengths are built without it (the extra code measured 1.5 % slower there; c a multiple of 256 without it 865 -> 906 us, dense D=64 368 -> 392).
-template <int D, bool BF16, bool PACKED, bool FP8, bool FAST>
+template <int D, bool BF16, bool PACKED, bool FP8, bool FAST, bool HELD>
 __global__ void __launch_bounds__(kThreads, 1)
 sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdArgs a) {
@@ -696,8 +740,11 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         KB_FACC(1);
         const bool warp_full = __all_sync(0xffffffffu, lo <= k0 && k0 + kBN <= hi);
         constexpr bool kLong = FP8 && FAST;
-        uint32_t sc[32];
-        const float row_max = warp_full ? softmax_row_max<false, kLong>(t_s, sc, k0, lo, hi) : softmax_row_max<true, kLong>(t_s, sc, k0, lo, hi);
+        uint32_t sc[32], held[HELD ? 4 : 1][32];
+        bool dead[4];
+        float row_max;
+        if constexpr (HELD) row_max = warp_full ? softmax_row_max_held<false>(t_s, held, dead, k0, lo, hi) : softmax_row_max_held<true>(t_s, held, dead, k0, lo, hi);
+        else row_max = warp_full ? softmax_row_max<false, kLong>(t_s, sc, k0, lo, hi) : softmax_row_max<true, kLong>(t_s, sc, k0, lo, hi);
         const float m_new = fmaxf(m_used, row_max * scale);
         // lazy rescale: keep the old reference maximum unless the new one is larger by more than the threshold
         const bool need = m_new > m_used + (FP8 ? kRescaleThresholdFp8 : kRescaleThreshold);
@@ -711,15 +758,20 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         KB_FACC(3);
         const float m_exp = m_used - p_off;  // 2^(s scale - m_exp) = p * 2^p_off
         const float m_safe = (m_exp == -INFINITY) ? 0.f : m_exp;
-        const uint64_t scale2 = f2_pack(scale, scale), negm2 = f2_pack(-m_safe, -m_safe);
-        SoftSum sum2;
-        sum2.s01 = sum2.s23 = f2_pack(0.f, 0.f);
-        if (warp_full) softmax_exp<BF16, false, FP8, kLong>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
-        else softmax_exp<BF16, true, FP8, kLong>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
-        float sum4[4];
-        f2_unpack(sum2.s01, sum4[0], sum4[1]);
-        f2_unpack(sum2.s23, sum4[2], sum4[3]);
-        const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+        float sum;
+        if constexpr (HELD) {
+          sum = warp_full ? softmax_exp_held<BF16, false>(t_s, held, dead, scale, m_safe) : softmax_exp_held<BF16, true>(t_s, held, dead, scale, m_safe);
+        } else {
+          const uint64_t scale2 = f2_pack(scale, scale), negm2 = f2_pack(-m_safe, -m_safe);
+          SoftSum sum2;
+          sum2.s01 = sum2.s23 = f2_pack(0.f, 0.f);
+          if (warp_full) softmax_exp<BF16, false, FP8, kLong>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
+          else softmax_exp<BF16, true, FP8, kLong>(t_s, sc, scale2, negm2, k0, lo, hi, sum2);
+          float sum4[4];
+          f2_unpack(sum2.s01, sum4[0], sum4[1]);
+          f2_unpack(sum2.s23, sum4[2], sum4[3]);
+          sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+        }
         // the rescale of O comes after the exponentials: the row's scores are dead by now, which keeps the
         // registers of the two from being live together
         if (lx > 0 && __any_sync(0xffffffffu, need)) {
@@ -838,15 +890,26 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
                 make_tile_map_4d(&tm_v, p.v, mapB, H_kv, mapT, D, kBN);
   if (!maps_ok || !make_tile_map_4d(&tm_o, out_view(p.o, p.o_stride, p.H, mapTq, D), mapB, p.H, mapTq, D, kBM))
     return KB_ERR_UNSUPPORTED;
+  int dev = 0, n_sm = 0;
+  if (!device_sm_count(&dev, &n_sm)) return KB_ERR_LAUNCH;
   // chunk lengths that are multiples of the work item's rows get the instance with the straight-line schedule
   const bool fast = c % (kBM * kQTiles) == 0;
-  auto kern = fast ? sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, true> : sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, false>;
+  const int64_t n_items = (int64_t)p.B * p.H * kb_cdiv_i32(Tq, kBM * kQTiles);
+  if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
+  // Head dim 64: the scores held in registers (softmax_row_max_held) where no CTA sees a second item, and where a row walks 12
+  // key tiles or more.  Two walks / held, us, fp16: one wave, dense T=2048 37.1 / 32.5, T=1500 34.0 / 31.3, T=900 21.3 / 19.6,
+  // c=10 T=1000 12.2 / 11.7; many, T=4000 unless said, dense T=2048 328 / 319, T=3333 379 / 355, T=1500 303 / 288, c=256 back=6
+  // 270 / 255, c=512 back=2 291 / 280, c=300 back=4 397 / 389, c=100 back=15 390 / 390.  Fewer tiles: c=256 T=1000 135 / 155,
+  // back=3 183 / 177, c=200 back=4 258 / 268, c=128 back=4 154 / 150, c=100 back=6 259 / 289, c=10 196 / 209, dense T=700 206 / 217.
+  constexpr bool kHolds = D == 64 && !FP8;
+  const int64_t row_keys = kb_min_i32(PACKED ? p.total_rows / p.B : p.T, (int32_t)std::min<int64_t>((int64_t)(back + 1) * c, INT32_MAX));
+  const bool held = kHolds && (n_items <= n_sm || row_keys >= 12 * kBN);
+  auto kern = fast ? (held ? sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, true, kHolds> : sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, true, false>)
+                   : (held ? sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, false, kHolds> : sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, false, false>);
   constexpr size_t smem = sizeof(FwdSmem<D>);
   static_assert(sizeof(FwdSmem<D>) <= 232448, "forward shared memory exceeds the 227 KB a CTA may have");
-  int dev = 0;
-  KB_CUDA_TRY(cudaGetDevice(&dev));
-  static std::atomic<bool> smem_opted_in[kMaxDevices], smem_opted_in_fast[kMaxDevices];
-  KB_CUDA_TRY(opt_in_smem_once(kern, smem, dev, fast ? smem_opted_in_fast : smem_opted_in));
+  static std::atomic<bool> smem_opted_in[2][2][kMaxDevices];
+  KB_CUDA_TRY(opt_in_smem_once(kern, smem, dev, smem_opted_in[fast][held]));
   FwdArgs a;
   a.o = p.o;
   a.lse = p.lse;
@@ -879,8 +942,6 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   a.v_scale_max = f8 ? f8->v_scale_max : nullptr;
   a.n128 = kb_cdiv_i32(p.T, 128);
   a.Hk = H_kv;
-  const int64_t n_items = (int64_t)p.B * p.H * kb_cdiv_i32(Tq, kBM * kQTiles);
-  if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
   kern<<<(unsigned)n_items, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
   KB_LAUNCH_CHECK("sa_fwd_sm100_kernel");
   return KB_OK;
