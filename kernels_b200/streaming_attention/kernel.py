@@ -374,10 +374,11 @@ class _StreamingAttention(torch.autograd.Function):
         # A transform or a mode around the backward pass meets the operator, and so does a pass that is to be
         # differentiated again: the operator has no gradient and says so.
         gradients = torch.ops.alexdremov_streaming_attention.backward
-        if not torch.is_grad_enabled() and _lib.plain_call(do):
+        if _lib.plain_call(do):
             if not do.is_contiguous() and not _rows_in_place(do):
                 do = do.contiguous()  # see _backward
-            gradients = _gradients
+            if not torch.is_grad_enabled():
+                gradients = _gradients
         return (*gradients(q, k, v, lens, o, lse, do, *ctx.args), None, None, None, None, None, None, None)
 
 

@@ -524,6 +524,22 @@ def test_gradients_of_any_layout_take_the_same_kernels(dtype, D):
         assert all(torch.equal(a, b) for a, b in zip(got, want)), name
 
 
+def test_expanded_gradients_under_create_graph_take_the_same_kernels():
+    """A backward pass that is to be differentiated again launches the kernels of an ordinary one, also where the output
+    gradient is expanded (``o.sum()``)."""
+    from kernels_b200 import _lib
+
+    q, k, v = (torch.randn(2, 3, 150, 64, device="cuda", dtype=torch.bfloat16).requires_grad_() for _ in range(3))
+    o = _api()(q, k, v, None, 24, 2)
+    do = torch.ones((), device="cuda", dtype=torch.bfloat16).expand_as(o)
+    n0 = _lib.launch_count()
+    want = torch.autograd.grad(o, (q, k, v), do.contiguous(), retain_graph=True)
+    n1 = _lib.launch_count()
+    got = torch.autograd.grad(o, (q, k, v), do, create_graph=True)
+    assert _lib.launch_count() - n1 == n1 - n0
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_numbers_that_are_not_pythons_own_are_refused():
     """Chunk length, look-back and scale as numpy numbers or zero-dimensional tensors: refused on an ordinary call as
     inside a compiled function."""
