@@ -434,9 +434,14 @@ def streaming_attention(
     # operators' own autograd wrappers 100 of the rest, where the kernels of a small one take 55.  Everything
     # that looks inside (an outer compilation, transforms, hooks, modes) still meets the compiled function, and so do numbers
     # that are not Python's own: it refuses numpy's and zero-dimensional tensors, which the body alone would take.
+    # Other arguments of types that the operator's schema does not name are left to the operator, which takes some of them
+    # (1 as a flag) and refuses others (a string or a list as one, numbers beyond 64 bits, a list of lengths).
     numbers = type(context_size) in (int, bool) and type(back_contexts) in (int, bool) and type(sm_scale) in (type(None), int, float)
     if numbers and _lib.plain_call(q, k, v):
-        attention = _streaming_attention_eager
+        named = (
+            type(autotune) is bool and type(return_lse) is bool and type(prescale_qk) is bool and type(precision) is str
+            and type(lens) in (type(None), torch.Tensor) and context_size.bit_length() < 64 and back_contexts.bit_length() < 64)
+        attention = _streaming_attention_eager if named else _streaming_attention_op
     else:
         attention = _streaming_attention
         if not torch.compiler.is_compiling():

@@ -557,6 +557,21 @@ def test_numbers_that_are_not_pythons_own_are_refused():
     assert torch.equal(streaming_attention(q, k, v, None, 16, 2, sm_scale=1), streaming_attention(q, k, v, None, 16, 2, sm_scale=1.0))
 
 
+@pytest.mark.parametrize("grad", [False, True])
+def test_arguments_outside_the_operators_schema(grad):
+    """What the operator's schema refuses is refused on an ordinary call, what it converts is taken."""
+    q, k, v = (torch.randn(1, 2, 64, 64, device="cuda", dtype=torch.float16).requires_grad_(grad) for _ in range(3))
+    for args, kw in (((16, 2), dict(prescale_qk="x")), ((16, 2), dict(autotune=[1])), ((2**64, 2), {}), ((16, 2**70), {})):
+        with pytest.raises(RuntimeError):
+            _api()(q, k, v, None, *args, **kw)
+    with pytest.raises(RuntimeError):
+        _api()(q, k, v, [64], 16, 2)
+    want = _api()(q, k, v, None, 16, 2)
+    for kw in (dict(prescale_qk=0), dict(autotune=1), dict(prescale_qk=None), dict(precision=b"ieee")):
+        assert torch.equal(_api()(q, k, v, None, 16, 2, **kw), want)
+    assert torch.equal(_api()(q, k, v, None, 2**63 - 1, True), _api()(q, k, v, None, 64, 1))
+
+
 @pytest.mark.parametrize("dtype, D", [(torch.float32, 32), (torch.bfloat16, 64)], ids=str)
 def test_backward_of_ordinary_calls(dtype, D):
     """Through the direct route: a second differentiation is refused, also where the output gradient needs none; batched
