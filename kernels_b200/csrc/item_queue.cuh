@@ -11,13 +11,18 @@
 // is complete, and would wait for ever behind a run of padded ones that fills the ring.)  It asks when it has
 // issued the loads of an item's last tiles: the answer takes 350 clocks, and an item claimed earlier would wait at a CTA that is still busy.
 // Or (n_fixed) it takes the items in turn with the grid's other CTAs; sa_bwd_fused_sm100.cu says where that is better.
+//
+// A block without work costs that answer all the same, so a packed batch does not launch a block for every tile of its
+// longest sequence times every sequence where that is mostly padding (PackedGrid).
 #pragma once
+#include "common.cuh"
 #include "sm100_ptx.cuh"
 
 namespace kb {
 namespace sm100 {
 
 constexpr int kItemSlots = 4;
+constexpr int kItemsOver = -1, kItemPadding = -2;
 enum ItemWaitSite { kWaitItemAnswer = 121, kWaitItemEmpty, kWaitItemFull };
 
 struct alignas(16) ItemQueue {
@@ -42,7 +47,7 @@ __device__ __forceinline__ void item_ask(ItemQueue* q) {
                "r"(smem_u32(&q->answered))
                : "memory");
 }
-// The block index in the answer, -1 if there was no block left to take over (after which none may be asked for).
+// The block index in the answer, kItemsOver if there was no block left to take over (after which none may be asked for).
 __device__ __forceinline__ int item_answer(const ItemQueue* q) {
   uint32_t got, x;
   asm volatile(
@@ -55,7 +60,7 @@ __device__ __forceinline__ int item_answer(const ItemQueue* q) {
       : "r"(smem_u32(q->answer))
       : "memory");
   fence_proxy_async();  // (the next answer is written through the async proxy)
-  return got ? (int)x : -1;
+  return got ? (int)x : kItemsOver;
 }
 // After a wait of the CTA gave up: the blocks not launched yet are taken over and dropped, so that the kernel ends with
 // the error code now and not after as many such waits as there are items left.  `answers`: answers taken so far.
@@ -69,14 +74,61 @@ static __device__ __noinline__ void item_drop_rest(ItemQueue* q, int answers, bo
   }
 }
 
+// The blocks of a packed batch, [sequence][head][tile of the sequence]: sequence b begins at block heads * (cu[b] / tile +
+// b).  That leaves every (sequence, head) room for its own tiles and at most one more, and needs nothing of the lengths but
+// their sum on the host and their offsets here.  With a block per tile of the longest sequence (n_seqs = 0, item = block)
+// one sequence of 32 768 rows among 1 000 of 100 (16 heads, D = 128, c = 64) has 4.1 M blocks in the main kernel, of which
+// 20 thousand have work.  Block per tile / this, us: forward 6 700 / 626, main 14 330 / 812, dQ 12 520 / 397; 16 384 among
+// 500 of 60 (8 heads, D = 64) 880 / 124, 1 850 / 177, 1 614 / 87.  Finding a block's item takes the loads of two searches
+// and two divisions, which batches of short items notice; so the host takes this grid where it has less than half as many
+// blocks: at 0.44 of them (2 048 rows and four of 448, forty times) forward 525 / 529, main 930 / 942, dQ 368 / 353.
+struct PackedGrid {
+  const int32_t* cu;
+  int32_t n_seqs, heads, shift, T, n_tiles;  // tiles of 2^shift rows; T: the longest sequence, n_tiles: its tiles
+};
+// The item of a block, as (sequence * heads + head) * n_tiles + tile, kItemPadding if it has none.  By a whole warp: 32
+// sequences are looked at at a time.  Out of line: in the main kernel's loop it cost every packed batch 3 to 5 %.
+static __device__ __noinline__ int packed_item(const int32_t* cu, int n_seqs, int heads, int shift, int T, int n_tiles, int block) {
+  const int lane = threadIdx.x & 31;
+  int b = 0;
+  for (int n = n_seqs; n > 1;) {  // the block belongs to one of the sequences [b, b + n)
+    const int step = (n + 31) >> 5, at = lane * step;
+    const bool begun = at < n && heads * ((cu[b + at] >> shift) + b + at) <= block;
+    const int skip = kb_max_i32(__popc(__ballot_sync(0xffffffffu, begun)) - 1, 0) * step;
+    b += skip;
+    n = kb_min_i32(step, n - skip);
+  }
+  const int row0 = cu[b], end = cu[b + 1];
+  const int per_head = kb_max_i32((end >> shift) - (row0 >> shift) + 1, 1);
+  const int rest = block - heads * ((row0 >> shift) + b);
+  const int h = rest / per_head, tile = rest - h * per_head;
+  if (rest < 0 || h >= heads || tile << shift >= kb_min_i32(end - row0, T)) return kItemPadding;
+  return (b * heads + h) * n_tiles + tile;
+}
+// ... and on the host: the number of blocks of a packed batch, and which of the two grids they are.
+inline int64_t packed_grid_blocks(PackedGrid& g, const int32_t* cu, int32_t B, int32_t heads, int32_t T, int32_t total, int32_t shift) {
+  const int32_t n_tiles = kb_cdiv_i32(T, 1 << shift);
+  const int64_t each = (int64_t)B * heads * n_tiles, own = (int64_t)heads * ((total >> shift) + B);
+  const bool by_rows = 2 * own < each;
+  g = PackedGrid{cu, by_rows ? B : 0, heads, shift, T, n_tiles};
+  return by_rows ? own : each;
+}
+
 // Used by a whole converged warp; item() is the same in all lanes, the rest is lane 0's.
+template <bool PACKED>
 struct ItemWriter {
   ItemQueue* q;
+  const PackedGrid& grid;         // (in the kernel's parameters; used if PACKED)
   int n_fixed;                    // > 0: the CTAs of the grid take these items in turn, nothing is asked for
-  int answers, published, item_;  // answers taken, items passed on so far; the current item, -1 after the last one
+  int answers, published, item_;  // answers taken, items passed on so far; the current item, kItemsOver after the last one
   bool asked, more, ok;          // a request is under way; no request has failed yet; no wait gave up
-  __device__ __forceinline__ explicit ItemWriter(ItemQueue& queue, int fixed = 0)
-      : q(&queue), n_fixed(fixed), answers(0), published(0), item_((int)blockIdx.x), asked(false), more(fixed == 0), ok(true) {}
+  __device__ __forceinline__ ItemWriter(ItemQueue& queue, const PackedGrid& packed_grid, int fixed = 0)
+      : q(&queue), grid(packed_grid), n_fixed(fixed), answers(0), published(0), item_(of_block((int)blockIdx.x)), asked(false), more(fixed == 0), ok(true) {}
+  __device__ __forceinline__ bool more_items() const { return PACKED ? item_ != kItemsOver : item_ >= 0; }
+  __device__ __forceinline__ int of_block(int block) const {
+    if (!PACKED || grid.n_seqs == 0 || block < 0) return block;
+    return packed_item(grid.cu, grid.n_seqs, grid.heads, grid.shift, grid.T, grid.n_tiles, block);
+  }
   __device__ __forceinline__ int item() const { return item_; }
   // Lane 0: ask for the next item ahead of next().
   __device__ __forceinline__ void ask() {
@@ -110,7 +162,7 @@ struct ItemWriter {
         }
       }
     }
-    item_ = __shfl_sync(0xffffffffu, got, 0);
+    item_ = of_block(__shfl_sync(0xffffffffu, got, 0));
   }
   // Lane 0, after the walk.
   __device__ __forceinline__ void finish(const WaitCtx& ctx) {

@@ -100,13 +100,14 @@ struct FusedArgs {
   int64_t lens_stride;
   int64_t lse_sb, lse_sh;                      // element strides of lse (b, h)
   int64_t dq_sb, dq_sh, dq_st, dkv_sb, dkv_sh, dkv_st;  // of dq and of dk / dv (b, h, t)
-  int32_t B, H, T, c, back, W;
+  int32_t H, T, c, back, W;
   int32_t Hk, group;  // key/value heads and query heads per key/value head (H = Hk * group)
   // Packed batch: sequence b owns the rows [cu[b], cu[b + 1]) of tensors with ONE batch entry (the maps' batch
   // extent is 1, every *_sb stride is 0), T is the longest sequence, lse and delta are [H, total rows], and the
   // dS scratch is indexed by packed key tile (ptile_id below), n_ptiles of them per head.  NULL: padded layout.
   const int32_t* cu;
   int32_t total, n_ptiles;
+  PackedGrid grid, grid_dq;  // of the main and of the dQ kernel
   KbFastDiv fd_tiles, fd_H, fd_Hk, fd_group, fd_c;  // division by ceil(T / 128), H, Hk, group and c
   int32_t n_fixed;  // > 0: the main kernel's CTAs take the items in turn (see ItemWriter)
   float scale_log2, sm_scale;
@@ -324,8 +325,9 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         prefetch_tensormap(&tm_do);
       }
       bool ok = true;
-      auto c = cursor_first<PACKED>(a, ItemWriter(sm.items, a.n_fixed), n_ktiles);
-      for (; c.valid; c.items.next(ok, ctx), cursor_open<PACKED>(a, c, n_ktiles)) {
+      auto c = cursor_first<PACKED>(a, ItemWriter<PACKED>(sm.items, a.grid, a.n_fixed), n_ktiles);
+      for (; c.items.more_items(); c.items.next(ok, ctx), cursor_open<PACKED>(a, c, n_ktiles)) {
+        if (PACKED && c.items.item() == kItemPadding) continue;
         if (c.it.qr.begin >= c.it.qr.end) {
           // the whole key tile lies in the padding: its gradients are zeros.  A packed batch has no padding rows.
           if (!PACKED) {
@@ -988,8 +990,9 @@ sa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     if (lane == 0) prefetch_tensormap(&tm_k);
     int u = 0;
     bool ok = true;
-    ItemWriter items(sm.items);
-    for (; items.item() >= 0; items.next(ok, ctx)) {
+    ItemWriter<PACKED> items(sm.items, a.grid_dq);
+    for (; items.more_items(); items.next(ok, ctx)) {
+      if (PACKED && items.item() == kItemPadding) continue;
       const DqItem it = decode_dq_item<PACKED>(a, items.item(), n_tiles_t);
       if (it.kr.begin >= it.kr.end) {
         // the whole query tile lies in the padding: its gradient is zero.  A packed batch has no padding rows.
@@ -1170,6 +1173,8 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.cu = PACKED ? p.cu_seqlens : nullptr;
   fa.total = PACKED ? p.total_rows : 0;
   fa.n_ptiles = PACKED ? packed_tiles(p.total_rows, p.B) : 0;
+  const int64_t n_blocks = PACKED ? packed_grid_blocks(fa.grid, p.cu_seqlens, p.B, Hk, p.T, p.total_rows, 7) : n_items_main;
+  const int64_t n_blocks_dq = PACKED ? packed_grid_blocks(fa.grid_dq, p.cu_seqlens, p.B, p.H, p.T, p.total_rows, 7) : n_items;
   fa.delta = p.delta_ws;
   fa.ds_ws = static_cast<uint8_t*>(p.ds_ws);
   fa.dk = p.dk;
@@ -1177,7 +1182,6 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.dq = p.dq;
   fa.lens = p.lens;
   fa.lens_stride = p.lens_stride;
-  fa.B = p.B;
   fa.H = p.H;
   fa.T = p.T;
   fa.c = c;
@@ -1199,14 +1203,14 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   // c=300 T=2048 787 / 742, fp16 D=64 c=256 T=1000 472 / 415; with lengths c=256 too (T=2048, in the fixed order 656 / 566).
   const bool fixed = D == 128 && c % (2 * kBK) == 0 && !p.lens && !PACKED;
   fa.n_fixed = fixed ? (int32_t)n_items_main : 0;
-  const unsigned grid_main = (unsigned)(fixed && n_items_main > n_sm ? n_sm : n_items_main);
+  const unsigned grid_main = (unsigned)(fixed && n_items_main > n_sm ? n_sm : n_blocks);
   fa.status = p.status;
   if (!(p.flags & KB_FLAG_BWD_SKIP_DKDV)) {
     main_kern<<<grid_main, kThreads, sizeof(FusedSmem<D>), s>>>(tm_k, tm_v, tm_q, tm_do, tm_dk, tm_dv, fa);
     KB_LAUNCH_CHECK("sa_bwd_fused_kernel");
   }
   if (!(p.flags & KB_FLAG_BWD_SKIP_DQ)) {
-    dq_kern<<<(unsigned)n_items, kDqThreads, sizeof(DqSmem<D>), s>>>(tm_k, tm_dq, fa);
+    dq_kern<<<(unsigned)n_blocks_dq, kDqThreads, sizeof(DqSmem<D>), s>>>(tm_k, tm_dq, fa);
     KB_LAUNCH_CHECK("sa_bwd_dq_kernel");
   }
   return KB_OK;

@@ -81,11 +81,12 @@ struct FwdArgs {
   const int32_t* lens;
   int64_t lens_stride;
   int64_t o_sb, o_sh, o_st, lse_sb, lse_sh;  // element strides of o (b, h, t) and of lse (b, h)
-  int32_t B, H, T, c, back;
+  int32_t H, T, c, back;
   int32_t q_start;  // the query rows are the positions [q_start, T): row r of q / o / lse is position q_start + r
   // Packed batch: sequence b owns the rows [cu[b], cu[b + 1]) of tensors with ONE batch entry (the maps' batch
   // extent is 1, o_sb = lse_sb = 0) and T is the longest sequence.  NULL: the padded layout.
   const int32_t* cu;
+  PackedGrid grid;
   KbFastDiv fd_qblocks, fd_H, fd_c, fd_group;  // division by ceil(T / 256), H, c and H / H_kv (query heads per K/V head)
   float scale_log2;
   int32_t* status;
@@ -383,8 +384,9 @@ sa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     int kc = 0, vc = 0;
     int items_x[kQTiles] = {0, 0};  // items in which q tile x was live so far
     bool ok = true;
-    ItemWriter items(sm.items);
-    for (; items.item() >= 0; items.next(ok, ctx)) {
+    ItemWriter<PACKED> items(sm.items, a.grid);
+    for (; items.more_items(); items.next(ok, ctx)) {
+      if (PACKED && items.item() == kItemPadding) continue;
       const Item it = decode(items.item());
       if (!it.act[0]) {  // (tile B is never live without tile A)
         // the q block lies wholly in the padding: its rows are zeros (a packed batch has no padding rows)
@@ -896,6 +898,8 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   const bool fast = c % (kBM * kQTiles) == 0;
   const int64_t n_items = (int64_t)p.B * p.H * kb_cdiv_i32(Tq, kBM * kQTiles);
   if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
+  FwdArgs a;
+  const int64_t n_blocks = PACKED ? packed_grid_blocks(a.grid, p.cu_seqlens, p.B, p.H, p.T, p.total_rows, 8) : n_items;
   // Head dim 64: the scores held in registers (softmax_row_max_held) where no CTA sees a second item, and where a row walks 12
   // key tiles or more.  Two walks / held, us, fp16: one wave, dense T=2048 37.1 / 32.5, T=1500 34.0 / 31.3, T=900 21.3 / 19.6,
   // c=10 T=1000 12.2 / 11.7; many, T=4000 unless said, dense T=2048 328 / 319, T=3333 379 / 355, T=1500 303 / 288, c=256 back=6
@@ -910,7 +914,6 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   static_assert(sizeof(FwdSmem<D>) <= 232448, "forward shared memory exceeds the 227 KB a CTA may have");
   static std::atomic<bool> smem_opted_in[2][2][kMaxDevices];
   KB_CUDA_TRY(opt_in_smem_once(kern, smem, dev, smem_opted_in[fast][held]));
-  FwdArgs a;
   a.o = p.o;
   a.lse = p.lse;
   a.lens = p.lens;
@@ -923,7 +926,6 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
     a.lse_sh = lse_packed ? (int64_t)mapTq : p.lse_stride[1];
     if (p.cu_seqlens) a.o_sb = a.lse_sb = 0;  // the sequence's first row carries the batch offset
   }
-  a.B = p.B;
   a.H = p.H;
   a.T = p.T;
   a.c = c;
@@ -942,7 +944,7 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   a.v_scale_max = f8 ? f8->v_scale_max : nullptr;
   a.n128 = kb_cdiv_i32(p.T, 128);
   a.Hk = H_kv;
-  kern<<<(unsigned)n_items, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
+  kern<<<(unsigned)n_blocks, kThreads, smem, s>>>(tm_q, tm_k, tm_v, tm_o, a);
   KB_LAUNCH_CHECK("sa_fwd_sm100_kernel");
   return KB_OK;
 }

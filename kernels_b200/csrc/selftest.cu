@@ -68,7 +68,8 @@ __global__ void __launch_bounds__(160) reader_group_selftest_kernel(int32_t* sta
   };
   if (warp == 4) {
     if (lane == 0) {
-      ItemWriter items(queue, 1);  // (a fixed walk: nothing is asked of the hardware)
+      const PackedGrid unused{};
+      ItemWriter<false> items(queue, unused, 1);  // (a fixed walk: nothing is asked of the hardware)
       items.publish(make_int4(5, 0, 0, 0), ctx);
       wait_for(&gone, 4);  // every warp has worked on item 5
       *ctx.abort_flag = 1;

@@ -38,10 +38,14 @@ def _cu(lens):
     # ... and with shared key/value heads: more (key tile, key/value head) items per sequence than CTAs too
     (16, 8, 2600, 128, 256, 2, torch.bfloat16, [2500, 77, 2600]),
     (16, 8, 2600, 64, 64, 2, torch.float16, [300, 2600, 2500]),
-    # few tiles per sequence, more items than CTAs: the padded and the one-launch call shift their items from wave to
-    # wave, the launches per sequence do not
+    # few tiles per sequence, more items than CTAs
     (4, 4, 500, 64, 10, 4, torch.float16, [(37 * i) % 501 for i in range(60)]),
     (4, 2, 1000, 128, 64, 2, torch.bfloat16, [(61 * i) % 1001 for i in range(40)]),
+    # one long sequence among short ones: the grid has a block per tile of the batch and not of the longest sequence;
+    # more sequences than a warp has lanes, than it has lanes squared; and lengths for which it stays as it is
+    (2, 2, 1500, 128, 64, 2, torch.bfloat16, [1, 0, 128, 129, 256, 257, 0, 1500] + [3] * 40 + [255]),
+    (2, 1, 900, 64, 10, 4, torch.float16, [5] * 700 + [900] + [2] * 400),
+    (4, 4, 256, 128, 128, 1, torch.bfloat16, [256] * 50),
 ])
 @pytest.mark.parametrize("single_launch", [True, False])
 def test_packed_equals_padded_bitwise(H, Hk, T, D, c, back, dtype, lens, single_launch):
@@ -116,6 +120,36 @@ def test_more_tiles_per_sequence_than_ctas_against_64_bits(D, c, back, dtype):
                     assert float(rel.max()) <= bound, (form, name, b, t0, rel.tolist())
             assert not pad[b, :, L:].any(), name  # padding rows are zeros
         r0 += L
+
+
+def test_blocks_follow_the_rows_of_a_packed_batch():
+    """One long sequence among many short ones costs about what its rows cost, not a block for every tile of the longest
+    sequence times every sequence: forward and backward take less than six times as long as the long sequence and the short
+    ones packed apart (measured 2.7 times, and 26 with such blocks)."""
+    from kernels_b200.streaming_attention import streaming_attention_varlen
+
+    def passes(lens):
+        q, k, v, do = (torch.randn(sum(lens), 8, 64, device="cuda", dtype=torch.float16).requires_grad_() for _ in range(4))
+        cu = _cu(lens)
+
+        def once():
+            torch.autograd.grad(streaming_attention_varlen(q, k, v, cu, 100, 1), (q, k, v), do)
+
+        return once
+
+    def device_us(once):
+        times = []
+        for i in range(8):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            once()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return sorted(times)[2]
+
+    both, long, short = (device_us(passes(lens)) for lens in ([32768] + [60] * 2000, [32768], [60] * 2000))
+    assert both < 6 * (long + short), (both, long, short)
 
 
 def test_packed_against_oracle_per_sequence():
