@@ -1196,12 +1196,14 @@ int launch_fused(const kb_sa_bwd_params& p, int32_t c, int32_t back, cudaStream_
   fa.fd_c = kb_fastdiv_make(c);
   fa.scale_log2 = p.sm_scale * kLog2e;
   fa.sm_scale = p.sm_scale;
-  // Where every sequence is as long and chunks are whole pairs of key tiles, CTAs 2 m and 2 m + 1 of the fixed order always
-  // work on the two key tiles of one chunk, which stream the same Q / dO tiles.  Fixed / taken as CTAs become free, us, bf16
-  // D=128: c=256 T=16384 1567 / 1650, T=8192 577 / 604, T=2048 542 / 563, T=1000 518 / 508; c=512 T=2048 842 / 861, T=1000
-  // 585 / 623, T=600 538 / 506.  Elsewhere the second: c=64 T=8192 290 / 254, c=128 420 / 382, c=200 T=1000 620 / 551,
-  // c=300 T=2048 787 / 742, fp16 D=64 c=256 T=1000 472 / 415; with lengths c=256 too (T=2048, in the fixed order 656 / 566).
-  const bool fixed = D == 128 && c % (2 * kBK) == 0 && !p.lens && !PACKED;
+  // Where every sequence is as long, an even number of key tiles, and chunks are whole pairs of key tiles, CTAs 2 m and 2 m + 1
+  // of the fixed order always work on the two key tiles of one chunk, which stream the same Q / dO tiles.  Fixed / taken as
+  // CTAs become free, us, bf16 D=128: c=256 T=16384 1567 / 1650, T=8192 577 / 604, T=2048 542 / 563, T=1536 1483 / 1480, T=1000
+  // (8 tiles) 518 / 508, c=512 T=2048 842 / 861, T=1000 585 / 623.  With an odd number every second sequence's pairs are split
+  // between CTAs 2 m + 1 and 2 m + 2: c=256 T=16500 1486 / 1452, T=4200 1634 / 1612, T=2100 1627 / 1564, T=1100 1507 / 1446, c=512
+  // T=600 538 / 506.  Elsewhere the second too: c=64 T=8192 290 / 254, c=128 420 / 382, c=200 T=1000 620 / 551,
+  // c=300 T=2048 787 / 742, fp16 D=64 c=256 T=1000 472 / 415; with lengths c=256 (T=2048, in the fixed order 656 / 566).
+  const bool fixed = D == 128 && c % (2 * kBK) == 0 && n_tiles % 2 == 0 && !p.lens && !PACKED;
   fa.n_fixed = fixed ? (int32_t)n_items_main : 0;
   const unsigned grid_main = (unsigned)(fixed && n_items_main > n_sm ? n_sm : n_blocks);
   fa.status = p.status;

@@ -188,6 +188,34 @@ def test_long_runs_of_padded_work_items(D, c, back):
     _run_case(6, 12, 1300, D, c, back, torch.bfloat16, torch.tensor([1300, 0, 1, 0, 700, 129], dtype=torch.int32), False)
 
 
+def _lib_check():
+    from kernels_b200 import _lib
+
+    torch.cuda.synchronize()
+    _lib.check_device_status()
+
+
+def _passes(q, k, v, lens, do, c, back):
+    o, lse = _api()(q, k, v, lens, c, back, return_lse=True)
+    return (o.detach(), lse, *torch.autograd.grad(o, (q, k, v), do))
+
+
+@pytest.mark.parametrize("T", [1024, 1100])
+def test_uniform_batches_in_either_item_order(T):
+    """Sequences of one length, an even (fixed item order) and an odd number of key tiles (the queue), several items per CTA:
+    the bits of calls in which no CTA sees a second one."""
+    B, H, few = 2, 60, 4
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn(B, H, T, 128, generator=g, device="cuda").bfloat16() for _ in range(4))
+    assert B * H * (T // 128) > 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    got = _passes(*(t.requires_grad_() for t in (q, k, v)), None, do, 256, 2)
+    for h in range(0, H, 5 * few):
+        part = [t.detach()[:, h:h + few] for t in (q, k, v, do)]
+        want = _passes(*(t.requires_grad_() for t in part[:3]), None, part[3], 256, 2)
+        assert all(torch.equal(a[:, h:h + few], b) for a, b in zip(got, want))
+    _lib_check()
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=str)
 @pytest.mark.parametrize("D", [64, 128])
 def test_rows_whose_last_tile_is_the_only_live_one(dtype, D):
