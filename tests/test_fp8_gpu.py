@@ -80,6 +80,33 @@ def test_fp8_forward_against_the_16_bit_kernel_at_length():
     assert float((lse - ref_lse).abs().max()) <= 5e-2
 
 
+@pytest.mark.parametrize("c, back", [(256, 2), (64, 8), (100, 1)])
+@pytest.mark.parametrize("lens", [None, [2048, 0, 777, 1]])
+def test_fp8_forward_with_many_items_per_cta(c, back, lens):
+    """Several work items per CTA, padded ones among them: the bits of calls in which no CTA sees a second one (those
+    are held against the oracle above)."""
+    from kernels_b200.streaming_attention import streaming_attention_fp8
+
+    B, H, T, few = 4, 32, 2048, 16
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert B * H * T // 256 > 6 * sms and few * T // 256 <= sms
+    g = torch.Generator(device="cuda").manual_seed(7)
+    t8 = [quantize_fp8_tiles(torch.randn(B, H, T, 128, generator=g, device="cuda")) for _ in range(3)]
+    lens = None if lens is None else torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+    def attend(cut):
+        (q, qs), (k, ks), (v, vs) = ((t[cut], s[cut]) for t, s in t8)
+        return streaming_attention_fp8(q, k, v, qs, ks, vs, None if lens is None else lens[cut[0]], c, back, return_lse=True)
+
+    got = attend((slice(0, B), slice(0, H)))
+    for b in range(B):
+        for h in (0, few):
+            cut = (slice(b, b + 1), slice(h, h + few))
+            assert all(torch.equal(a[cut], w) for a, w in zip(got, attend(cut)))
+    torch.cuda.synchronize()
+    _lib.check_device_status()
+
+
 def test_fp8_forward_rejects_what_the_kernel_does_not_take():
     import ctypes
 

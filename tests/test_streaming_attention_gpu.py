@@ -184,7 +184,7 @@ def test_long_sequence_class_with_several_work_items_per_cta(D):
 @pytest.mark.parametrize("c, back", [(10, 9), (128, 1), (256, 2)])
 def test_long_runs_of_padded_work_items(D, c, back):
     """More work items than CTAs, and between the live ones runs of up to 72 (132 in the backward) that lie wholly in the
-    padding: a CTA takes many of them in a row, their outputs are zeros, the next live item is found."""
+    padding: their outputs are zeros, the next live item is found."""
     _run_case(6, 12, 1300, D, c, back, torch.bfloat16, torch.tensor([1300, 0, 1, 0, 700, 129], dtype=torch.int32), False)
 
 
@@ -200,6 +200,27 @@ def _passes(q, k, v, lens, do, c, back):
     return (o.detach(), lse, *torch.autograd.grad(o, (q, k, v), do))
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("c, back", [(10, 9), (128, 1), (256, 2)])
+def test_many_live_items_per_cta_between_padded_ones(D, c, back):
+    """Every CTA of the three kernels works on more items than its ring has entries, runs of padded items between them: the
+    bits of calls on a few heads, in which no CTA sees a second one."""
+    H, T, lens = 72, 1300, [1300, 0, 1, 0, 700, 129]
+    sms, few = torch.cuda.get_device_properties(0).multi_processor_count, 1
+    live = [sum(-(-n // rows) for n in lens) for rows in (256, 128)]  # items per head: forward; main and dQ
+    assert H * live[0] > 5 * sms and H * live[1] > 5 * sms and few * len(lens) * -(-T // 128) <= sms
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(len(lens), H, T, D, generator=g, device="cuda").bfloat16().requires_grad_() for _ in range(3))
+    do = torch.randn(len(lens), H, T, D, generator=g, device="cuda").bfloat16()
+    lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    got = _passes(q, k, v, lens, do, c, back)
+    for h in range(0, H, 6 * few):  # (a sixth of the heads)
+        part = [t[:, h:h + few] for t in (q, k, v, do)]
+        want = _passes(*(t.detach().requires_grad_() for t in part[:3]), lens, part[3], c, back)
+        assert all(torch.equal(a[:, h:h + few], b) for a, b in zip(got, want))
+    _lib_check()
+
+
 @pytest.mark.parametrize("T", [1024, 1100])
 def test_uniform_batches_in_either_item_order(T):
     """Sequences of one length, an even (fixed item order) and an odd number of key tiles (the queue), several items per CTA:
@@ -213,6 +234,27 @@ def test_uniform_batches_in_either_item_order(T):
         part = [t.detach()[:, h:h + few] for t in (q, k, v, do)]
         want = _passes(*(t.requires_grad_() for t in part[:3]), None, part[3], 256, 2)
         assert all(torch.equal(a[:, h:h + few], b) for a, b in zip(got, want))
+    _lib_check()
+
+
+def test_two_streams_at_once():
+    """Two calls whose CTAs take work items at the same time, on streams of their own: each gives its own results."""
+    cases = []
+    for i, (D, c) in enumerate(((128, 64), (64, 10))):
+        g = torch.Generator(device="cuda").manual_seed(i)
+        q, k, v, do = (torch.randn(4, 24, 1500, D, generator=g, device="cuda").bfloat16() for _ in range(4))
+        lens = torch.tensor([1500, 400, 0, 1111], dtype=torch.int32, device="cuda")
+        args = (*(t.requires_grad_() for t in (q, k, v)), lens, do, c, 3)
+        cases.append((torch.cuda.Stream(), args, _passes(*args)))
+    torch.cuda.synchronize()
+    for _ in range(5):
+        got = []
+        for stream, args, _ in cases:
+            with torch.cuda.stream(stream):
+                got.append(_passes(*args))
+        torch.cuda.synchronize()
+        for mine, (_, _, want) in zip(got, cases):
+            assert all(torch.equal(a, b) for a, b in zip(mine, want))
     _lib_check()
 
 
