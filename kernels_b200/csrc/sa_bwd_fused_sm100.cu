@@ -128,11 +128,8 @@ inline int32_t fused_slots(int32_t T, int32_t c, int32_t back) {
 // its rows alone would need.
 inline int32_t packed_tiles(int32_t total, int32_t B) { return total / kBK + B + 1; }
 
-// dO tiles in shared memory.  With one, dO(g + 1) sets out when dV(g) is complete and dP(g + 1) waits for it: 350 to 640
-// of a tile's 4 300 to 6 000 clocks.  Head dim 64 has room for two (one / two, us: fp16 c=10 T=1353 300 / 298, c=37 T=1000
-// 208 / 191, c=128 T=4096 206 / 204, c=200 T=3000 181 / 174, packed c=50 393 / 385); head dim 128 has none left.
 template <int D>
-constexpr int kDoStages = D == 64 ? 2 : 1;
+constexpr int kDoStages = tiles::main_stages_do(D);
 
 template <int D>
 struct alignas(1024) FusedSmem {
@@ -509,8 +506,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           if (last) mma_commit(&sm.dv_done);  // the epilogue warps start on dV while dK(last) still runs
           KB_FTR(1, g, 2);
           KB_ACC(3);  // issue dV
-          // S(g+1): of this item, or the first of the next live one.  (Looking for the next item before the wait for
-          // P instead, off the chain, as the other classes' loop below does, measured 1 % slower in this one.)
+          // S(g+1): of this item, or the first of the next one.  (Reading the next item before the wait for P instead,
+          // off the chain, as the other classes' loop below does, measured 1 % slower in this one.)
           if (last) {
             items.next(ctx);
             cnt_next = item_tiles();
@@ -557,8 +554,8 @@ sa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           int cnt_next = 0;
           for (int t = 0; ok && t < cnt; ++t, ++g) {
             const bool first = t == 0, last = t == cnt - 1;
-            // The look for the next live item (a decode per candidate) is done here, before the wait for P: from
-            // that wait to the issue of S(g+1) the thread is on the kernel's critical chain.
+            // The next item (an entry of the ring, which may have to be waited for) is read here, before the wait for
+            // P: from that wait to the issue of S(g+1) the thread is on the kernel's critical chain.
             if (last) {
               items.next(ctx);
               cnt_next = item_tiles();

@@ -6,8 +6,8 @@
 // per FLOP against one q tile per CTA.  Ten warps, three roles (K and V rings two deep; output rows leave through shared memory and TMA stores):
 //   warps 0-3 / 4-7  softmax of q tile A / B: thread r owns query row r of its tile (= TMEM lane
 //              r).  Walks its row of a 128 x 128 block of S in TMEM twice, 32 columns at a time (row
-//              maximum, then exponentials in packed fp32 arithmetic), keeps the running max / sum,
-//              writes P (16-bit) back over S, rescales O when the max moved by more than 2^8,
+//              maximum, then exponentials in packed fp32 arithmetic; head dim 64 has an instance that holds
+//              the row in registers instead), keeps the running max / sum, writes P (16-bit) back over S, rescales O when the max moved by more than 2^8,
 //              writes O / LSE at the end;
 //   warp 8     TMA producer (one lane): Q once, then a ring of K tiles and a ring of V tiles; takes the work
 //              items from the hardware's queue (item_queue.cuh) and clears the outputs of padded ones;
@@ -115,7 +115,7 @@ struct alignas(1024) FwdSmem {
 enum WaitSite { kWaitQ = 1, kWaitQEmpty, kWaitOFree, kWaitKEmpty, kWaitVEmpty, kWaitKFull, kWaitVFull, kWaitSReady, kWaitPReady, kWaitEpilogue };
 constexpr int kErrSmemAlign = 11;
 
-// The softmax warps walk their row of a 128 x 128 block twice, 32 columns at a time, the next 32 on their way out of TMEM
+// But for the instance of head dim 64 below, the softmax warps walk their row of a 128 x 128 block twice, 32 columns at a time, the next 32 on their way out of TMEM
 // meanwhile.  The loops stay loops and there is one copy of the arithmetic with masks and one without: the code of a
 // block is what the MMA-issuing warp competes with for the instruction cache.  Both passes unrolled over the
 // row / as loops: bf16 D=128 c=64 806 / 682 us; the masked copy 64 columns wide / 32: packed c=64 649 / 569; one pass with all

@@ -26,10 +26,11 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
-// True in one lane of a converged warp.  MMA, commit and TMA instructions are issued under this predicate and not under
-// `lane == 0`: the compiler then knows that one lane is active and need not provide for more around every one of them
-// (their operands are registers of the warp).  `lane == 0` / this, us: main backward kernel fp16 D=64 c=10 363 / 324, c=128
-// 248 / 225, bf16 D=128 c=64 1276 / 1180, c=256 T=16384 1600 / 1553; forward 215 / 193, 140 / 132, 641 / 590, 813 / 808.
+// True in one lane of a converged warp.  The attention kernels issue their MMA and commit instructions under this predicate
+// and not under `lane == 0`: the compiler then knows that one lane is active and need not provide for more around every one of them
+// (their operands are registers of the warp).  `lane == 0` / this, us: main backward kernel fp16 D=64 c=10 363 / 323, c=128
+// 250 / 227, bf16 D=128 c=64 1276 / 1200, c=256 T=16384 1639 / 1592; forward (whose MMA warp became converged for it) 215 /
+// 194, 140 / 132, 641 / 600, packed c=64 622 / 580.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
