@@ -900,14 +900,16 @@ int launch(const kb_sa_fwd_params& p, int32_t c, int32_t back, cudaStream_t s, c
   if (n_items > (int64_t)1 << 30) return KB_ERR_TOO_LARGE;
   FwdArgs a;
   const int64_t n_blocks = PACKED ? packed_grid_blocks(a.grid, p.cu_seqlens, p.B, p.H, p.T, p.total_rows, 8) : n_items;
-  // Head dim 64: the scores held in registers (softmax_row_max_held) where no CTA sees a second item, and where a row walks 12
-  // key tiles or more.  Two walks / held, us, fp16: one wave, dense T=2048 37.1 / 32.5, T=1500 34.0 / 31.3, T=900 21.3 / 19.6,
+  // Head dim 64: the scores held in registers (softmax_row_max_held) where no CTA sees a second item, where a row walks 12
+  // key tiles or more, and in steps of one item per sequence and head whose rows walk three or more.  Two walks / held, us, fp16: one wave, dense T=2048 37.1 / 32.5, T=1500 34.0 / 31.3, T=900 21.3 / 19.6,
   // c=10 T=1000 12.2 / 11.7; many, T=4000 unless said, dense T=2048 328 / 319, T=3333 379 / 355, T=1500 303 / 288, c=256 back=6
   // 270 / 255, c=512 back=2 291 / 280, c=300 back=4 397 / 389, c=100 back=15 390 / 390.  Fewer tiles: c=256 T=1000 135 / 155,
   // back=3 183 / 177, c=200 back=4 258 / 268, c=128 back=4 154 / 150, c=100 back=6 259 / 289, c=10 196 / 209, dense T=700 206 / 217.
+  // Steps, bf16, new rows x all: 141 x 1269 94.5 / 88.4, 100 x 500 82.7 / 79.5, 50 x 400 222 / 212, 200 x 1000 172 / 166, 128 x 1024 106.9 /
+  // 106.9; 64 x 256 35.4 / 39.9; two items, 300 x 900 1014 / 1041.
   constexpr bool kHolds = D == 64 && !FP8;
   const int64_t row_keys = kb_min_i32(PACKED ? p.total_rows / p.B : p.T, (int32_t)std::min<int64_t>((int64_t)(back + 1) * c, INT32_MAX));
-  const bool held = kHolds && (n_items <= n_sm || row_keys >= 12 * kBN);
+  const bool held = kHolds && (n_items <= n_sm || row_keys >= 12 * kBN || (Tq <= kBM * kQTiles && row_keys >= 3 * kBN));
   auto kern = fast ? (held ? sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, true, kHolds> : sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, true, false>)
                    : (held ? sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, false, kHolds> : sa_fwd_sm100_kernel<D, BF16, PACKED, FP8, false, false>);
   constexpr size_t smem = sizeof(FwdSmem<D>);

@@ -85,6 +85,24 @@ def test_step_on_any_start_against_full_call_and_oracle(T, Tq, D, c, back, dtype
     assert torch.isfinite(lse).all()
 
 
+@pytest.mark.parametrize("Tq,T,c,back", [(64, 256, 64, 3), (141, 600, 141, 3), (256, 384, 256, 1), (128, 383, 128, 2), (300, 900, 300, 2)])
+def test_steps_of_many_streams_bitwise(Tq, T, c, back):
+    """Head dim 64, more streams than CTAs: both instances that such calls may take give the bits of calls on a few streams,
+    in which no CTA sees a second work item."""
+    from kernels_b200.streaming_attention import streaming_attention_step
+
+    B, H, few = 50, 8, 8
+    assert B * H > torch.cuda.get_device_properties(0).multi_processor_count >= few * H * -(-Tq // 256)
+    q, k, v = (t.cuda() for t in _inputs(B, H, H, T, 64, torch.bfloat16))
+    got = streaming_attention_step(q[:, :, T - Tq:], k, v, None, c, back, return_lse=True)
+    for b in range(0, B, 2 * few):
+        cut = slice(b, b + few)
+        want = streaming_attention_step(q[cut, :, T - Tq:], k[cut], v[cut], None, c, back, return_lse=True)
+        assert all(torch.equal(a[cut], w) for a, w in zip(got, want))
+    torch.cuda.synchronize()
+    _lib.check_device_status()
+
+
 def test_rolling_cache_reproduces_the_whole_sequence():
     from kernels_b200.streaming_attention import streaming_attention, streaming_attention_step
 
